@@ -70,16 +70,16 @@ rl_status lu_decompose_host(size_t n, T *a, size_t lda, uint64_t *perm) {
     RL_TRY(ensure_device());
     cudaStream_t s = cudaStreamPerThread;
     DevBuf<T> dA;
-    DevBuf<int> dpiv;
-    DevBuf<uint64_t> dperm, scratch;
+    DevBuf<int> dpiv, rows;
+    DevBuf<uint64_t> dperm;
     RL_TRY(dA.alloc(n * n, s));
     RL_TRY(dpiv.alloc(n, s));
     RL_TRY(dperm.alloc(n, s));
-    RL_TRY(scratch.alloc(n, s));
+    RL_TRY(rows.alloc(n, s));
     RL_TRY(copy_h2d(dA.p, n, a, lda, n, n, s));
     rl_status st = lu_factor_dev<T>(dA.p, (long long)n, (int)n, dpiv.p, s);
     if (st == RL_OK) {
-        RL_LAUNCH(ipiv_to_perm_kernel, 1, 32, 0, s, dpiv.p, (int)n, dperm.p, scratch.p);
+        RL_TRY(pivots_to_rows(dpiv.p, (int)n, rows.p, dperm.p, s));
         RL_TRY_CUDA(cudaMemcpyAsync(perm, dperm.p, n * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     }
     RL_TRY(copy_d2h(a, lda, dA.p, n, n, n, s));
@@ -333,18 +333,18 @@ rl_status matrix_solve_host(size_t n, T *a, size_t lda, T *b) {
     RL_TRY(ensure_device());
     cudaStream_t s = cudaStreamPerThread;
     DevBuf<T> dA, dB;
-    DevBuf<int> dpiv;
-    DevBuf<uint64_t> dperm, scratch;
+    DevBuf<int> dpiv, rows;
+    DevBuf<uint64_t> dperm;
     RL_TRY(dA.alloc(n * n, s));
     RL_TRY(dB.alloc(n, s));
     RL_TRY(dpiv.alloc(n, s));
     RL_TRY(dperm.alloc(n, s));
-    RL_TRY(scratch.alloc(n, s));
+    RL_TRY(rows.alloc(n, s));
     RL_TRY(copy_h2d(dA.p, n, a, lda, n, n, s));
     RL_TRY_CUDA(cudaMemcpyAsync(dB.p, b, n * sizeof(T), cudaMemcpyHostToDevice, s));
     rl_status st = lu_factor_dev<T>(dA.p, (long long)n, (int)n, dpiv.p, s);
     if (st == RL_OK) {
-        RL_LAUNCH(ipiv_to_perm_kernel, 1, 32, 0, s, dpiv.p, (int)n, dperm.p, scratch.p);
+        RL_TRY(pivots_to_rows(dpiv.p, (int)n, rows.p, dperm.p, s));
         st = factor_solve_dev<T>(dA.p, (long long)n, (int)n, 0, dperm.p, dB.p, 1, 1, s);
     }
     if (st == RL_OK) RL_TRY_CUDA(cudaMemcpyAsync(b, dB.p, n * sizeof(T), cudaMemcpyDeviceToHost, s));
@@ -360,19 +360,19 @@ rl_status matrix_inverse_host(size_t n, T *a, size_t lda, T *inv, size_t ldi) {
     RL_TRY(ensure_device());
     cudaStream_t s = cudaStreamPerThread;
     DevBuf<T> dA;
-    DevBuf<int> dpiv;
-    DevBuf<uint64_t> dperm, scratch;
+    DevBuf<int> dpiv, rows;
+    DevBuf<uint64_t> dperm;
     RL_TRY(dA.alloc(n * n, s));
     RL_TRY(dpiv.alloc(n, s));
     RL_TRY(dperm.alloc(n, s));
-    RL_TRY(scratch.alloc(n, s));
+    RL_TRY(rows.alloc(n, s));
     RL_TRY(copy_h2d(dA.p, n, a, lda, n, n, s));
     rl_status st = lu_factor_dev<T>(dA.p, (long long)n, (int)n, dpiv.p, s);
     if (st != RL_OK) {
         RL_TRY_CUDA(cudaStreamSynchronize(s));
         return st;
     }
-    RL_LAUNCH(ipiv_to_perm_kernel, 1, 32, 0, s, dpiv.p, (int)n, dperm.p, scratch.p);
+    RL_TRY(pivots_to_rows(dpiv.p, (int)n, rows.p, dperm.p, s));
     return inverse_from_factors<T>(dA.p, (int)n, 0, dperm.p, inv, ldi, s);
 }
 
@@ -433,9 +433,10 @@ rl_status matrix_det_host(size_t n, T *a, size_t lda, T *det) {
         RL_TRY_CUDA(cudaStreamSynchronize(s));
         return RL_OK;
     }
-    DevBuf<int> dpiv;
+    DevBuf<int> dpiv, rows;
     DevBuf<uint64_t> dperm, scratch;
     RL_TRY(dpiv.alloc(n, s));
+    RL_TRY(rows.alloc(n, s));
     RL_TRY(dperm.alloc(n, s));
     RL_TRY(scratch.alloc(n, s));
     rl_status st = lu_factor_dev<T>(dA.p, (long long)n, (int)n, dpiv.p, s);
@@ -445,7 +446,7 @@ rl_status matrix_det_host(size_t n, T *a, size_t lda, T *det) {
         return RL_OK;
     }
     RL_TRY(st);
-    RL_LAUNCH(ipiv_to_perm_kernel, 1, 32, 0, s, dpiv.p, (int)n, dperm.p, scratch.p);
+    RL_TRY(pivots_to_rows(dpiv.p, (int)n, rows.p, dperm.p, s));
     RL_LAUNCH(det_kernel<T>, 1, 32, 0, s, dA.p, (long long)n, (int)n, dperm.p, scratch.p, 0, dout.p);
     RL_TRY_CUDA(cudaMemcpyAsync(det, dout.p, sizeof(T), cudaMemcpyDeviceToHost, s));
     RL_TRY_CUDA(cudaStreamSynchronize(s));

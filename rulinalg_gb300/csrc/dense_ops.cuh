@@ -589,18 +589,6 @@ rl_status tri_solve_inv_dev(const TA *A, long long lda, int n, const T *Dinv, T 
     return RL_OK;
 }
 
-static __global__ void ipiv_to_perm_kernel(const int *ipiv, int n, uint64_t *perm, uint64_t *scratch) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    for (int i = 0; i < n; i++) scratch[i] = i;
-    for (int j = 0; j < n; j++) {
-        const int p = ipiv[j];
-        const uint64_t t = scratch[j];
-        scratch[j] = scratch[p];
-        scratch[p] = t;
-    }
-    for (int i = 0; i < n; i++) perm[scratch[i]] = i;  // the stored form is the inverse
-}
-
 // Solve with factors already on the device. kind 0 = LU (dperm: stored permutation),
 // 1 = Cholesky. B (n x nrhs, stride ldb) is overwritten.
 template <class T>

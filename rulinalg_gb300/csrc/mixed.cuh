@@ -94,14 +94,17 @@ static __global__ void colnorm_kernel(const double *__restrict__ V, long long ld
     }
 }
 
-// W = (float)(R / scale[c]) for the active columns (scale given as bits of a double).
+// W = (float)(R / scale[c]) (scale given as bits of a double), row i of W from row
+// rows[i] of R when a row map is given (the pivoting of an LU factor).
 static __global__ void scale_to_f32_kernel(const double *__restrict__ R, long long ldr, int n, int nrhs,
-                                    const unsigned long long *scale_bits, float *__restrict__ W, long long ldw) {
+                                    const unsigned long long *scale_bits, const int *__restrict__ rows,
+                                    float *__restrict__ W, long long ldw) {
     const long long total = (long long)n * nrhs;
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
         const int i = (int)(e / nrhs), c = (int)(e - (long long)i * nrhs);
         const double sc = __longlong_as_double((long long)scale_bits[c]);
-        W[(long long)i * ldw + c] = (float)(sc > 0 ? R[(long long)i * ldr + c] / sc : 0.0);
+        const int r = rows ? rows[i] : i;
+        W[(long long)i * ldw + c] = (float)(sc > 0 ? R[(long long)r * ldr + c] / sc : 0.0);
     }
 }
 

@@ -66,15 +66,15 @@ struct SweepInv {
     int *ctl = nullptr;  // 2 x sweep_ctl_words(n, nrhs) words, zeroed before each pair of sweeps
 };
 
-// W <- M^-1 W with the FP32 factor (LU: ipiv swaps, unit L, U; Cholesky: L, L^T). No
+// W <- M^-1 W with the FP32 factor (LU: unit L, U, W's rows already in pivoted order;
+// Cholesky: L, L^T). No
 // absolute-epsilon rule here: only a pivot below FLT_MIN counts as singular. With inv.D1
 // set, the sweeps apply the diagonal blocks' inverses (up to kSweepGroups x kSweepRhs
 // right-hand sides).
-inline rl_status precond_solve(const float *F, int n, int kind, const int *ipiv, float *W, long long ldw, int nrhs,
+inline rl_status precond_solve(const float *F, int n, int kind, float *W, long long ldw, int nrhs,
                                int *dstatus, cudaStream_t s, const SweepInv &inv = SweepInv()) {
     const float tiny = FLT_MIN;
     const int m1 = kind == RL_KIND_LU ? 0 : 1, m2 = kind == RL_KIND_LU ? 2 : 3;
-    if (kind == RL_KIND_LU) RL_TRY(laswp<float>(W, ldw, nrhs, 0, 0, ipiv, 0, n, s));
     if (inv.D1 && sweep_groups(nrhs) > 0) {
         const int words = sweep_ctl_words(n, nrhs);
         RL_TRY_CUDA(cudaMemsetAsync(inv.ctl, 0, 2 * words * sizeof(int), s));
@@ -88,9 +88,8 @@ inline rl_status precond_solve(const float *F, int n, int kind, const int *ipiv,
 // dst = M^-1 src for one FP64 vector with the solves in FP32 (the vector scaled by its
 // inf-norm around them): the semi-normal-equations preconditioner of lstsq_mixed.
 struct Minv32 {
-    const float *F;
-    int n, kind;
-    const int *ipiv;
+    const float *F;  // L of a Cholesky factor
+    int n;
     float *w32;
     unsigned long long *bits;  // 1 scale
     int *one;                  // device int 1
@@ -98,8 +97,8 @@ struct Minv32 {
     rl_status apply(const double *src, double *dst, cudaStream_t s) const {
         RL_TRY(colnorm_dev(src, 1, n, 1, bits, s));
         const int g = std::min(4 * num_sms(), ceil_div(n, 256));
-        RL_LAUNCH(scale_to_f32_kernel, g, 256, 0, s, src, 1LL, n, 1, bits, w32, 1LL);
-        RL_TRY(precond_solve(F, n, kind, ipiv, w32, 1, 1, dstatus, s));
+        RL_LAUNCH(scale_to_f32_kernel, g, 256, 0, s, src, 1LL, n, 1, bits, (const int *)nullptr, w32, 1LL);
+        RL_TRY(precond_solve(F, n, RL_KIND_CHOLESKY, w32, 1, 1, dstatus, s));
         RL_TRY_CUDA(cudaMemsetAsync(dst, 0, n * sizeof(double), s));
         RL_LAUNCH(update_x_kernel, g, 256, 0, s, dst, 1LL, w32, 1LL, n, 1, bits, one);
         return RL_OK;
@@ -116,7 +115,7 @@ struct Minv32 {
 struct Minv {
     const float *F;
     int n, kind;
-    const int *ipiv;
+    const int *rows;  // LU: the row map of the pivots (pivots_to_rows)
     int *dstatus;
     DevBuf<double> D1, D2;
     DevBuf<int> ctl;  // the two sweeps' ticket and block flags
@@ -131,9 +130,11 @@ struct Minv {
         return diag_inverse<double, float>(F, n, n, mode2(), D2.p, dstatus, s, FLT_MIN);
     }
     rl_status apply(const double *src, double *dst, cudaStream_t s) const {
-        RL_TRY_CUDA(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
         const double tiny = FLT_MIN;
-        if (kind == RL_KIND_LU) RL_TRY(laswp<double>(dst, 1, 1, 0, 0, ipiv, 0, n, s));
+        if (kind == RL_KIND_LU)
+            RL_TRY(gather_rows<double>(src, 1, dst, 1, n, 1, rows, s));
+        else
+            RL_TRY_CUDA(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
         const int words = 1 + ceil_div(n, kSweepRows);
         RL_TRY_CUDA(cudaMemsetAsync(ctl.p, 0, 2 * words * sizeof(int), s));
         RL_TRY((tri_solve_inv_dev<double, float>(F, n, n, D1.p, dst, 1, 1, mode1(), dstatus, s, tiny, ctl.p)));
@@ -250,6 +251,18 @@ inline rl_status gmres_ir(const double *A, long long lda, int n, const Minv &M, 
     return RL_OK;
 }
 
+// X = P B for an LU factor's pivots: a gather by their row map, or (X overlapping B, an
+// in-place solve) a copy and the swaps themselves.
+inline rl_status pivoted_copy(const double *B, long long ldb, double *X, long long ldx, int n, int nrhs, const int *ipiv,
+                              const int *rows, cudaStream_t s) {
+    if (X < B + (n - 1) * ldb + nrhs && B < X + (n - 1) * ldx + nrhs) {
+        RL_TRY_CUDA(cudaMemcpy2DAsync(X, ldx * sizeof(double), B, ldb * sizeof(double), nrhs * sizeof(double), n,
+                                      cudaMemcpyDeviceToDevice, s));
+        return laswp<double>(X, ldx, nrhs, 0, 0, ipiv, 0, n, s);
+    }
+    return gather_rows<double>(B, ldb, X, ldx, n, nrhs, rows, s);
+}
+
 // Plain FP64: copy A, factor, solve X = A^-1 B (LU: reference epsilon rules).
 inline rl_status solve_fp64(const double *A, long long lda, int n, int kind, const double *B, long long ldb, double *X,
                      long long ldx, int nrhs, cudaStream_t s) {
@@ -261,14 +274,17 @@ inline rl_status solve_fp64(const double *A, long long lda, int n, int kind, con
     RL_TRY_CUDA(cudaMemsetAsync(st.p, 0, sizeof(int), s));
     RL_TRY_CUDA(cudaMemcpy2DAsync(F.p, n * sizeof(double), A, lda * sizeof(double), n * sizeof(double), n,
                                   cudaMemcpyDeviceToDevice, s));
-    RL_TRY_CUDA(cudaMemcpy2DAsync(X, ldx * sizeof(double), B, ldb * sizeof(double), nrhs * sizeof(double), n,
-                                  cudaMemcpyDeviceToDevice, s));
     if (kind == RL_KIND_LU) {
         RL_TRY(lu_factor_dev<double>(F.p, n, n, ipiv.p, s));
-        RL_TRY(laswp<double>(X, ldx, nrhs, 0, 0, ipiv.p, 0, n, s));
+        DevBuf<int> rows;
+        RL_TRY(rows.alloc(n, s));
+        RL_TRY(pivots_to_rows(ipiv.p, n, rows.p, nullptr, s));
+        RL_TRY(pivoted_copy(B, ldb, X, ldx, n, nrhs, ipiv.p, rows.p, s));
         RL_TRY(tri_solve_dev<double>(F.p, n, n, X, ldx, nrhs, 0, st.p, s));
         RL_TRY(tri_solve_dev<double>(F.p, n, n, X, ldx, nrhs, 2, st.p, s));
     } else {
+        RL_TRY_CUDA(cudaMemcpy2DAsync(X, ldx * sizeof(double), B, ldb * sizeof(double), nrhs * sizeof(double), n,
+                                      cudaMemcpyDeviceToDevice, s));
         RL_TRY(chol_factor_dev<double>(F.p, n, n, s));
         RL_TRY(tri_solve_dev<double>(F.p, n, n, X, ldx, nrhs, 1, st.p, s));
         RL_TRY(tri_solve_dev<double>(F.p, n, n, X, ldx, nrhs, 3, st.p, s));
@@ -312,11 +328,11 @@ struct MixedFactor {
     long long lda = 0;
     double *A_own = nullptr;
     float *F = nullptr;
-    int *ipiv = nullptr;
+    int *ipiv = nullptr, *rows = nullptr;  // LU: the FP32 factor's pivots and their row map
     double anorm = 0.0;
     bool f32_ok = false;
     double *F64 = nullptr;
-    int *ipiv64 = nullptr;
+    int *ipiv64 = nullptr, *rows64 = nullptr;
     float *Dinv = nullptr;  // RL_TUNE_MIXED_SWEEP_INV: both triangles' inverted diagonal blocks
     rl_status f64_status = RL_OK;
     bool f64_ready = false;
@@ -328,18 +344,19 @@ struct MixedFactor {
     ~MixedFactor() { release(); }
 
     void release() {
-        void *ps[] = {A_own, F, ipiv, F64, ipiv64, Dinv};
+        void *ps[] = {A_own, F, ipiv, rows, F64, ipiv64, rows64, Dinv};
         for (void *p : ps)
             if (p) cudaFreeAsync(p, home);
-        A_own = nullptr, F = nullptr, ipiv = nullptr, F64 = nullptr, ipiv64 = nullptr, Dinv = nullptr;
+        A_own = nullptr, F = nullptr, ipiv = nullptr, rows = nullptr;
+        F64 = nullptr, ipiv64 = nullptr, rows64 = nullptr, Dinv = nullptr;
     }
 
     size_t dinv_elems() const { return (size_t)ceil_div(n, kSweepRows) * kSweepRows * kSweepRows; }
 
     size_t bytes() const {
-        size_t b = (size_t)n * n * sizeof(float) + (size_t)n * sizeof(int);
+        size_t b = (size_t)n * n * sizeof(float) + 2 * (size_t)n * sizeof(int);
         if (A_own) b += (size_t)n * n * sizeof(double);
-        if (F64) b += (size_t)n * n * sizeof(double) + (size_t)n * sizeof(int);
+        if (F64) b += (size_t)n * n * sizeof(double) + 2 * (size_t)n * sizeof(int);
         if (Dinv) b += 2 * dinv_elems() * sizeof(float);
         return b;
     }
@@ -390,6 +407,10 @@ struct MixedFactor {
                                                  : chol_factor_dev<float>(F, n, n, s, FLT_MIN);
         if (fst != RL_OK && fst != RL_ERR_DIV_BY_ZERO && fst != RL_ERR_DECOMP_FAILURE) return fst;
         f32_ok = fst == RL_OK;
+        if (f32_ok && kind == RL_KIND_LU) {
+            RL_TRY(alloc(rows, (size_t)n, s));
+            RL_TRY(pivots_to_rows(ipiv, n, rows, nullptr, s));
+        }
         unsigned long long hb = 0;
         RL_TRY_CUDA(cudaMemcpyAsync(&hb, nb.p, sizeof hb, cudaMemcpyDeviceToHost, s));
         RL_TRY_CUDA(cudaStreamSynchronize(s));
@@ -406,6 +427,10 @@ struct MixedFactor {
                                       cudaMemcpyDeviceToDevice, s));
         f64_status = kind == RL_KIND_LU ? lu_factor_dev<double>(F64, n, n, ipiv64, s)
                                         : chol_factor_dev<double>(F64, n, n, s);
+        if (f64_status == RL_OK && kind == RL_KIND_LU) {
+            RL_TRY(alloc(rows64, (size_t)n, s));
+            RL_TRY(pivots_to_rows(ipiv64, n, rows64, nullptr, s));
+        }
         f64_ready = true;
         return f64_status;
     }
@@ -418,13 +443,13 @@ struct MixedFactor {
         DevBuf<int> st;
         RL_TRY(st.alloc(1, s));
         RL_TRY_CUDA(cudaMemsetAsync(st.p, 0, sizeof(int), s));
-        RL_TRY_CUDA(cudaMemcpy2DAsync(X, ldx * sizeof(double), B, ldb * sizeof(double), nrhs * sizeof(double), n,
-                                      cudaMemcpyDeviceToDevice, s));
         if (kind == RL_KIND_LU) {
-            RL_TRY(laswp<double>(X, ldx, nrhs, 0, 0, ipiv64, 0, n, s));
+            RL_TRY(pivoted_copy(B, ldb, X, ldx, n, nrhs, ipiv64, rows64, s));
             RL_TRY(tri_solve_dev<double>(F64, n, n, X, ldx, nrhs, 0, st.p, s));
             RL_TRY(tri_solve_dev<double>(F64, n, n, X, ldx, nrhs, 2, st.p, s));
         } else {
+            RL_TRY_CUDA(cudaMemcpy2DAsync(X, ldx * sizeof(double), B, ldb * sizeof(double), nrhs * sizeof(double), n,
+                                          cudaMemcpyDeviceToDevice, s));
             RL_TRY(tri_solve_dev<double>(F64, n, n, X, ldx, nrhs, 1, st.p, s));
             RL_TRY(tri_solve_dev<double>(F64, n, n, X, ldx, nrhs, 3, st.p, s));
         }
@@ -462,8 +487,8 @@ struct MixedFactor {
         std::vector<int> conv(nrhs, 0), near(nrhs, 0);
         std::vector<double> prev(nrhs, INFINITY), bnorm(nrhs, 0.0);
         // x0 = M^-1 b
-        RL_LAUNCH(scale_to_f32_kernel, ge, 256, 0, s, B, ldb, n, nrhs, bn_b, W.p, (long long)nrhs);
-        RL_TRY(precond_solve(F, n, kind, ipiv, W.p, nrhs, nrhs, dstatus.p, s, inv));
+        RL_LAUNCH(scale_to_f32_kernel, ge, 256, 0, s, B, ldb, n, nrhs, bn_b, rows, W.p, (long long)nrhs);
+        RL_TRY(precond_solve(F, n, kind, W.p, nrhs, nrhs, dstatus.p, s, inv));
         RL_TRY_CUDA(cudaMemset2DAsync(X, ldx * sizeof(double), 0, nrhs * sizeof(double), n, s));
         RL_LAUNCH(update_x_kernel, ge, 256, 0, s, X, ldx, W.p, (long long)nrhs, n, nrhs, bn_b, active.p);
         std::vector<unsigned long long> hb(3 * nrhs);
@@ -512,8 +537,9 @@ struct MixedFactor {
                 break;
             }
             RL_TRY_CUDA(cudaMemcpyAsync(active.p, act.data(), nrhs * sizeof(int), cudaMemcpyHostToDevice, s));
-            RL_LAUNCH(scale_to_f32_kernel, ge, 256, 0, s, R.p, (long long)nrhs, n, nrhs, rn_b, W.p, (long long)nrhs);
-            RL_TRY(precond_solve(F, n, kind, ipiv, W.p, nrhs, nrhs, dstatus.p, s, inv));
+            RL_LAUNCH(scale_to_f32_kernel, ge, 256, 0, s, R.p, (long long)nrhs, n, nrhs, rn_b, rows, W.p,
+                      (long long)nrhs);
+            RL_TRY(precond_solve(F, n, kind, W.p, nrhs, nrhs, dstatus.p, s, inv));
             RL_LAUNCH(update_x_kernel, ge, 256, 0, s, X, ldx, W.p, (long long)nrhs, n, nrhs, rn_b, active.p);
         }
         if (!need_fp64) {
@@ -536,7 +562,7 @@ struct MixedFactor {
             DevBuf<double> xb, bb;
             RL_TRY(xb.alloc(n, s));
             RL_TRY(bb.alloc(n, s));
-            Minv M{F, n, kind, ipiv, dstatus.p + 1, {}, {}, {}};
+            Minv M{F, n, kind, rows, dstatus.p + 1, {}, {}, {}};
             RL_TRY(M.init(s));
             for (int c = 0; c < nrhs && !need_fp64; c++) {
                 if (conv[c]) continue;
@@ -651,7 +677,7 @@ inline rl_status lstsq_mixed(const double *A, long long lda, int m, int n, const
     RL_TRY(qr_factor_dev<float>(Q32.p, n, m, n, n, tau32.p, s));
     RL_LAUNCH(upper_to_lower_t_kernel, (int)std::min<long long>(8 * num_sms(), ((long long)n * n + 255) / 256), 256, 0, s,
               Q32.p, (long long)n, n, L.p);
-    Minv32 M{L.p, n, RL_KIND_CHOLESKY, nullptr, w32.p, bits.p + 2, one.p, dstatus.p};
+    Minv32 M{L.p, n, w32.p, bits.p + 2, one.p, dstatus.p};
     GemvT At{partial.p, chunks, rows_per};
     const int gv = std::min(4 * num_sms(), ceil_div(n, 256));
     // x0 = (R^T R)^-1 A^T b
