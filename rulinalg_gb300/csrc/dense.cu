@@ -24,7 +24,7 @@ rl_status gemm_public(int m, int n, int k, const T *a, long long lda, const T *b
                       cudaStream_t s, bool &used_tc) {
     NvtxRange nvtx_("rl.gemm");
     used_tc = false;
-    if constexpr (std::is_same<T, float>::value) used_tc = sgemm_tc_eligible(m, n, k);
+    used_tc = std::is_same<T, float>::value ? sgemm_tc_eligible(m, n, k) : dgemm_tc_eligible(m, n, k);
     return gemm<T, false, false>(m, n, k, T(1), a, lda, b, ldb, T(0), c, ldc, s);
 }
 

@@ -2,8 +2,8 @@
 // updates of the blocked factorisations:
 //     C = alpha * op(A) * op(B) + beta * C,   row-major, op = identity or transpose.
 // FP32 uses FFMA (74 TFLOP/s on GB300); FP64 uses DFMA (GB300's FP64 rate is the same
-// ~1 TFLOP/s through DFMA and through DMMA, so the SIMT form loses nothing and keeps one
-// code path). Tiles are double-buffered through shared memory; every thread owns a
+// ~1 TFLOP/s through DFMA and through DMMA) for small products and for what the tensor-core
+// form (gemm_f64tc.cuh) leaves. Tiles are double-buffered through shared memory; every thread owns a
 // TM x TN register tile split into 4x4 quadrants to keep shared-memory reads
 // conflict-free.
 #pragma once
@@ -11,6 +11,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "gemm_f64tc.cuh"
 #include "gemm_tc.cuh"
 
 namespace rl {
@@ -43,11 +44,12 @@ __device__ __forceinline__ void lds4<double>(const double *p, double (&o)[4]) {
 // op(A) is m x k: A[i * lda + p] (TA = false) or A[p * lda + i] (TA = true).
 // op(B) is k x n: B[p * ldb + j] (TB = false) or B[j * ldb + p] (TB = true).
 // LOWER = true computes only the tiles that touch the lower triangle (i >= j) and only
-// writes elements with i >= j (the SYRK form used by Cholesky).
+// writes elements with i >= j (the SYRK form used by Cholesky). only.flags restricts the
+// output to the tiles that the tensor-core kernel left (FP64, gemm_f64tc.cuh).
 template <class T, bool TA, bool TB, bool LOWER>
 __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T>::BN / GemmCfg<T>::TN))
     gemm_kernel(int m, int n, int k, T alpha, const T *__restrict__ A, long long lda, const T *__restrict__ B,
-                long long ldb, T beta, T *__restrict__ C, long long ldc, int kslice, long long zstride) {
+                long long ldb, T beta, T *__restrict__ C, long long ldc, int kslice, long long zstride, DgemmTcTiles only) {
     constexpr int BM = GemmCfg<T>::BM, BN = GemmCfg<T>::BN, BK = GemmCfg<T>::BK;
     constexpr int TM = GemmCfg<T>::TM, TN = GemmCfg<T>::TN;
     constexpr int NTX = BN / TN, NTY = BM / TM, NT = NTX * NTY;
@@ -69,6 +71,16 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
     const int tx = tid % NTX, ty = tid / NTX;
     const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
     if (LOWER && col0 > row0 + BM - 1) return;  // tile strictly above the diagonal
+    const int *flag_row = nullptr;
+    if (only.flags) {
+        if (*only.nfail == 0) return;
+        static_assert(!std::is_same<T, double>::value || tc64::BM % BM == 0, "one flag row per tile");
+        flag_row = only.flags + (row0 / tc64::BM) * only.gx;
+        const int c1 = min(n, col0 + BN) - 1;
+        int any = 0;
+        for (int c = col0 / only.bn; c <= c1 / only.bn; c++) any |= flag_row[c];
+        if (!any) return;
+    }
 
     T acc[TM][TN];
 #pragma unroll
@@ -185,6 +197,7 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
             const int gj = col0 + (j / 4) * (BN / SN_) + tx * 4 + (j % 4);
             if (gj >= n) continue;
             if (LOWER && gj > gi) continue;
+            if (flag_row && !flag_row[gj / only.bn]) continue;
             T *cp = C + (long long)gi * ldc + gj;
             T v = alpha * acc[i][j];
             if (beta != T(0)) v = fma(beta, *cp, v);
@@ -214,6 +227,14 @@ rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T 
             return sgemm_tc<TA, TB>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, LOWER, stream, ks);
         }
     }
+    DevBuf<unsigned char> ws;
+    DgemmTcTiles left;
+    if constexpr (std::is_same<T, double>::value) {  // FP64 with enough work: exact slices on the tensor cores
+        bool taken = false;
+        if (dgemm_tc_eligible(m, n, k))
+            RL_TRY((dgemm_tc<TA, TB>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, LOWER, stream, ws, left, taken)));
+        // what follows computes the tiles that were left (usually none), or all of C
+    }
     int ksplit = 1;
     if (!LOWER && tiles < sms && k >= 1024) ksplit = std::min({16, ceil_div(2 * sms, tiles), k / 256});
     if (ksplit > 1) {
@@ -224,13 +245,19 @@ rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T 
         RL_TRY(part.alloc((size_t)ksplit * zstride, stream));
         grid.z = ksplit;
         RL_LAUNCH((gemm_kernel<T, TA, TB, LOWER>), grid, NT, 0, stream, m, n, k, T(1), A, lda, B, ldb, T(0), part.p, (long long)n,
-                  kslice, zstride);
-        RL_LAUNCH(splitk_reduce_kernel<T>, std::min(4 * sms, ceil_div(zstride, 256)), 256, 0, stream, m, n, ksplit, alpha,
-                  part.p, beta, C, ldc);
+                  kslice, zstride, left);
+        const int rg = std::min(4 * sms, ceil_div(zstride, 256));
+        if constexpr (std::is_same<T, double>::value)
+            if (left.flags) {
+                RL_LAUNCH(dgemm_tc_reduce_kernel, rg, 256, 0, stream, m, n, ksplit, alpha, part.p, beta, C, ldc, left.flags,
+                          left.nfail, left.bn, left.gx, 1);
+                return RL_OK;
+            }
+        RL_LAUNCH(splitk_reduce_kernel<T>, rg, 256, 0, stream, m, n, ksplit, alpha, part.p, beta, C, ldc);
         return RL_OK;
     }
     RL_LAUNCH((gemm_kernel<T, TA, TB, LOWER>), grid, NT, 0, stream, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, k,
-              0ll);
+              0ll, left);
     return RL_OK;
 }
 
