@@ -17,8 +17,8 @@ namespace {
 // ------------------------------------------------------------- host entry points --
 
 // The public GEMM: FP32 with at least one 128 x 128 tile's worth of C and K >= 256 runs
-// on the tensor cores (3xTF32, FP32 accuracy); everything else, and all FP64, on the
-// SIMT kernel; both split a long K when the product has few output tiles (gemm()).
+// on the tensor cores (3xTF32, FP32 accuracy), FP64 from 6e6 multiply-adds on as exact BF16
+// slices; everything else on the SIMT kernel; both split a long K when the product has few output tiles (gemm()).
 template <class T>
 rl_status gemm_public(int m, int n, int k, const T *a, long long lda, const T *b, long long ldb, T *c, long long ldc,
                       cudaStream_t s, bool &used_tc) {

@@ -238,167 +238,457 @@ __device__ __forceinline__ void warp_amax_key(unsigned long long &k, int &i) {
     i = (int)__reduce_min_sync(0xffffffffu, top ? (unsigned)i : 0xffffffffu);
 }
 
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Cluster primitives of the panel kernels: a 16-byte store into another CTA's shared memory
+// that counts its bytes on that CTA's mbarrier, and the (bounded) wait for them.
+__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t a, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_async16(uint32_t dst, uint4 v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+                 "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void cl_mbar_init(uint64_t *bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void cl_mbar_expect(uint64_t *bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool cl_mbar_wait(uint64_t *bar, unsigned parity, unsigned long long limit) {
+    const uint32_t a = smem_addr(bar);
+    unsigned long long t0 = 0;
+    for (unsigned spin = 0;; spin++) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(a), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if ((spin & 63u) == 63u) {  // the timer is read once per 64 polls
+            if (t0 == 0)
+                t0 = global_ns();
+            else if (global_ns() - t0 > limit)
+                return false;
+        }
+    }
+}
+
 // LU panel on one thread-block cluster (up to 16 CTAs): the same algorithm as
-// lu_panel_kernel with the cross-CTA exchange moved on chip. CTA g owns rows
-// [g * rows_per, ...) in shared memory; inside a CTA, `tpr` consecutive threads (1, 2, 4
-// or 8) share each row, thread q of a row owning the columns c = q (mod tpr), and thread
-// group t the rows t, t + 256 / tpr, ... The panel's row updates run at the SM's FP64
-// rate, so spreading a few rows over all four schedulers of every SM of the cluster is
-// what shortens a column. Per column:
-//   1. each thread searches column j of its rows (the thread that wrote them), the warps
-//      reduce on integer keys, one CTA barrier, every thread combines the warps' maxima;
-//   2. the CTA pushes its candidate row (and row j, if it holds it) into every CTA's
-//      tables with 16-byte remote shared-memory stores, and its record (key, row,
-//      1 / pivot);
-//   3. one cluster barrier (release / acquire); every warp picks the same winner from
-//      its own CTA's table, where the winning row and row j already are;
-//   4. the swap and the update run at once, each element stored by one thread: thread
-//      c < kb stores column c of the new row j and, for c < j, of row wi; the threads of
-//      row wi compute its columns >= j from the old row j; every other row below j
-//      updates itself, the multiplier broadcast within the row's threads by a shuffle.
-// Tables and records are double-buffered by column parity: a CTA writes slot s again
-// only after the next cluster barrier, which every CTA reaches after it has read slot s.
-// Every CTA runs the same barrier sequence (a failing pivot is seen by all at the same
-// column).
+// lu_panel_kernel with the cross-CTA exchange on chip. CTA g owns the rows
+// [g * rows_per, ...), staged in shared memory. The panel is factored 16 columns at a time
+// in registers: TPR consecutive threads share a row (TPR > 1 when a CTA holds few rows, so
+// that the FP64 updates use every scheduler), thread q of them owning the columns
+// c = q (mod TPR) of the 16, and a thread group holds RPT rows. Per column:
+//   1. the threads search the column of their rows, the warps reduce on integer keys, each
+//      warp's best row goes to shared memory; one CTA barrier;
+//   2. the CTA pushes its candidate (16 columns), row j if it holds it, and its record (key,
+//      row, 1 / pivot) into every CTA's tables with st.async, which counts the bytes on the
+//      receiver's mbarrier: one one-way trip, no cluster barrier;
+//   3. every CTA waits for its own table to be complete; every warp picks the same winner;
+//   4. swap and update in registers.
+// After the 16 columns the row swaps reach the panel's other columns: their composition (at
+// most 32 rows) is formed from the pivots, the moved rows and the 16 pivot rows are read from
+// the CTAs that hold them, one cluster barrier, then U12 = L11^-1 A12 (in every
+// CTA) and the update of the columns to the right, each row adding its 16 products in
+// column order: every element sees the operations of the unblocked elimination, in the same
+// order. Tables and barriers are double-buffered by column parity: a CTA pushes column
+// j + 2 only after it has received every CTA's column j + 1, which those push after their
+// last read of column j's tables.
+// Bound by a column's chain of dependent steps (FP32: ~2,500 cycles, of which the exchange
+// is ~500) or by the FP64 unit of the cluster's SMs. The form before pushed all 64 columns
+// and passed a cluster barrier per column, with the panel in shared memory: 172 us per FP32
+// panel averaged over n = 4096, 89 now; 16 CTAs of 512 rows 250 and 119 us; FP64 234 and
+// 201 us.
+// A failing pivot is seen by all CTAs at the same column and acted on after the next CTA
+// barrier (the flag is kept per column parity, so a thread ahead by a column does not show
+// its finding to one that still has to read the last column's). Every wait is bounded
+// (RL_ERR_TIMEOUT); a CTA whose wait ran out tells the others before it leaves.
+constexpr int kPanelSub = 16;
 template <class T>
+struct PanelTables {
+    static constexpr int RECW = sizeof(T) == 4 ? 1 : 2;  // 16-byte words of a record
+    uint4 rec[2][16][RECW];                             // {key lo, key hi | 1 / pivot, row, -}, {1 / pivot}
+    T tab[2][16][kPanelSub];                            // every CTA's candidate row
+    T rowj[2][kPanelSub];                               // row j
+    T cand[2][8][kPanelSub];                            // the warps' candidates
+    T candj[2][kPanelSub];                              // row j, in the CTA that holds it
+    T L11t[kPanelSub][kPanelSub];                       // L11t[k][i] = l_ik of the pivot rows
+    T U[64 - kPanelSub][kPanelSub];                     // U12 by columns
+    unsigned long long s_k[2][8];
+    int s_i[2][8];
+    int piv[kPanelSub];
+    int dst[32];        // moved rows of this CTA: where to (-1: none) ...
+    uint32_t src[32];   // ... and where every moved row is (cluster shared address)
+    uint64_t full[2];
+    int fail[2];  // by column parity: 1 = a wait ran out, 2 = a failing pivot
+    int dead;     // another CTA's wait ran out
+};
+
+__device__ __forceinline__ float ld_cluster(uint32_t a, float) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ double ld_cluster(uint32_t a, double) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+    return v;
+}
+// N consecutive values (16-byte aligned) from / to shared memory, 16 bytes at a time.
+template <int N, class T>
+__device__ __forceinline__ void ldv(const T *p, T (&v)[N]) {
+    constexpr int W = 16 / (int)sizeof(T);
+#pragma unroll
+    for (int i = 0; i < N; i += W) {
+        const uint4 x = *reinterpret_cast<const uint4 *>(p + i);
+        const T *e = reinterpret_cast<const T *>(&x);
+#pragma unroll
+        for (int u = 0; u < W; u++) v[i + u] = e[u];
+    }
+}
+template <int N, class T>
+__device__ __forceinline__ void stv(T *p, const T (&v)[N]) {
+    constexpr int W = 16 / (int)sizeof(T);
+#pragma unroll
+    for (int i = 0; i < N; i += W) {
+        uint4 x;
+        T *e = reinterpret_cast<T *>(&x);
+#pragma unroll
+        for (int u = 0; u < W; u++) e[u] = v[i + u];
+        *reinterpret_cast<uint4 *>(p + i) = x;
+    }
+}
+
+// Rows in the tables and in registers are kept rotated: at local column step jo the entry
+// q L + i of a row is its column ((jo + i) mod L) TPR + q.
+template <class T, int TPR, int RPT>
 static __global__ void __launch_bounds__(256) lu_panel_cluster_kernel(T *P, long long lda, int mrows, int kb, int k0,
-                                                              int rows_per, int tpr, int *ipiv, int *err, T tiny) {
+                                                              int rows_per, int *ipiv, int *err, T tiny,
+                                                              unsigned long long wait_ns) {
     namespace cg = cooperative_groups;
-    constexpr int NB = PanelNB<T>::value;
-    constexpr int LDR = NB + 1;
-    constexpr int CMAX = 16;
-    constexpr int VW = 16 / (int)sizeof(T);  // elements per 16-byte chunk of a row
+    constexpr int NB = PanelNB<T>::value, LDR = NB + 1, SW = kPanelSub, L = SW / TPR, G = 256 / TPR;
+    constexpr int RECW = PanelTables<T>::RECW, CH = SW * (int)sizeof(T) / 16;  // 16-byte words of a record, a row
+    static_assert(16 * CH <= 224, "one candidate word per thread of warps 1 .. 7");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *tab = reinterpret_cast<T *>(smem_raw);  // 2 x CMAX x NB: every CTA's candidate row
-    T *rowj = tab + 2 * CMAX * NB;             // 2 x NB: row j (pushed by the CTA holding it)
-    T *R = rowj + 2 * NB;                      // rows_per x LDR
-    __shared__ unsigned long long s_k[8], rec_k[2 * CMAX];
-    __shared__ int s_i[8], rec_i[2 * CMAX];
-    __shared__ T rec_inv[2 * CMAX];
+    T *R = reinterpret_cast<T *>(smem_raw);  // rows_per x LDR
+    __shared__ __align__(16) PanelTables<T> S;
     cg::cluster_group cluster = cg::this_cluster();
     const int C = (int)cluster.num_blocks(), g = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r0 = g * rows_per, r1 = min(mrows, r0 + rows_per), nr = max(0, r1 - r0);
-    const int q = tid & (tpr - 1), grp = tid / tpr, G = (int)blockDim.x / tpr;
-    const int rpt = (rows_per + G - 1) / G;  // rows per thread group, the same in every thread
+    const int q = tid & (TPR - 1), grp = tid / TPR;
     const unsigned long long ktiny = amax_key(tiny);
+    const unsigned bytes = (unsigned)(16 * (C * (RECW + CH) + CH));
     if (g == 0)
-        for (int j = tid; j < kb; j += blockDim.x) ipiv[j] = k0 + j;
-    for (int idx = tid; idx < nr * kb; idx += blockDim.x) {
+        for (int j = tid; j < kb; j += 256) ipiv[j] = k0 + j;
+    for (int idx = tid; idx < nr * kb; idx += 256) {
         const int r = idx / kb, c = idx - r * kb;
         R[r * LDR + c] = P[(long long)(r0 + r) * lda + c];
     }
-    __syncthreads();
-    for (int j = 0; j < kb; j++) {
-        const int slot = j & 1, qj = j & (tpr - 1);
-        // 1. local candidate
-        unsigned long long bk = 0ull;
-        int bi = INT_MAX;
-        if (q == qj)
-            for (int k = 0; k < rpt; k++) {
-                const int r = grp + k * G;
-                if (r < nr && r0 + r >= j) {
-                    const unsigned long long key = amax_key(R[r * LDR + j]);
-                    if (key > bk) {
-                        bk = key;
-                        bi = r0 + r;
+    if (tid == 0) {
+        S.fail[0] = S.fail[1] = S.dead = 0;
+        cl_mbar_init(&S.full[0], 1);
+        cl_mbar_init(&S.full[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    cluster.sync();
+    cluster_arrive();  // waited for before the first read of other CTAs' rows
+    bool arrived = true, stop = false;
+    // what this thread pushes per column: warp 0 lane d the record to CTA d, thread 32 + e
+    // word e % CH of the candidate (and of row j) to CTA e / CH
+    const int pe = tid - 32, pto = warp == 0 ? lane : pe / CH, pch = pe & (CH - 1);
+    const bool pusher = warp == 0 ? lane < C : pe < C * CH;
+    const int peer = min(pto, C - 1);
+    const uint32_t bar_to = cluster_addr(smem_addr(&S.full[0]), peer);
+    const uint32_t tab_to = cluster_addr(warp == 0 ? smem_addr(&S.rec[0][g][0]) : smem_addr(S.tab[0][g]) + 16 * pch, peer);
+    const uint32_t rowj_to = cluster_addr(smem_addr(S.rowj[0]) + 16 * (pch & (CH - 1)), peer);
+    for (int c0 = 0; c0 < kb && !stop; c0 += SW) {
+        const int w = min(SW, kb - c0);
+        T a[RPT][L];
+#pragma unroll
+        for (int k = 0; k < RPT; k++) {
+            const int r = grp + k * G;
+#pragma unroll
+            for (int i = 0; i < L; i++) {
+                const int c = c0 + i * TPR + q;
+                a[k][i] = (r < nr && c < kb) ? R[r * LDR + c] : T(0);
+            }
+        }
+        // The column loop is rolled over jl / TPR, the body unrolled over the TPR owners.
+        for (int jo = 0; jo < L && !stop; jo++) {
+#pragma unroll
+            for (int qj = 0; qj < TPR; qj++) {
+                const int jl = jo * TPR + qj, j = c0 + jl, slot = j & 1;
+                if (jl >= w || stop) break;
+                // 1. local candidate
+                unsigned long long bk = 0ull;
+                int bi = INT_MAX;
+                if (q == qj)
+#pragma unroll
+                    for (int k = 0; k < RPT; k++) {
+                        const int r = grp + k * G;
+                        if (r < nr && r0 + r >= j) {
+                            const unsigned long long key = amax_key(a[k][0]);
+                            if (key > bk) {
+                                bk = key;
+                                bi = r0 + r;
+                            }
+                        }
+                    }
+                warp_amax_key<T>(bk, bi);
+#pragma unroll
+                for (int k = 0; k < RPT; k++) {
+                    const int gr = r0 + grp + k * G;
+                    if (gr == bi && bk != 0ull) stv<L>(&S.cand[slot][warp][q * L], a[k]);
+                    if (gr == j && j < r1) stv<L>(&S.candj[slot][q * L], a[k]);
+                }
+                if (lane == 0) {
+                    S.s_k[slot][warp] = bk;
+                    S.s_i[slot][warp] = bi;
+                }
+                __syncthreads();
+                if (*(volatile int *)&S.fail[slot ^ 1]) {
+                    stop = true;
+                    break;
+                }
+                bk = lane < 8 ? S.s_k[slot][lane] : 0ull;
+                bi = lane < 8 ? S.s_i[slot][lane] : INT_MAX;
+                const unsigned long long mk = bk;
+                const int mi = bi;
+                warp_amax_key<T>(bk, bi);
+                const int bw = bk != 0ull ? __ffs(__ballot_sync(0xffffffffu, mk == bk && mi == bi)) - 1 : 0;
+                // 2. push
+                const uint32_t bar = bar_to + 8 * slot;
+                if (warp == 0) {
+                    if (lane == 0) cl_mbar_expect(&S.full[slot], bytes);
+                    // the candidate's entry in column j: owner qj, rotated index 0
+                    const T inv = bk != 0ull ? T(1) / S.cand[slot][bw][qj * L] : T(0);
+                    if (pusher) {
+                        const uint32_t d = tab_to + slot * (unsigned)sizeof(S.rec[0]);
+                        const unsigned row = bk != 0ull ? (unsigned)bi : (unsigned)INT_MAX;
+                        if (sizeof(T) == 4) {
+                            st_async16(d, make_uint4((unsigned)bk, __float_as_uint((float)inv), row, 0u), bar);
+                        } else {
+                            st_async16(d, make_uint4((unsigned)bk, (unsigned)(bk >> 32), row, 0u), bar);
+                            const unsigned long long ib = (unsigned long long)__double_as_longlong((double)inv);
+                            st_async16(d + 16, make_uint4((unsigned)ib, (unsigned)(ib >> 32), 0u, 0u), bar);
+                        }
+                    }
+                } else if (pusher) {
+                    st_async16(tab_to + slot * (unsigned)sizeof(S.tab[0]),
+                               reinterpret_cast<const uint4 *>(S.cand[slot][bw])[pch], bar);
+                    if (j >= r0 && j < r1)
+                        st_async16(rowj_to + slot * (unsigned)sizeof(S.rowj[0]),
+                                   reinterpret_cast<const uint4 *>(S.candj[slot])[pch], bar);
+                }
+                // 3. the winner, the same in every warp of every CTA
+                if (!cl_mbar_wait(&S.full[slot], (j >> 1) & 1, wait_ns)) S.fail[slot] = 1;
+                unsigned long long wk = 0ull;
+                int wi = INT_MAX;
+                if (lane < C) {
+                    const uint4 v = S.rec[slot][lane][0];
+                    wk = sizeof(T) == 4 ? (unsigned long long)v.x : ((unsigned long long)v.y << 32) | v.x;
+                    wi = (int)v.z;
+                }
+                const unsigned long long rk = wk;
+                const int ri = wi;
+                warp_amax_key<T>(wk, wi);
+                int wg = -1;
+                if (wk != 0ull) {
+                    wg = __ffs(__ballot_sync(0xffffffffu, rk == wk && ri == wi)) - 1;
+                    wi = min(max(wi, j), mrows - 1);  // in range even after a wait that ran out
+                    if (wk < ktiny) {                 // the same decision in every CTA
+                        if (g == 0 && tid == 0) atomicCAS(err, 0, RL_ERR_DIV_BY_ZERO);
+                        S.fail[slot] = 2;
+                    }
+                } else {  // no finite candidate (NaN column): keep the diagonal
+                    wi = j;
+                }
+                const T *oldj = S.rowj[slot];
+                const T *prow = wg >= 0 ? S.tab[slot][wg] : oldj;
+                T inv_p;
+                if (wg < 0) {
+                    inv_p = T(1) / oldj[qj * L];
+                } else if (sizeof(T) == 4) {
+                    inv_p = (T)__uint_as_float(S.rec[slot][wg][0].y);
+                } else {
+                    const uint4 v = S.rec[slot][wg][RECW - 1];
+                    inv_p = (T)__longlong_as_double((long long)(((unsigned long long)v.y << 32) | v.x));
+                }
+                // 4. swap and update
+                T pr[L];
+                ldv<L>(prow + q * L, pr);
+#pragma unroll
+                for (int k = 0; k < RPT; k++) {
+                    const int r = grp + k * G, gr = r0 + r;
+                    const bool live = r < nr && gr > j;
+                    if (wi != j && r < nr && (gr == j || gr == wi)) ldv<L>((gr == j ? prow : oldj) + q * L, a[k]);
+                    T l = a[k][0] * inv_p;  // the thread that owns column j
+                    if (TPR > 1) l = __shfl_sync(0xffffffffu, l, qj, TPR);
+                    if (qj < TPR - 1) {
+                        if (live) {
+                            if (q == qj)
+                                a[k][0] = l;
+                            else if (q > qj)
+                                a[k][0] = fma(-l, pr[0], a[k][0]);
+#pragma unroll
+                            for (int i = 1; i < L; i++)
+                                if (jo + i < L) a[k][i] = fma(-l, pr[i], a[k][i]);
+                        }
+                    } else {  // the last owner: update and rotate at once
+                        T first = a[k][0];
+                        if (live) {
+                            if (q == qj) first = l;
+#pragma unroll
+                            for (int i = 1; i < L; i++) a[k][i - 1] = jo + i < L ? fma(-l, pr[i], a[k][i]) : a[k][i];
+                        } else {
+#pragma unroll
+                            for (int i = 1; i < L; i++) a[k][i - 1] = a[k][i];
+                        }
+                        a[k][L - 1] = first;
                     }
                 }
+                if (warp == 7) {  // for the block's end: the pivot and row jl of L11
+                    if (lane == 0) {
+                        S.piv[jl] = wi;
+                        if (g == 0) ipiv[j] = k0 + wi;
+                    }
+                    if (lane < SW) S.L11t[lane][jl] = prow[(lane & (TPR - 1)) * L + ((lane / TPR - jo) & (L - 1))];
+                }
             }
-        warp_amax_key<T>(bk, bi);
-        if (lane == 0) {
-            s_k[warp] = bk;
-            s_i[warp] = bi;
-        }
-        __syncthreads();  // also: every row's update for the previous column is done
-        bk = s_k[0];
-        bi = s_i[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
-            const unsigned long long k2 = s_k[w];
-            const int i2 = s_i[w];
-            if (k2 > bk || (k2 == bk && i2 < bi)) {
-                bk = k2;
-                bi = i2;
-            }
-        }
-        // 2. push the candidate row (and row j, from the CTA holding it) into every CTA's
-        // tables in 16-byte stores, and the record
-        const int nch = (kb + VW - 1) / VW;
-        if (bk != 0ull)
-            for (int idx = tid; idx < C * nch; idx += blockDim.x) {
-                const int dst = idx / nch, ch = idx - dst * nch;
-                const T *src = R + (size_t)(bi - r0) * LDR + ch * VW;
-                uint4 v;
-                T *vt = reinterpret_cast<T *>(&v);
+            if (jo * TPR + TPR > w && !stop) {  // a short last block skipped the rotating step
 #pragma unroll
-                for (int e = 0; e < VW; e++) vt[e] = src[e];
-                *reinterpret_cast<uint4 *>(cluster.map_shared_rank(tab + (slot * CMAX + g) * NB + ch * VW, dst)) = v;
-            }
-        if (j >= r0 && j < r1)
-            for (int idx = tid; idx < C * nch; idx += blockDim.x) {
-                const int dst = idx / nch, ch = idx - dst * nch;
-                const T *src = R + (size_t)(j - r0) * LDR + ch * VW;
-                uint4 v;
-                T *vt = reinterpret_cast<T *>(&v);
+                for (int k = 0; k < RPT; k++) {
+                    const T first = a[k][0];
 #pragma unroll
-                for (int e = 0; e < VW; e++) vt[e] = src[e];
-                *reinterpret_cast<uint4 *>(cluster.map_shared_rank(rowj + slot * NB + ch * VW, dst)) = v;
+                    for (int i = 1; i < L; i++) a[k][i - 1] = a[k][i];
+                    a[k][L - 1] = first;
+                }
             }
+        }
+        if (stop) break;
+        // registers back to the staged rows (after L rotations the columns are in order)
+#pragma unroll
+        for (int k = 0; k < RPT; k++) {
+            const int r = grp + k * G;
+#pragma unroll
+            for (int i = 0; i < L; i++) {
+                const int c = c0 + i * TPR + q;
+                if (r < nr && c < kb) R[r * LDR + c] = a[k][i];
+            }
+        }
+        if (kb <= SW) break;
+        // The swaps in the panel's other columns. Lane l < 16 of warp 0 takes position c0 + l,
+        // lane 16 + t the outside position first swapped in at column t, and follows the
+        // swaps backwards to the row that ends there.
+        const int nright = kb - c0 - w, nother = c0 + nright;
+        cluster_wait();  // every CTA's last update of these columns is visible
+        arrived = false;
+        __syncthreads();
+        if (*(volatile int *)&S.fail[(c0 + w - 1) & 1]) break;
         if (warp == 0) {
-            const T inv = bk != 0ull ? T(1) / R[(bi - r0) * LDR + j] : T(0);
-            if (lane < C) {
-                const int e = slot * CMAX + g;
-                *cluster.map_shared_rank(rec_k + e, lane) = bk;
-                *cluster.map_shared_rank(rec_i + e, lane) = bk != 0ull ? bi : INT_MAX;
-                *cluster.map_shared_rank(rec_inv + e, lane) = inv;
+            const int t0 = lane & 15;
+            int pos = lane < 16 ? c0 + lane : (t0 < w ? S.piv[t0] : -1);
+            if (lane >= 16 && pos < c0 + SW) pos = -1;
+            for (int t = 0; t < t0; t++)
+                if (lane >= 16 && S.piv[t] == pos) pos = -1;
+            int at = pos;
+            for (int t = w - 1; t >= 0; t--) {
+                const int x = S.piv[t], y = c0 + t;
+                at = at == x ? y : (at == y ? x : at);
             }
+            const int sg = max(at, 0) / rows_per;
+            S.dst[lane] = pos >= 0 && at != pos && pos >= r0 && pos < r1 ? pos - r0 : -1;
+            S.src[lane] = cluster_addr(smem_addr(R + (max(at, 0) - sg * rows_per) * LDR), min(sg, C - 1));
         }
-        cluster.sync();
-        // 3. the winner, the same in every warp of every CTA
-        unsigned long long wk = lane < C ? rec_k[slot * CMAX + lane] : 0ull;
-        int wi = lane < C ? rec_i[slot * CMAX + lane] : INT_MAX;
-        warp_amax_key<T>(wk, wi);
-        int wg = -1;
-        if (wk != 0ull) {
-            if (wk < ktiny) {  // the same decision in every CTA
-                if (g == 0 && tid == 0) atomicCAS(err, 0, RL_ERR_DIV_BY_ZERO);
-                break;
+        __syncthreads();
+        constexpr int MV = 32 * (NB - SW) / 256, UV = SW * (NB - SW) / 256;
+        T mv[MV], uv[UV];
+#pragma unroll
+        for (int i = 0; i < MV; i++) {
+            const int e = tid + i * 256, m = e / (NB - SW), cc = e % (NB - SW), c = cc < c0 ? cc : cc + w;
+            if (cc < nother && S.dst[m] >= 0) mv[i] = ld_cluster(S.src[m] + c * (unsigned)sizeof(T), T(0));
+        }
+        if (nright > 0)
+#pragma unroll
+            for (int i = 0; i < UV; i++) {
+                const int e = tid + i * 256, m = e / (NB - SW), cc = e % (NB - SW);
+                if (cc < nright) uv[i] = ld_cluster(S.src[m] + (c0 + SW + cc) * (unsigned)sizeof(T), T(0));
             }
-            wg = wi / rows_per;
-        } else {  // no finite candidate (NaN column): keep the diagonal
-            wi = j;
+        if (nright > 0)
+#pragma unroll
+            for (int i = 0; i < UV; i++) {
+                const int e = tid + i * 256, m = e / (NB - SW), cc = e % (NB - SW);
+                if (cc < nright) S.U[cc][m] = uv[i];
+            }
+        cluster.sync();  // every read of the old rows is done
+        if (*(volatile int *)&S.dead) break;
+#pragma unroll
+        for (int i = 0; i < MV; i++) {
+            const int e = tid + i * 256, m = e / (NB - SW), cc = e % (NB - SW), c = cc < c0 ? cc : cc + w;
+            if (cc < nother && S.dst[m] >= 0) R[S.dst[m] * LDR + c] = mv[i];
         }
-        const T *oldj = rowj + slot * NB;                                // the old row j
-        const T *prow = wg >= 0 ? tab + (slot * CMAX + wg) * NB : oldj;  // the pivot row
-        if (g == 0 && tid == 0) ipiv[j] = k0 + wi;
-        const T inv_p = wg >= 0 ? rec_inv[slot * CMAX + wg] : T(1) / oldj[j];
-        // 4. swap and update
-        if (wi != j && tid < kb) {
-            if (j >= r0 && j < r1) R[(j - r0) * LDR + tid] = prow[tid];
-            if (wi >= r0 && wi < r1 && tid < j) R[(wi - r0) * LDR + tid] = oldj[tid];
+        if (nright <= 0) break;
+        // w = 16 here: U12 = L11^-1 A12, a thread per column, rows in order
+        if (tid < nright) {
+            T x[SW];
+            ldv<SW>(S.U[tid], x);
+#pragma unroll
+            for (int k = 0; k < SW - 1; k++) {
+                T l[SW];
+                ldv<SW>(S.L11t[k], l);
+#pragma unroll
+                for (int i = k + 1; i < SW; i++) x[i] = fma(-l[i], x[k], x[i]);
+            }
+            stv<SW>(S.U[tid], x);
         }
-        const int cfirst = j + 1 + ((q - j - 1) & (tpr - 1));  // this thread's first column > j
-        for (int k = 0; k < rpt; k++) {
+        __syncthreads();
+        // the rows below the pivots: A22 -= L21 U12; the pivot rows: U12 itself
+        for (int k = 0; k < RPT; k++) {
             const int r = grp + k * G, gr = r0 + r;
-            const bool valid = r < nr && gr > j;
-            T *row = R + (size_t)(valid ? r : 0) * LDR;
-            const T *src = gr == wi ? oldj : row;
-            T l = T(0);
-            if (valid && q == qj) l = src[j] * inv_p;
-            if (tpr > 1) l = __shfl_sync(0xffffffffu, l, qj, tpr);
-            if (valid) {
-                if (q == qj) row[j] = l;
-#pragma unroll 4
-                for (int c = cfirst; c < kb; c += tpr) row[c] = fma(-l, prow[c], src[c]);
+            if (r >= nr || gr < c0) continue;
+            T *row = R + (size_t)r * LDR + c0;
+            if (gr < c0 + SW) {
+                for (int c = q; c < nright; c += TPR) row[SW + c] = S.U[c][gr - c0];
+                continue;
+            }
+            T l[SW];
+#pragma unroll
+            for (int i = 0; i < SW; i++) l[i] = row[i];
+#pragma unroll 2
+            for (int c = q; c < nright; c += TPR) {
+                T v = row[SW + c], u[SW];
+                ldv<SW>(S.U[c], u);
+#pragma unroll
+                for (int i = 0; i < SW; i++) v = fma(-l[i], u[i], v);
+                row[SW + c] = v;
             }
         }
+        __syncthreads();
+        cluster_arrive();
+        arrived = true;
     }
     __syncthreads();
-    for (int idx = tid; idx < nr * kb; idx += blockDim.x) {
+    if (S.fail[0] == 1 || S.fail[1] == 1) {
+        if (tid == 0) atomicCAS(err, 0, RL_ERR_TIMEOUT);
+        if (tid < C) *cluster.map_shared_rank(&S.dead, tid) = 1;
+    }
+    if (arrived) cluster_wait();
+    __syncthreads();
+    for (int idx = tid; idx < nr * kb; idx += 256) {
         const int r = idx / kb, c = idx - r * kb;
         P[(long long)(r0 + r) * lda + c] = R[r * LDR + c];
     }
-    cluster.sync();  // no CTA leaves while another may still read its shared memory
+    cluster.sync();  // no CTA leaves while another may still use its shared memory
 }
 
 // The same panel with look-ahead across columns. After column j's winner is known a CTA
@@ -410,9 +700,6 @@ static __global__ void __launch_bounds__(256) lu_panel_cluster_kernel(T *P, long
 // lu_panel_cluster_kernel, so the factors and pivots are identical. The tables have three
 // slots: a CTA may push column j + 1 while another still eliminates with column j - 1's
 // pivot row.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
 template <class T>
 static __global__ void __launch_bounds__(256) lu_panel_cluster_la_kernel(T *P, long long lda, int mrows, int kb, int k0,
                                                                   int rows_per, int tpr, int *ipiv, int *err, T tiny) {

@@ -101,13 +101,18 @@ constexpr int panel_target_rows() {
     return sizeof(T) == 8 ? 64 : 256;
 }
 constexpr size_t kClusterSmem = 224 * 1024;
+// dynamic shared memory of lu_panel_cluster_kernel beside its static tables, for 1024 rows a
+// CTA at most (FP32; FP64 holds fewer by size)
+template <class T>
+constexpr size_t kPanelSmem = kClusterSmem - sizeof(PanelTables<T>);
 inline int cluster_shape(int mrows, size_t row_bytes, size_t extra, int cmax, int target_rows, int &rows_per) {
     const int cmin = (int)(((size_t)mrows * row_bytes + (kClusterSmem - extra) - 1) / (kClusterSmem - extra));
     if (cmin > cmax || cmax == 0) return 0;
     int C = std::max(cmin, std::min(cmax, ceil_div(mrows, target_rows)));
     C = std::max(C, 2);
+    while (C < cmax && ceil_div(mrows, C) * row_bytes > kClusterSmem - extra) C++;  // whole rows round up
     rows_per = ceil_div(mrows, C);
-    return C;
+    return rows_per * row_bytes > kClusterSmem - extra ? 0 : C;
 }
 
 template <class K, class... Args>
@@ -129,27 +134,52 @@ rl_status launch_cluster(K kern, int C, size_t smem, cudaStream_t s, Args... arg
     return RL_OK;
 }
 
-// The LU panel on one cluster when it fits (launched = true), else nothing.
+// The LU panel on one cluster when it fits (launched = true), else nothing. Threads per row
+// and rows per thread follow the rows a CTA holds (256 threads).
+template <class T, int TPR, int RPT>
+rl_status lu_panel_cluster_launch(T *P, long long lda, int mrows, int kb, int k0, int C, int rows_per, int *ipiv, int *err,
+                                  T tiny, cudaStream_t s) {
+    static const int cmax = probe_cluster(lu_panel_cluster_kernel<T, TPR, RPT>, kPanelSmem<T>);
+    if (C > cmax) return RL_ERR_CUDA;
+    return launch_cluster(lu_panel_cluster_kernel<T, TPR, RPT>, C, (size_t)rows_per * (PanelNB<T>::value + 1) * sizeof(T), s, P,
+                          lda, mrows, kb, k0, rows_per, ipiv, err, tiny, wait_ns());
+}
+
 template <class T>
 rl_status lu_panel_cluster(T *P, long long lda, int mrows, int kb, int k0, int *ipiv, int *err, T tiny, cudaStream_t s,
                            bool &launched) {
     constexpr int NB = PanelNB<T>::value;
     launched = false;
-    // look-ahead form (RL_TUNE_PANEL_LOOKAHEAD): three table slots instead of two
-    const bool la = tune(RL_TUNE_PANEL_LOOKAHEAD) != 0;
-    auto kern = la ? lu_panel_cluster_la_kernel<T> : lu_panel_cluster_kernel<T>;
-    static const int cmax_hw = probe_cluster(lu_panel_cluster_kernel<T>, kClusterSmem);
-    static const int cmax_hw_la = probe_cluster(lu_panel_cluster_la_kernel<T>, kClusterSmem);
-    const int cmax = std::min<int>(la ? cmax_hw_la : cmax_hw, (int)tune(RL_TUNE_PANEL_CLUSTER_MAX));
-    const int slots = la ? 3 : 2;
-    const size_t row_bytes = (NB + 1) * sizeof(T), extra = (slots * 16 * NB + slots * NB) * sizeof(T);
+    const size_t row_bytes = (NB + 1) * sizeof(T);
     int rows_per = 0;
-    const int C = cluster_shape(mrows, row_bytes, extra, cmax, panel_target_rows<T>(), rows_per);
+    if (tune(RL_TUNE_PANEL_LOOKAHEAD) != 0) {  // look-ahead form: three table slots
+        auto kern = lu_panel_cluster_la_kernel<T>;
+        static const int cmax_hw = probe_cluster(kern, kClusterSmem);
+        const size_t extra = (3 * 16 * NB + 3 * NB) * sizeof(T);
+        const int C = cluster_shape(mrows, row_bytes, extra, std::min<int>(cmax_hw, (int)tune(RL_TUNE_PANEL_CLUSTER_MAX)),
+                                    panel_target_rows<T>(), rows_per);
+        if (C == 0) return RL_OK;
+        int tpr = 1;  // threads per row: every thread busy when the CTA holds few rows
+        while (tpr < 8 && rows_per * tpr * 2 <= 256) tpr *= 2;
+        RL_TRY(launch_cluster(kern, C, (size_t)rows_per * row_bytes + extra, s, P, lda, mrows, kb, k0, rows_per, tpr, ipiv,
+                              err, tiny));
+        launched = true;
+        return RL_OK;
+    }
+    static const int cmax_hw = probe_cluster(lu_panel_cluster_kernel<T, 1, 1>, kPanelSmem<T>);
+    const int C = cluster_shape(mrows, row_bytes, kClusterSmem - kPanelSmem<T>,
+                                std::min<int>(cmax_hw, (int)tune(RL_TUNE_PANEL_CLUSTER_MAX)), panel_target_rows<T>(), rows_per);
     if (C == 0) return RL_OK;
-    int tpr = 1;  // threads per row: every thread busy when the CTA holds few rows
-    while (tpr < 8 && rows_per * tpr * 2 <= 256) tpr *= 2;
-    RL_TRY(launch_cluster(kern, C, (size_t)rows_per * row_bytes + extra, s, P, lda, mrows, kb, k0, rows_per, tpr, ipiv,
-                          err, tiny));
+    if (rows_per <= 64)
+        RL_TRY((lu_panel_cluster_launch<T, 4, 1>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s)));
+    else if (rows_per <= 128)
+        RL_TRY((lu_panel_cluster_launch<T, 2, 1>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s)));
+    else if (rows_per <= 256)
+        RL_TRY((lu_panel_cluster_launch<T, 1, 1>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s)));
+    else if (rows_per <= 512)
+        RL_TRY((lu_panel_cluster_launch<T, 1, 2>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s)));
+    else if constexpr (sizeof(T) == 4)  // FP64 rows of 520 bytes end at 407
+        RL_TRY((lu_panel_cluster_launch<T, 1, 4>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s)));
     launched = true;
     return RL_OK;
 }
