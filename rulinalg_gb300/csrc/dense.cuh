@@ -1370,282 +1370,328 @@ static __global__ void __launch_bounds__(128) trsm_diag_kernel(const T *D, long 
 }
 
 // ------------------------------------------- few-right-hand-side triangular sweep --
-// op(A) X = Y in place for nrhs <= 8 right-hand sides in ONE launch of at most
-// kSweepCtas CTAs: each CTA takes 64-row blocks of the solution in solve order by an
-// atomic ticket (forward for modes 0 / 1, backward for modes 2 / 3; the modes are those
-// of tri_solve_dev), one after another. A block folds in the contribution of every block
-// solved before it as each one is published (its flag in ctl), overlapping that GEMV
-// work with the blocks still being solved, then solves its diagonal block by
-// substitution (one warp per right-hand side, the multipliers by the diagonal's
-// reciprocals) and publishes its rows. A CTA waits only on tickets taken before its own,
-// by CTAs that are running, so the sweep always progresses; a waiting thread sleeps
-// between polls (other streams' kernels share the SMs), and every wait is bounded by
-// wait_ns (RL_TUNE_WAIT_TIMEOUT_NS; RL_ERR_TIMEOUT). withhold >= 0 is a test setting
-// (RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK): that block is solved but never published, so the
-// waits for it run out. With Dinv (the inverses of the operated diagonal blocks, 64 x 64
-// row-major per block, from diag_inverse_kernel) a block's solve is the product
-// x_b = Dinv_b (y_b - folded sums), 16-term dot products over all 256 threads, instead
-// of the 64-step substitution chain: in FP64 that chain's dependent DFMAs cost ~20 us
-// per block on this part.
+// op(A) X = Y in place for up to 8 right-hand sides in ONE launch: each CTA takes BR-row
+// blocks of the solution in solve order by an atomic ticket (forward for modes 0 / 1,
+// backward for modes 2 / 3; the modes are those of tri_solve_dev). A block folds in every
+// block solved before it as it is published, solves its diagonal block and publishes its
+// rows. The sweep is a chain of n / BR blocks, so the kernel is built around the time from
+// one block's solution to the next one's:
+//   * solutions travel through a separate buffer preset to a NaN pattern that no result has
+//     (all bits set): a reader polls the values themselves, so publishing needs neither a
+//     flag nor a fence, one trip to L2 instead of three;
+//   * the tile of A that meets the awaited block is in registers before the wait, a warp
+//     holding 8 rows and a lane the columns lane + 32 u; the products stay per lane over all
+//     blocks and are reduced once, after the last one;
+//   * the diagonal block is in shared memory from the start: as its inverse (Dinv, from
+//     diag_inverse: the solve is one more BR x BR product) or scaled by its reciprocal
+//     diagonal, so that a substitution step is one shuffle and one multiply-add.
+// BR = 128 for FP32; 64 for FP64, where the products of a tile are bound by the FP64 unit.
+// The form before (64-row blocks, a flag per block behind a fence, the folded sums through
+// shared memory) against this one, per sweep: FP32 with inverses n = 3000 132 and 52 us,
+// n = 4096 220 and 74; n = 8192 with 64 right-hand sides 2216 and 1022; FP64 by substitution
+// n = 4096 992 and 461; FP32 n = 1501 176 (substitution) and 22 (inverses).
+// A CTA waits only on tickets taken before its own, by CTAs that are running, so the sweep
+// always progresses; every wait is bounded by wait_ns (RL_TUNE_WAIT_TIMEOUT_NS,
+// RL_ERR_TIMEOUT), after which the CTA goes on with zeros and publishes, so no later block
+// waits in turn. withhold >= 0 is a test setting (RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK): that
+// block is solved but never published.
 // More than kSweepRhs right-hand sides run as groups of kSweepRhs columns side by side:
-// blockIdx.y is the group, with its own ticket and block flags; groups never wait on one
-// another.
-// Per-launch state, per group g: ctl[g (1 + nb)] = ticket, ctl[g (1 + nb) + 1 + b] =
-// block b published, zeroed by the host.
-constexpr int kSweepRows = 64, kSweepRhs = 8, kSweepCtas = 32, kSweepGroups = 16;
+// blockIdx.y is the group, with its own ticket and solutions.
+// ws: sweep_ws_bytes, all bits set: per group the solutions (n x RW), then the tickets.
+constexpr int kSweepRhs = 8, kSweepGroups = 16;
+template <class T>
+constexpr int sweep_rows() {
+    return sizeof(T) == 4 ? 128 : 64;
+}
 
 // Right-hand-side groups of a sweep over nrhs columns, 0 when the sweep does not take
-// them (more than kSweepGroups groups); ctl words it needs for n rows.
+// them (more than kSweepGroups groups); columns a group holds; bytes of the workspace.
 inline int sweep_groups(int nrhs) {
     const int g = (nrhs + kSweepRhs - 1) / kSweepRhs;
     return g <= kSweepGroups ? g : 0;
 }
-inline int sweep_ctl_words(int n, int nrhs) {
-    return sweep_groups(nrhs) * (1 + (n + kSweepRows - 1) / kSweepRows);
+inline int sweep_width(int nrhs) { return nrhs == 1 ? 1 : kSweepRhs; }
+template <class T>
+inline size_t sweep_ws_bytes(int n, int nrhs) {
+    return (size_t)sweep_groups(nrhs) * ((size_t)n * sweep_width(nrhs) * sizeof(T) + 16);
 }
-template <class T, class TA = T, int RW = kSweepRhs>
-static __global__ void __launch_bounds__(256) trsv_sweep_kernel(const TA *__restrict__ A, long long lda, int n,
-                                                             T *__restrict__ Y, long long ldy, int nrhs, int mode,
-                                                             int *ctl, int *status, T tiny,
+
+__device__ __forceinline__ float sweep_peek(const float *p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return __uint_as_float(v);
+}
+__device__ __forceinline__ double sweep_peek(const double *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return __longlong_as_double((long long)v);
+}
+__device__ __forceinline__ bool sweep_unset(float v) { return __float_as_uint(v) == 0xffffffffu; }
+__device__ __forceinline__ bool sweep_unset(double v) { return (unsigned long long)__double_as_longlong(v) == ~0ull; }
+// The published value at p, waiting for it (bounded; 0 and *fail set when the wait runs out).
+template <class T>
+__device__ __forceinline__ T sweep_get(const T *p, volatile int *fail, unsigned long long limit) {
+    T v = sweep_peek(p);
+    unsigned long long t0 = 0;
+    for (unsigned spin = 0; sweep_unset(v); spin++) {
+        if ((spin & 63u) == 63u) {
+            if (*fail) return T(0);
+            const unsigned long long t = global_ns();
+            if (t0 == 0)
+                t0 = t;
+            else if (t - t0 > limit) {
+                *fail = 1;
+                return T(0);
+            }
+        }
+        v = sweep_peek(p);
+    }
+    return v;
+}
+__device__ __forceinline__ void sweep_put(float *p, float v) {
+    const unsigned u = __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(u == 0xffffffffu ? 0x7fffffffu : u) : "memory");
+}
+__device__ __forceinline__ void sweep_put(double *p, double v) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(u == ~0ull ? 0x7fffffffffffffffull : u) : "memory");
+}
+
+template <class T, int RW>
+struct SweepCfg {
+    static constexpr int BR = sweep_rows<T>(), WARPS = BR / 8, THREADS = 32 * WARPS, CPL = BR / 32, LDD = BR + 1;
+    // the diagonal block; v and the awaited solution, or the warps' column sums (L^T)
+    static constexpr size_t SMEM = sizeof(T) * (BR * LDD + 2 * BR * RW + (size_t)WARPS * BR * RW);
+};
+
+template <class T, class TA, int RW>
+static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_kernel(const TA *__restrict__ A, long long lda,
+                                                             int n, T *__restrict__ Y, long long ldy, int nrhs, int mode,
+                                                             T *ws, int *tickets, int *status, T tiny,
                                                              unsigned long long wait_ns, int withhold,
                                                              const T *__restrict__ Dinv) {
-    constexpr int BR = kSweepRows, LDD = BR + 1;
-    constexpr int FB = sizeof(T) == 4 ? 8 : 2;  // published blocks folded per barrier round
-    __shared__ T Ds[BR * LDD];                  // the diagonal block
-    __shared__ T inv[BR];                        // 1 / d_ii
-    __shared__ T xs[FB * BR * kSweepRhs];        // a round's published solutions, then the folded sums
-    __shared__ int s_t, s_fail, s_m;
+    using cfg = SweepCfg<T, RW>;
+    constexpr int BR = cfg::BR, CPL = cfg::CPL, LDD = cfg::LDD, THREADS = cfg::THREADS, WARPS = cfg::WARPS;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *Ds = reinterpret_cast<T *>(smem_raw);  // BR x LDD: the inverse, or the scaled diagonal block
+    T *v = Ds + BR * LDD;                     // BR x RW: right-hand side minus the folded sums
+    T *xs = v + BR * RW;                      // BR x RW: the awaited block's solution (RW > 1)
+    T *red = xs + BR * RW;                    // WARPS x BR x RW: column sums of the warps (L^T)
+    __shared__ T inv[BR];
+    __shared__ int s_t, s_fail;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nb = (n + BR - 1) / BR;
     const bool fwd = mode <= 1, trans = mode == 3;
-    // this CTA's group of right-hand sides
     Y += (long long)blockIdx.y * kSweepRhs;
     nrhs = min(kSweepRhs, nrhs - (int)blockIdx.y * kSweepRhs);
-    ctl += (long long)blockIdx.y * (1 + nb);
+    ws += (size_t)blockIdx.y * n * RW;
     if (tid == 0) s_fail = 0;
     for (;;) {
         __syncthreads();  // the previous block's shared state is no longer read
-        if (tid == 0) s_t = atomicAdd(ctl, 1);
+        if (tid == 0) s_t = atomicAdd(tickets + blockIdx.y, 1) + 1;  // preset to -1
         __syncthreads();
         if (s_t >= nb) break;
         const int b = fwd ? s_t : nb - 1 - s_t, r0 = b * BR, bs = min(BR, n - r0);
-        // Loads that do not wait on other blocks, issued before the fold: this block's
-        // right-hand-side rows (only this block writes them) and, with Dinv, its row of
-        // the inverted diagonal block; first read after the fold, off the chain.
-        const int rr = tid >> 2, qq = tid & 3;
-        T dpre[16], ypre[2];
+        // The row whose sum this lane ends with (8 rows of the warp, 4 lanes a row) and its
+        // right-hand side; L^T: thread t ends with element t of the block.
+        const int mrow = warp * 8 + (lane >> 2);
+        T y[RW];
+        if (!trans)
+#pragma unroll
+            for (int c = 0; c < RW; c++) y[c] = (mrow < bs && c < nrhs) ? Y[(long long)(r0 + mrow) * ldy + c] : T(0);
         if (Dinv) {
-            const T *Db = Dinv + (long long)b * BR * BR + (long long)rr * BR + qq * 16;
-    #pragma unroll
-            for (int jj = 0; jj < 16; jj++) dpre[jj] = (rr < bs && qq * 16 + jj < bs) ? Db[jj] : T(0);
-    #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int idx = tid + h * 256, i = idx / nrhs, c = idx - i * nrhs;
-                ypre[h] = idx < bs * nrhs ? __ldcg(Y + (long long)(r0 + i) * ldy + c) : T(0);
-            }
+            const T *Db = Dinv + (long long)b * BR * BR;
+            for (int e = tid; e < BR * BR; e += THREADS) Ds[(e / BR) * LDD + e % BR] = Db[e];
         } else {
-    #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int i = lane + 32 * h;
-                ypre[h] = (warp < nrhs && i < bs) ? __ldcg(Y + (long long)(r0 + i) * ldy + warp) : T(0);
+            for (int e = tid; e < BR * BR; e += THREADS) {
+                const int i = e / BR, j = e % BR;
+                T d = T(0);
+                if (i < bs && j < bs) d = T(A[(long long)(r0 + i) * lda + r0 + j]);
+                if (trans)
+                    Ds[j * LDD + i] = d;
+                else
+                    Ds[i * LDD + j] = d;
             }
-        }
-        // the diagonal block and its reciprocal diagonal: no dependence on other blocks
-        if (!Dinv)
-            for (int idx = tid; idx < bs * bs; idx += blockDim.x) {
-                const int i = idx / bs, j = idx - i * bs;
-                Ds[i * LDD + j] = T(A[(long long)(r0 + i) * lda + r0 + j]);
+            __syncthreads();
+            if (tid < BR) {
+                const T d = tid < bs ? Ds[tid * LDD + tid] : T(1);
+                if (mode != 0 && absT(d) < tiny) atomicCAS(status, 0, RL_ERR_DIV_BY_ZERO);
+                inv[tid] = mode == 0 ? T(1) : T(1) / d;
             }
-        __syncthreads();
-        if (tid < bs && !Dinv) {
-            const T d = Ds[tid * LDD + tid];
-            if (mode != 0 && absT(d) < tiny) atomicCAS(status, 0, RL_ERR_DIV_BY_ZERO);
-            inv[tid] = mode == 0 ? T(1) : T(1) / d;
+            __syncthreads();
+            if (mode != 0)
+                for (int e = tid; e < BR * BR; e += THREADS) Ds[(e / BR) * LDD + e % BR] *= inv[e / BR];
         }
-        // thread (row r, quarter q): non-transposed reads A[r][q * 16 + jj] (a thread's 16
-        // columns contiguous), transposed reads A[q * 16 + jj][r] (a warp's rows contiguous)
-        const int r = trans ? (tid & (BR - 1)) : (tid >> 2), q = trans ? (tid >> 6) : (tid & 3);
-        T acc[RW];
-    #pragma unroll
-        for (int c = 0; c < RW; c++) acc[c] = T(0);
+        // the fold: acc[i][c] of row warp 8 + i over this lane's columns; L^T: acc[u][c] of
+        // column lane + 32 u of the block over this warp's 8 rows of the earlier block
+        constexpr int NA = 8;  // rows a warp holds of a tile
+        T acc[(CPL > NA ? CPL : NA)][RW];
+#pragma unroll
+        for (int i = 0; i < (CPL > NA ? CPL : NA); i++)
+#pragma unroll
+            for (int c = 0; c < RW; c++) acc[i][c] = T(0);
         const int nk = fwd ? b : nb - 1 - b;  // blocks solved before this one
-        // The fold, in rounds of up to FB published blocks: thread 0 waits (bounded) for the
-        // round's first block and takes the consecutive published ones after it; their
-        // solutions go to shared memory under one barrier, and the round's products run
-        // without barriers between blocks. (One block per round cost three barriers and a
-        // dependent memory round trip per earlier block: O(b) latencies for block b.) Each
-        // thread adds the blocks in the same order as before, so the sums are unchanged.
-        for (int kk0 = 0; kk0 < nk;) {
-            // FP32, one right-hand side: the A tile of the block about to be waited for is
-            // loaded before the wait (with 8 right-hand sides the extra registers cost more)
-            constexpr bool PRE = sizeof(T) == 4 && RW == 1;
-            T apre[PRE ? 16 : 1];
-            if (PRE) {
-                const int k = fwd ? kk0 : nb - 1 - kk0, c0 = k * BR, ks = min(BR, n - c0);
-    #pragma unroll
-                for (int jj = 0; jj < (PRE ? 16 : 1); jj++) {
-                    const int j = q * 16 + jj;
-                    apre[jj] = (r < bs && j < ks)
-                                   ? T(trans ? A[(long long)(c0 + j) * lda + r0 + r] : A[(long long)(r0 + r) * lda + c0 + j])
-                                   : T(0);
-                }
-            }
-            if (tid == 0 && !s_fail) {
-                const int k = fwd ? kk0 : nb - 1 - kk0;
-                const unsigned long long t0 = global_ns();
-                while (ld_acquire(ctl + 1 + k) == 0) {
-                    if (global_ns() - t0 > wait_ns) {
-                        s_fail = 1;
-                        break;
-                    }
-                    __nanosleep(100);
-                }
-                int m = 1;
-                while (!s_fail && m < FB && kk0 + m < nk &&
-                       ld_acquire(ctl + 1 + (fwd ? kk0 + m : nb - 1 - (kk0 + m))) != 0)
-                    m++;
-                s_m = m;
-            }
-            __syncthreads();
-            if (s_fail) break;
-            const int m = s_m;
-            // rows ks..BR-1 of a short last block are zeroed: they meet a[jj] = 0, and a
-            // stale shared value there could be a NaN (0 * NaN = NaN)
-            for (int idx = tid; idx < m * BR * nrhs; idx += blockDim.x) {
-                const int u = idx / (BR * nrhs), rem = idx - u * (BR * nrhs), i = rem / nrhs, c = rem - i * nrhs;
-                const int k = fwd ? kk0 + u : nb - 1 - (kk0 + u), c0 = k * BR, ks = min(BR, n - c0);
-                xs[(u * BR + i) * kSweepRhs + c] = i < ks ? __ldcg(Y + (long long)(c0 + i) * ldy + c) : T(0);
-            }
-            __syncthreads();
-    #pragma unroll 2
-            for (int u = 0; u < m; u++) {
-                const int k = fwd ? kk0 + u : nb - 1 - (kk0 + u), c0 = k * BR, ks = min(BR, n - c0);
-                T a[16];
-    #pragma unroll
-                for (int jj = 0; jj < 16; jj++) {
-                    const int j = q * 16 + jj;
-                    if (PRE && u == 0)
-                        a[jj] = apre[PRE ? jj : 0];
+        TA cur[NA][CPL], nxt[NA][CPL];
+        auto load = [&](int kk, TA (&t)[NA][CPL]) {
+            const int k = fwd ? kk : nb - 1 - kk, c0 = k * BR, ks = min(BR, n - c0);
+#pragma unroll
+            for (int i = 0; i < NA; i++)
+#pragma unroll
+                for (int u = 0; u < CPL; u++) {
+                    const int wr = warp * 8 + i, lc = lane + 32 * u;
+                    if (trans)
+                        t[i][u] = (wr < ks && lc < bs) ? A[(long long)(c0 + wr) * lda + r0 + lc] : TA(0);
                     else
-                        a[jj] = (r < bs && j < ks)
-                                    ? T(trans ? A[(long long)(c0 + j) * lda + r0 + r] : A[(long long)(r0 + r) * lda + c0 + j])
-                                    : T(0);
+                        t[i][u] = (wr < bs && lc < ks) ? A[(long long)(r0 + wr) * lda + c0 + lc] : TA(0);
                 }
-    #pragma unroll
-                for (int jj = 0; jj < 16; jj++) {
-                    const int j = q * 16 + jj;
-    #pragma unroll
-                    for (int c = 0; c < RW; c++)
-                        if (c < nrhs) acc[c] = fma(a[jj], xs[(u * BR + j) * kSweepRhs + c], acc[c]);
-                }
-            }
-            __syncthreads();  // xs is refilled by the next round
-            kk0 += m;
-        }
-        // sum of the 4 column quarters of each row into xs
-        if (!trans) {
-    #pragma unroll
-            for (int c = 0; c < RW; c++) {
-                acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 1);
-                acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 2);
-            }
-            if (q == 0)
-    #pragma unroll
-                for (int c = 0; c < RW; c++) xs[r * kSweepRhs + c] = acc[c];
-            __syncthreads();
-        } else {
-            for (int qq = 0; qq < 4; qq++) {
-                if (q == qq)
-    #pragma unroll
-                    for (int c = 0; c < RW; c++) xs[r * kSweepRhs + c] = (qq ? xs[r * kSweepRhs + c] : T(0)) + acc[c];
-                __syncthreads();
-            }
-        }
-        if (Dinv) {
-            // x_b = Dinv_b v, v = y_b - folded sums (in xs); thread (row rr, quarter qq)
-    #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int idx = tid + h * 256, i = idx / nrhs, c = idx - i * nrhs;
-                if (idx < bs * nrhs) xs[i * kSweepRhs + c] = ypre[h] - xs[i * kSweepRhs + c];
-            }
-            __syncthreads();
-            T xo[RW];
-    #pragma unroll
-            for (int c = 0; c < RW; c++) xo[c] = T(0);
-    #pragma unroll
-            for (int jj = 0; jj < 16; jj++) {
-                const int j = qq * 16 + jj;
-    #pragma unroll
-                for (int c = 0; c < RW; c++)
-                    if (c < nrhs) xo[c] = fma(dpre[jj], xs[j * kSweepRhs + c], xo[c]);
-            }
-    #pragma unroll
-            for (int c = 0; c < RW; c++) {
-                xo[c] += __shfl_xor_sync(0xffffffffu, xo[c], 1);
-                xo[c] += __shfl_xor_sync(0xffffffffu, xo[c], 2);
-            }
-            if (qq == 0 && rr < bs && !s_fail)
-    #pragma unroll
-                for (int c = 0; c < RW; c++)
-                    if (c < nrhs) __stcg(Y + (long long)(r0 + rr) * ldy + c, xo[c]);
-        }
-        // substitution: warp c solves right-hand side c; lane l holds rows l and l + 32
-        if (!Dinv && warp < nrhs && !s_fail) {
-            const int c = warp;
-            T y[2];
-    #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int i = lane + 32 * h;
-                T v = T(0);
-                if (i < bs) v = ypre[h] - xs[i * kSweepRhs + c];
-                y[h] = v;
-            }
-            if (fwd) {
-                for (int k = 0; k < bs; k++) {
-                    const int h = k >> 5;
-                    T xk = __shfl_sync(0xffffffffu, h ? y[1] : y[0], k & 31) * inv[k];
-                    if (lane == (k & 31)) {
-                        if (h)
-                            y[1] = xk;
-                        else
-                            y[0] = xk;
+        };
+        if (nk > 0) load(0, cur);
+        for (int kk = 0; kk < nk; kk++) {
+            // One right-hand side: the next tile is under way while this one waits. With 8
+            // the sums take those registers.
+            if (RW == 1 && kk + 1 < nk) load(kk + 1, nxt);
+            const int k = fwd ? kk : nb - 1 - kk, c0 = k * BR, ks = min(BR, n - c0);
+            if (RW == 1) {
+                if (!trans) {
+#pragma unroll
+                    for (int u = 0; u < CPL; u++) {
+                        const int lc = lane + 32 * u;
+                        const T x = lc < ks ? sweep_get(ws + c0 + lc, &s_fail, wait_ns) : T(0);
+#pragma unroll
+                        for (int i = 0; i < NA; i++) acc[i][0] = fma(T(cur[i][u]), x, acc[i][0]);
                     }
-    #pragma unroll
-                    for (int hh = 0; hh < 2; hh++) {
-                        const int i = lane + 32 * hh;
-                        if (i > k && i < bs) y[hh] = fma(-Ds[i * LDD + k], xk, y[hh]);
+                } else {
+                    const int wr = warp * 8 + (lane & 7);
+                    const T xl = wr < ks ? sweep_get(ws + c0 + wr, &s_fail, wait_ns) : T(0);
+#pragma unroll
+                    for (int i = 0; i < NA; i++) {
+                        const T x = __shfl_sync(0xffffffffu, xl, i);
+#pragma unroll
+                        for (int u = 0; u < CPL; u++) acc[u][0] = fma(T(cur[i][u]), x, acc[u][0]);
                     }
                 }
             } else {
-                for (int k = bs - 1; k >= 0; k--) {
-                    const int h = k >> 5;
-                    T xk = __shfl_sync(0xffffffffu, h ? y[1] : y[0], k & 31) * inv[k];
-                    if (lane == (k & 31)) {
-                        if (h)
-                            y[1] = xk;
-                        else
-                            y[0] = xk;
-                    }
-    #pragma unroll
-                    for (int hh = 0; hh < 2; hh++) {
-                        const int i = lane + 32 * hh;
-                        if (i < k) y[hh] = fma(-(trans ? Ds[k * LDD + i] : Ds[i * LDD + k]), xk, y[hh]);
+                __syncthreads();  // the last block's solution is no longer read
+                for (int e = tid; e < BR * RW; e += THREADS)
+                    xs[e] = e < ks * RW && e % RW < nrhs ? sweep_get(ws + (size_t)c0 * RW + e, &s_fail, wait_ns) : T(0);
+                __syncthreads();
+#pragma unroll
+                for (int w0 = 0; w0 < (trans ? NA : CPL); w0++) {
+                    T x[RW];
+                    ldv<RW>(xs + (trans ? warp * 8 + w0 : lane + 32 * w0) * RW, x);
+                    if (trans) {
+#pragma unroll
+                        for (int u = 0; u < CPL; u++)
+#pragma unroll
+                            for (int c = 0; c < RW; c++) acc[u][c] = fma(T(cur[w0][u]), x[c], acc[u][c]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < NA; i++)
+#pragma unroll
+                            for (int c = 0; c < RW; c++) acc[i][c] = fma(T(cur[i][w0 & (CPL - 1)]), x[c], acc[i][c]);
                     }
                 }
+                if (kk + 1 < nk) load(kk + 1, cur);
             }
-    #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int i = lane + 32 * h;
-                if (i < bs) __stcg(Y + (long long)(r0 + i) * ldy + c, y[h]);
+            if (RW == 1)
+#pragma unroll
+                for (int i = 0; i < NA; i++)
+#pragma unroll
+                    for (int u = 0; u < CPL; u++) cur[i][u] = nxt[i][u];
+        }
+        // v = y - sums
+        if (!trans) {
+#pragma unroll
+            for (int c = 0; c < RW; c++) {
+                T s8[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) s8[i] = acc[i][c];
+                int row;
+                const T sum = warp_reduce_scatter<8>(s8, lane, row);
+                if ((lane & 3) == 0) v[mrow * RW + c] = y[c] - sum;
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < CPL; u++)
+#pragma unroll
+                for (int c = 0; c < RW; c++) red[((size_t)warp * BR + lane + 32 * u) * RW + c] = acc[u][c];
+            __syncthreads();
+            for (int e = tid; e < BR * RW; e += THREADS) {
+                T sum = T(0);
+#pragma unroll
+                for (int wq = 0; wq < WARPS; wq++) sum += red[(size_t)wq * BR * RW + e];
+                const int i = e / RW, c = e % RW;
+                v[e] = (i < bs && c < nrhs ? Y[(long long)(r0 + i) * ldy + c] : T(0)) - sum;
             }
         }
         __syncthreads();
-        if (tid == 0) {
-            if (s_fail) atomicCAS(status, 0, RL_ERR_TIMEOUT);
-            __threadfence();
-            // published even after a timeout, so no later block waits forever
-            if (b != withhold) st_release(ctl + 1 + b, 1);
+        auto publish = [&](int i, int c, T x) {
+            if (i < bs && c < nrhs) {
+                if (b != withhold) sweep_put(ws + (size_t)(r0 + i) * RW + c, x);
+                Y[(long long)(r0 + i) * ldy + c] = x;
+            }
+        };
+        if (Dinv) {
+            T o[8][RW];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int c = 0; c < RW; c++) o[i][c] = T(0);
+#pragma unroll
+            for (int u = 0; u < CPL; u++) {
+                T x[RW];
+                if constexpr (RW == 1)
+                    x[0] = v[lane + 32 * u];
+                else
+                    ldv<RW>(v + (lane + 32 * u) * RW, x);
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const T d = Ds[(warp * 8 + i) * LDD + lane + 32 * u];
+#pragma unroll
+                    for (int c = 0; c < RW; c++) o[i][c] = fma(d, x[c], o[i][c]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < RW; c++) {
+                T s8[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) s8[i] = o[i][c];
+                int row;
+                const T x = warp_reduce_scatter<8>(s8, lane, row);
+                if ((lane & 3) == 0) publish(mrow, c, x);
+            }
+        } else if (warp < RW) {
+            // substitution with the scaled rows: warp c solves right-hand side c, lane l
+            // holds the rows l + 32 h
+            const int c = warp;
+            T z[CPL];
+#pragma unroll
+            for (int h = 0; h < CPL; h++) z[h] = v[(lane + 32 * h) * RW + c] * inv[lane + 32 * h];
+            if (fwd) {
+#pragma unroll
+                for (int hb = 0; hb < CPL; hb++)  // the 32 unknowns being eliminated
+#pragma unroll 4
+                    for (int q = 0; q < 32; q++) {
+                        const T xk = __shfl_sync(0xffffffffu, z[hb], q);
+#pragma unroll
+                        for (int h = hb; h < CPL; h++)
+                            if (h > hb || lane > q) z[h] = fma(-Ds[(lane + 32 * h) * LDD + hb * 32 + q], xk, z[h]);
+                    }
+            } else {
+#pragma unroll
+                for (int hb = CPL - 1; hb >= 0; hb--)
+#pragma unroll 4
+                    for (int q = 31; q >= 0; q--) {
+                        const T xk = __shfl_sync(0xffffffffu, z[hb], q);
+#pragma unroll
+                        for (int h = 0; h <= hb; h++)
+                            if (h < hb || lane < q) z[h] = fma(-Ds[(lane + 32 * h) * LDD + hb * 32 + q], xk, z[h]);
+                    }
+            }
+#pragma unroll
+            for (int h = 0; h < CPL; h++) publish(lane + 32 * h, c, z[h]);
         }
+        if (tid == 0 && *(volatile int *)&s_fail) atomicCAS(status, 0, RL_ERR_TIMEOUT);
     }
 }
 
@@ -1657,7 +1703,7 @@ static __global__ void __launch_bounds__(256) trsv_sweep_kernel(const TA *__rest
 template <class T, class TA>
 static __global__ void __launch_bounds__(64) diag_inverse_kernel(const TA *__restrict__ A, long long lda, int n, int mode,
                                                              T *__restrict__ Dinv, int *status, T tiny) {
-    constexpr int BR = kSweepRows;
+    constexpr int BR = 64;
     __shared__ T M[BR][BR + 1];  // op(D_b)
     __shared__ T X[BR][BR + 1];  // column j: thread j's solution
     const int b = blockIdx.x, r0 = b * BR, bs = min(BR, n - r0), j = threadIdx.x;
@@ -1690,6 +1736,66 @@ static __global__ void __launch_bounds__(64) diag_inverse_kernel(const TA *__res
     __syncthreads();
     T *out = Dinv + (long long)b * BR * BR;
     for (int idx = j; idx < BR * BR; idx += blockDim.x) out[idx] = X[idx / BR][idx % BR];
+}
+
+// The inverses of 128 x 128 diagonal blocks from those of their 64 x 64 halves (D64, from
+// diag_inverse_kernel): [X1 0; -X2 M X1, X2] for a lower op(D), [X1, -X1 M X2; 0 X2] for an
+// upper one, M the off-diagonal 64 x 64 block. One CTA per block.
+template <class T, class TA>
+static __global__ void __launch_bounds__(256) diag_join_kernel(const TA *__restrict__ A, long long lda, int n, int mode,
+                                                           const T *__restrict__ D64, T *__restrict__ Dinv) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *X = reinterpret_cast<T *>(smem_raw), *Z = X + 64 * 65, *M = Z + 64 * 65, *P = M + 64 * 65;
+    const int b = blockIdx.x, r0 = b * 128, tid = threadIdx.x;
+    const bool lower = mode <= 1;
+    const int nb64 = (n + 63) / 64;
+    for (int e = tid; e < 64 * 64; e += 256) {
+        const int i = e / 64, j = e % 64;
+        X[i * 65 + j] = D64[(long long)(2 * b) * 4096 + e];
+        Z[i * 65 + j] = 2 * b + 1 < nb64 ? D64[(long long)(2 * b + 1) * 4096 + e] : T(0);
+        // op(D) at (64 + i, j) (lower) or (i, 64 + j) (upper)
+        const int oi = r0 + (lower ? 64 + i : i), oj = r0 + (lower ? j : 64 + j);
+        T m = T(0);
+        if (oi < n && oj < n) m = T(mode == 3 ? A[(long long)oj * lda + oi] : A[(long long)oi * lda + oj]);
+        M[i * 65 + j] = m;
+    }
+    __syncthreads();
+    const T *first = lower ? X : Z, *second = lower ? Z : X;  // -second (M first)
+    const int tx = tid & 15, ty = tid >> 4;
+    auto product = [&](const T *l, const T *r, T (&o)[4][4]) {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) o[i][j] = T(0);
+        for (int k = 0; k < 64; k++) {
+            T li[4], rj[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) li[i] = l[(ty + 16 * i) * 65 + k], rj[i] = r[k * 65 + tx + 16 * i];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) o[i][j] = fma(li[i], rj[j], o[i][j]);
+        }
+    };
+    T o[4][4];
+    product(M, first, o);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) P[(ty + 16 * i) * 65 + tx + 16 * j] = o[i][j];
+    __syncthreads();
+    product(second, P, o);
+    T *out = Dinv + (long long)b * 128 * 128;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int r = ty + 16 * i, c = tx + 16 * j;
+            out[(lower ? 64 + r : r) * 128 + (lower ? c : 64 + c)] = -o[i][j];
+            out[(lower ? r : 64 + r) * 128 + (lower ? 64 + c : c)] = T(0);
+            out[r * 128 + c] = X[r * 65 + c];
+            out[(64 + r) * 128 + 64 + c] = Z[r * 65 + c];
+        }
 }
 
 // Row-wise solve X D^T = Y for the rows of Y (m x bs, stride ldy), D lower bs x bs:

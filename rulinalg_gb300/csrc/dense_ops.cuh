@@ -490,6 +490,35 @@ rl_status qr_apply_q_dev(const T *QR, long long lda, int m, int n, const T *tau,
     return RL_OK;
 }
 
+// One launch of the triangular sweep: the 1-wide instance for one right-hand side (the
+// 8-wide one would issue 8 FMAs per element, 7 of them predicated off, each a full issue of
+// the FP64 pipe for T = double). ws as trsv_sweep_kernel takes it.
+template <class T, class TA, int RW>
+rl_status sweep_launch_w(const TA *A, long long lda, int n, const T *Dinv, T *Y, long long ldy, int nrhs, int mode, int *dstatus,
+                         cudaStream_t s, T tiny, void *ws) {
+    using cfg = SweepCfg<T, RW>;
+    auto kern = trsv_sweep_kernel<T, TA, RW>;
+    static int per_sm = 0;
+    static const cudaError_t attr = [&] {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg::SMEM);
+        return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, cfg::THREADS, cfg::SMEM);
+    }();
+    RL_TRY_CUDA(attr);
+    const int groups = sweep_groups(nrhs), nb = ceil_div(n, cfg::BR);
+    T *x = static_cast<T *>(ws);
+    int *tickets = reinterpret_cast<int *>(x + (size_t)groups * n * RW);
+    const dim3 grid(std::min(nb, std::max(1, per_sm) * num_sms()), groups);
+    RL_LAUNCH(kern, grid, cfg::THREADS, cfg::SMEM, s, A, lda, n, Y, ldy, nrhs, mode, x, tickets, dstatus, tiny, wait_ns(),
+              (int)tune(RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK), Dinv);
+    return RL_OK;
+}
+template <class T, class TA>
+rl_status sweep_launch(const TA *A, long long lda, int n, const T *Dinv, T *Y, long long ldy, int nrhs, int mode, int *dstatus,
+                       cudaStream_t s, T tiny, void *ws) {
+    return sweep_width(nrhs) == 1 ? sweep_launch_w<T, TA, 1>(A, lda, n, Dinv, Y, ldy, nrhs, mode, dstatus, s, tiny, ws)
+                                  : sweep_launch_w<T, TA, kSweepRhs>(A, lda, n, Dinv, Y, ldy, nrhs, mode, dstatus, s, tiny, ws);
+}
+
 // Blocked triangular solve op(A) X = Y in place (A n x n, Y n x nrhs).
 // mode 0: unit lower, 1: lower, 2: upper, 3: L^T with L lower. |d_ii| < eps is
 // recorded as RL_ERR_DIV_BY_ZERO in *dstatus. A may be stored in a narrower type TA than
@@ -538,20 +567,10 @@ rl_status tri_solve_dev(const TA *A, long long lda, int n, T *Y, long long ldy, 
         // (trsv_sweep_kernel, groups of kSweepRhs columns side by side). The blocked form
         // below costs two launches per 64-row block, a 64-step chain on a few CTAs and a
         // GEMM whose tiles would be mostly empty.
-        const int nb = ceil_div(n, kSweepRows), words = sweep_ctl_words(n, nrhs);
-        DevBuf<int> ctl;
-        RL_TRY(ctl.alloc(words, s));
-        RL_TRY_CUDA(cudaMemsetAsync(ctl.p, 0, sizeof(int) * words, s));
-        // one right-hand side: the 1-wide instance (the 8-wide one would issue 8 FMAs per
-        // element, 7 of them predicated off, each a full issue of the FP64 pipe for T = double)
-        const dim3 grid(std::min(nb, kSweepCtas), sweep_groups(nrhs));
-        if (nrhs == 1)
-            RL_LAUNCH((trsv_sweep_kernel<T, TA, 1>), grid, 256, 0, s, A, lda, n, Y, ldy, nrhs, mode, ctl.p, dstatus, tiny,
-                      wait_ns(), (int)tune(RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK), (const T *)nullptr);
-        else
-            RL_LAUNCH((trsv_sweep_kernel<T, TA>), grid, 256, 0, s, A, lda, n, Y, ldy, nrhs, mode, ctl.p, dstatus, tiny,
-                      wait_ns(), (int)tune(RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK), (const T *)nullptr);
-        return RL_OK;
+        DevBuf<unsigned char> ws;
+        RL_TRY(ws.alloc(sweep_ws_bytes<T>(n, nrhs), s));
+        RL_TRY_CUDA(cudaMemsetAsync(ws.p, 0xff, sweep_ws_bytes<T>(n, nrhs), s));
+        return sweep_launch<T, TA>(A, lda, n, nullptr, Y, ldy, nrhs, mode, dstatus, s, tiny, ws.p);
     }
     if constexpr (!std::is_same<T, TA>::value) {
         return RL_ERR_INVALID_ARG;  // mixed storage: few right-hand sides only
@@ -587,36 +606,41 @@ rl_status tri_solve_dev(const TA *A, long long lda, int n, T *Y, long long ldy, 
     }
 }
 
-// Inverses of op(A)'s 64 x 64 diagonal blocks, formed in T (ceil(n / 64) row-major
-// 64 x 64 blocks in Dinv; diag_inverse_kernel).
+// Inverses of op(A)'s diagonal blocks of sweep_rows<T>() rows, formed in T (row-major blocks
+// in Dinv, diag_inverse_elems<T>(n) values; zero beyond a partial last block).
+template <class T>
+inline size_t diag_inverse_elems(int n) {
+    return (size_t)ceil_div(n, sweep_rows<T>()) * sweep_rows<T>() * sweep_rows<T>();
+}
 template <class T, class TA>
 rl_status diag_inverse(const TA *A, long long lda, int n, int mode, T *Dinv, int *dstatus, cudaStream_t s, T tiny) {
     if (n <= 0) return RL_OK;
-    RL_LAUNCH((diag_inverse_kernel<T, TA>), ceil_div(n, kSweepRows), 64, 0, s, A, lda, n, mode, Dinv, dstatus, tiny);
+    const int nb64 = ceil_div(n, 64);
+    if constexpr (sweep_rows<T>() == 64) {
+        RL_LAUNCH((diag_inverse_kernel<T, TA>), nb64, 64, 0, s, A, lda, n, mode, Dinv, dstatus, tiny);
+    } else {
+        DevBuf<T> half;
+        RL_TRY(half.alloc((size_t)nb64 * 64 * 64, s));
+        RL_LAUNCH((diag_inverse_kernel<T, TA>), nb64, 64, 0, s, A, lda, n, mode, half.p, dstatus, tiny);
+        const size_t smem = 4 * 64 * 65 * sizeof(T);
+        RL_TRY(set_smem(diag_join_kernel<T, TA>, smem));
+        RL_LAUNCH((diag_join_kernel<T, TA>), ceil_div(n, 128), 256, smem, s, A, lda, n, mode, half.p, Dinv);
+    }
     return RL_OK;
 }
 
 // op(A) Y = Y' for at most kSweepGroups x kSweepRhs right-hand sides in one sweep launch
 // whose block solves are products with the diagonal blocks' inverses Dinv
-// (diag_inverse). ctl: sweep_ctl_words(n, nrhs) zeroed ints (each group's ticket and
-// block flags). More right-hand sides, or a GPU shared with other streams of this
-// library (the serving workers, see tri_solve_dev), take tri_solve_dev's substitution
-// paths instead.
+// (diag_inverse). ws: sweep_ws_bytes<T>(n, nrhs) bytes with all bits set. More right-hand
+// sides, or a GPU shared with other streams of this library (the serving workers, see
+// tri_solve_dev), take tri_solve_dev's substitution paths instead.
 template <class T, class TA>
 rl_status tri_solve_inv_dev(const TA *A, long long lda, int n, const T *Dinv, T *Y, long long ldy, int nrhs, int mode,
-                            int *dstatus, cudaStream_t s, T tiny, int *ctl) {
+                            int *dstatus, cudaStream_t s, T tiny, void *ws) {
     if (sweep_groups(nrhs) == 0 || g_shared_gpu)
         return tri_solve_dev<T, TA>(A, lda, n, Y, ldy, nrhs, mode, dstatus, s, tiny);
     if (n <= 0 || nrhs <= 0) return RL_OK;
-    const int nb = ceil_div(n, kSweepRows);
-    const dim3 grid(std::min(nb, kSweepCtas), sweep_groups(nrhs));
-    if (nrhs == 1)
-        RL_LAUNCH((trsv_sweep_kernel<T, TA, 1>), grid, 256, 0, s, A, lda, n, Y, ldy, nrhs, mode, ctl, dstatus, tiny,
-                  wait_ns(), (int)tune(RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK), Dinv);
-    else
-        RL_LAUNCH((trsv_sweep_kernel<T, TA>), grid, 256, 0, s, A, lda, n, Y, ldy, nrhs, mode, ctl, dstatus, tiny,
-                  wait_ns(), (int)tune(RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK), Dinv);
-    return RL_OK;
+    return sweep_launch<T, TA>(A, lda, n, Dinv, Y, ldy, nrhs, mode, dstatus, s, tiny, ws);
 }
 
 // Solve with factors already on the device. kind 0 = LU (dperm: stored permutation),

@@ -59,11 +59,11 @@ inline rl_status colnorm_dev(const double *V, long long ldv, int n, int nrhs, un
     return RL_OK;
 }
 
-// Inverted 64 x 64 diagonal blocks of the two triangles of an FP32 factor (FP32, formed
-// once) and the sweep flags that use them: the form of RL_TUNE_MIXED_SWEEP_INV.
+// Inverted diagonal blocks of the two triangles of an FP32 factor (FP32, formed once) and
+// the workspace of the sweeps that use them: the form of RL_TUNE_MIXED_SWEEP_INV.
 struct SweepInv {
     const float *D1 = nullptr, *D2 = nullptr;
-    int *ctl = nullptr;  // 2 x sweep_ctl_words(n, nrhs) words, zeroed before each pair of sweeps
+    unsigned char *ws = nullptr;  // 2 x sweep_ws_bytes<float>(n, nrhs), set before each pair of sweeps
 };
 
 // W <- M^-1 W with the FP32 factor (LU: unit L, U, W's rows already in pivoted order;
@@ -76,10 +76,10 @@ inline rl_status precond_solve(const float *F, int n, int kind, float *W, long l
     const float tiny = FLT_MIN;
     const int m1 = kind == RL_KIND_LU ? 0 : 1, m2 = kind == RL_KIND_LU ? 2 : 3;
     if (inv.D1 && sweep_groups(nrhs) > 0) {
-        const int words = sweep_ctl_words(n, nrhs);
-        RL_TRY_CUDA(cudaMemsetAsync(inv.ctl, 0, 2 * words * sizeof(int), s));
-        RL_TRY((tri_solve_inv_dev<float, float>(F, n, n, inv.D1, W, ldw, nrhs, m1, dstatus, s, tiny, inv.ctl)));
-        return tri_solve_inv_dev<float, float>(F, n, n, inv.D2, W, ldw, nrhs, m2, dstatus, s, tiny, inv.ctl + words);
+        const size_t bytes = sweep_ws_bytes<float>(n, nrhs);
+        RL_TRY_CUDA(cudaMemsetAsync(inv.ws, 0xff, 2 * bytes, s));
+        RL_TRY((tri_solve_inv_dev<float, float>(F, n, n, inv.D1, W, ldw, nrhs, m1, dstatus, s, tiny, inv.ws)));
+        return tri_solve_inv_dev<float, float>(F, n, n, inv.D2, W, ldw, nrhs, m2, dstatus, s, tiny, inv.ws + bytes);
     }
     RL_TRY(tri_solve_dev<float>(F, n, n, W, ldw, nrhs, m1, dstatus, s, tiny));
     return tri_solve_dev<float>(F, n, n, W, ldw, nrhs, m2, dstatus, s, tiny);
@@ -94,11 +94,12 @@ struct Minv32 {
     unsigned long long *bits;  // 1 scale
     int *one;                  // device int 1
     int *dstatus;
+    SweepInv inv;              // the sweeps' form with inverted diagonal blocks, or none
     rl_status apply(const double *src, double *dst, cudaStream_t s) const {
         RL_TRY(colnorm_dev(src, 1, n, 1, bits, s));
         const int g = std::min(4 * num_sms(), ceil_div(n, 256));
         RL_LAUNCH(scale_to_f32_kernel, g, 256, 0, s, src, 1LL, n, 1, bits, (const int *)nullptr, w32, 1LL);
-        RL_TRY(precond_solve(F, n, RL_KIND_CHOLESKY, w32, 1, 1, dstatus, s));
+        RL_TRY(precond_solve(F, n, RL_KIND_CHOLESKY, w32, 1, 1, dstatus, s, inv));
         RL_TRY_CUDA(cudaMemsetAsync(dst, 0, n * sizeof(double), s));
         RL_LAUNCH(update_x_kernel, g, 256, 0, s, dst, 1LL, w32, 1LL, n, 1, bits, one);
         return RL_OK;
@@ -110,7 +111,7 @@ struct Minv32 {
 // working precision the preconditioner lets GMRES-IR converge where the FP32-applied form
 // stalls (Carson & Higham's analysis assumes it; on kappa = 1e8 systems with geometric
 // singular values, n = 1024, a CPU model of both took 121 against 313 GMRES iterations).
-// The block solves use the FP64 inverses of the two triangles' 64 x 64 diagonal blocks
+// The block solves use the FP64 inverses of the two triangles' diagonal blocks
 // (D1 for L, D2 for U or L^T), formed once by init().
 struct Minv {
     const float *F;
@@ -118,14 +119,13 @@ struct Minv {
     const int *rows;  // LU: the row map of the pivots (pivots_to_rows)
     int *dstatus;
     DevBuf<double> D1, D2;
-    DevBuf<int> ctl;  // the two sweeps' ticket and block flags
+    DevBuf<unsigned char> ws;  // the two sweeps' solutions and tickets
     int mode1() const { return kind == RL_KIND_LU ? 0 : 1; }
     int mode2() const { return kind == RL_KIND_LU ? 2 : 3; }
     rl_status init(cudaStream_t s) {
-        const size_t blocks = (size_t)ceil_div(n, kSweepRows) * kSweepRows * kSweepRows;
-        RL_TRY(D1.alloc(blocks, s));
-        RL_TRY(D2.alloc(blocks, s));
-        RL_TRY(ctl.alloc(2 * (size_t)(1 + ceil_div(n, kSweepRows)), s));
+        RL_TRY(D1.alloc(diag_inverse_elems<double>(n), s));
+        RL_TRY(D2.alloc(diag_inverse_elems<double>(n), s));
+        RL_TRY(ws.alloc(2 * sweep_ws_bytes<double>(n, 1), s));
         RL_TRY((diag_inverse<double, float>(F, n, n, mode1(), D1.p, dstatus, s, FLT_MIN)));
         return diag_inverse<double, float>(F, n, n, mode2(), D2.p, dstatus, s, FLT_MIN);
     }
@@ -135,10 +135,10 @@ struct Minv {
             RL_TRY(gather_rows<double>(src, 1, dst, 1, n, 1, rows, s));
         else
             RL_TRY_CUDA(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        const int words = 1 + ceil_div(n, kSweepRows);
-        RL_TRY_CUDA(cudaMemsetAsync(ctl.p, 0, 2 * words * sizeof(int), s));
-        RL_TRY((tri_solve_inv_dev<double, float>(F, n, n, D1.p, dst, 1, 1, mode1(), dstatus, s, tiny, ctl.p)));
-        return tri_solve_inv_dev<double, float>(F, n, n, D2.p, dst, 1, 1, mode2(), dstatus, s, tiny, ctl.p + words);
+        const size_t bytes = sweep_ws_bytes<double>(n, 1);
+        RL_TRY_CUDA(cudaMemsetAsync(ws.p, 0xff, 2 * bytes, s));
+        RL_TRY((tri_solve_inv_dev<double, float>(F, n, n, D1.p, dst, 1, 1, mode1(), dstatus, s, tiny, ws.p)));
+        return tri_solve_inv_dev<double, float>(F, n, n, D2.p, dst, 1, 1, mode2(), dstatus, s, tiny, ws.p + bytes);
     }
 };
 
@@ -351,7 +351,7 @@ struct MixedFactor {
         F64 = nullptr, ipiv64 = nullptr, rows64 = nullptr, Dinv = nullptr;
     }
 
-    size_t dinv_elems() const { return (size_t)ceil_div(n, kSweepRows) * kSweepRows * kSweepRows; }
+    size_t dinv_elems() const { return diag_inverse_elems<float>(n); }
 
     size_t bytes() const {
         size_t b = (size_t)n * n * sizeof(float) + 2 * (size_t)n * sizeof(int);
@@ -473,11 +473,11 @@ struct MixedFactor {
         unsigned long long *bn_b = nb.p, *rn_b = nb.p + nrhs, *xn_b = nb.p + 2 * nrhs;
         RL_TRY_CUDA(cudaMemsetAsync(dstatus.p, 0, 2 * sizeof(int), s));
         SweepInv inv;
-        DevBuf<int> sweep_ctl;
+        DevBuf<unsigned char> sweep_ws;
         if (tune(RL_TUNE_MIXED_SWEEP_INV) && sweep_groups(nrhs) > 0 && n > CTA_NMAX && !g_shared_gpu) {
             RL_TRY(ensure_dinv(dstatus.p, s));
-            RL_TRY(sweep_ctl.alloc(2 * (size_t)sweep_ctl_words(n, nrhs), s));
-            inv = SweepInv{Dinv, Dinv + dinv_elems(), sweep_ctl.p};
+            RL_TRY(sweep_ws.alloc(2 * sweep_ws_bytes<float>(n, nrhs), s));
+            inv = SweepInv{Dinv, Dinv + dinv_elems(), sweep_ws.p};
         }
         std::vector<int> act(nrhs + 1, 1);
         RL_TRY_CUDA(cudaMemcpyAsync(active.p, act.data(), act.size() * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -677,7 +677,19 @@ inline rl_status lstsq_mixed(const double *A, long long lda, int m, int n, const
     RL_TRY(qr_factor_dev<float>(Q32.p, n, m, n, n, tau32.p, s));
     RL_LAUNCH(upper_to_lower_t_kernel, (int)std::min<long long>(8 * num_sms(), ((long long)n * n + 255) / 256), 256, 0, s,
               Q32.p, (long long)n, n, L.p);
-    Minv32 M{L.p, n, w32.p, bits.p + 2, one.p, dstatus.p};
+    // 4 to 20 sweeps follow: inverted diagonal blocks, as in the mixed single-system solver
+    DevBuf<float> Dinv;
+    DevBuf<unsigned char> sweep_ws;
+    SweepInv inv;
+    if (tune(RL_TUNE_MIXED_SWEEP_INV) && n > CTA_NMAX && !g_shared_gpu) {
+        const size_t de = diag_inverse_elems<float>(n);
+        RL_TRY(Dinv.alloc(2 * de, s));
+        RL_TRY(sweep_ws.alloc(2 * sweep_ws_bytes<float>(n, 1), s));
+        RL_TRY((diag_inverse<float, float>(L.p, n, n, 1, Dinv.p, dstatus.p, s, FLT_MIN)));
+        RL_TRY((diag_inverse<float, float>(L.p, n, n, 3, Dinv.p + de, dstatus.p, s, FLT_MIN)));
+        inv = SweepInv{Dinv.p, Dinv.p + de, sweep_ws.p};
+    }
+    Minv32 M{L.p, n, w32.p, bits.p + 2, one.p, dstatus.p, inv};
     GemvT At{partial.p, chunks, rows_per};
     const int gv = std::min(4 * num_sms(), ceil_div(n, 256));
     // x0 = (R^T R)^-1 A^T b
