@@ -1842,78 +1842,120 @@ static __global__ void extract_v_kernel(const T *P, long long lda, int mrows, in
     V[idx] = r > c ? P[(long long)r * lda + c] : (r == c ? T(1) : T(0));
 }
 
-// Partial Gram matrices of the reflector block V (mrows x kb, row stride kb, kb <= 64):
-// CTA c sums V[r]^T V[r] over its chunk of rows into part[c] (64 x 64). A plain GEMM of
-// this 64 x 64 product over thousands of rows is one tile, one CTA, one long K loop.
-constexpr int kGramRows = 256;  // rows per chunk
+// W[i][j] = V[j][i] for i < kb, j < cols (V with row stride kb).
 template <class T>
-static __global__ void __launch_bounds__(256) gram_partial_kernel(const T *__restrict__ V, int mrows, int kb,
+static __global__ void v_transpose_kernel(const T *V, int kb, int cols, T *W, long long ldw) {
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (long long)kb * cols) return;
+    const int i = (int)(idx / cols), j = (int)(idx - (long long)i * cols);
+    W[(long long)i * ldw + j] = V[(long long)j * kb + i];
+}
+
+// Partial Gram matrices of the reflector block V (mrows x kb, row stride kb, kb <= 64): CTA
+// (c, t) sums V[r]^T V[r] over chunk c of the rows for tile t of the 10 16 x 16 tiles on or
+// above the diagonal, into part[c] (64 x 64; the tiles below are not written). FP64 is bound
+// by the SMs' FP64 units, so the product is cut into enough CTAs for all of them: 256-row
+// chunks with whole 64 x 64 products took 267 us at m = 1201.
+constexpr int kGramRows = 128;  // rows per chunk
+template <class T>
+static __global__ void __launch_bounds__(128) gram_partial_kernel(const T *__restrict__ V, int mrows, int kb,
                                                                   T *__restrict__ part) {
-    __shared__ T Vs[32][64];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    __shared__ T Va[64][17], Vb[64][17];
+    int t = blockIdx.y, ti = 0;  // tile row ti, column tj >= ti
+    while (t >= 4 - ti) t -= 4 - ti++;
+    const int tj = ti + t, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    if (tj * 16 >= kb) return;
     const int rbeg = blockIdx.x * kGramRows, rend = min(mrows, rbeg + kGramRows);
-    T acc[4][4];
+    T acc0 = T(0), acc1 = T(0);
+    for (int r0 = rbeg; r0 < rend; r0 += 64) {
 #pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = T(0);
-    for (int r0 = rbeg; r0 < rend; r0 += 32) {
-        for (int idx = tid; idx < 32 * 64; idx += 256) {
-            const int r = idx >> 6, c = idx & 63;
-            Vs[r][c] = (r0 + r < rend && c < kb) ? V[(long long)(r0 + r) * kb + c] : T(0);
+        for (int e = tid; e < 64 * 16; e += 128) {
+            const int r = e >> 4, c = e & 15;
+            Va[r][c] = (r0 + r < rend && ti * 16 + c < kb) ? V[(long long)(r0 + r) * kb + ti * 16 + c] : T(0);
+            Vb[r][c] = (r0 + r < rend && tj * 16 + c < kb) ? V[(long long)(r0 + r) * kb + tj * 16 + c] : T(0);
         }
         __syncthreads();
-#pragma unroll 4
-        for (int r = 0; r < 32; r++) {
-            T va[4], vb[4];
-#pragma unroll
-            for (int a = 0; a < 4; a++) va[a] = Vs[r][4 * ty + a];
-#pragma unroll
-            for (int b = 0; b < 4; b++) vb[b] = Vs[r][4 * tx + b];
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) acc[a][b] = fma(va[a], vb[b], acc[a][b]);
+        const int lim = min(64, rend - r0);
+#pragma unroll 8
+        for (int r = 0; r < lim; r++) {
+            const T b = Vb[r][tx];
+            acc0 = fma(Va[r][ty], b, acc0);
+            acc1 = fma(Va[r][ty + 8], b, acc1);
         }
         __syncthreads();
     }
-    T *out = part + (size_t)blockIdx.x * 64 * 64;
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) out[(4 * ty + a) * 64 + 4 * tx + b] = acc[a][b];
+    T *out = part + (size_t)blockIdx.x * 64 * 64 + (ti * 16) * 64 + tj * 16 + tx;
+    out[ty * 64] = acc0;
+    out[(ty + 8) * 64] = acc1;
 }
 
-// T factor of H_0 ... H_{kb-1} = I - V T V^T (upper triangular, kb x kb): the Gram
-// matrix Gm = V^T V is the sum of the nparts partial Gram matrices (added in part order),
-// then T[j][j] = tau_j, T[0:j, j] = -tau_j T[0:j, 0:j] Gm[0:j, j], all in shared memory.
+// T factor of H_0 ... H_{kb-1} = I - V T V^T (upper triangular, kb x kb): the Gram matrix
+// Gm = V^T V is the sum of the partial Gram matrices (added in part order). The four 16 x 16
+// diagonal blocks of T follow from T[j][j] = tau_j, T[0:j, j] = -tau_j T[0:j, 0:j] Gm[0:j, j],
+// a warp each; two diagonal blocks join by T12 = -T1 (Gm12 T2), 16 and 16 columns, then 32 and
+// 32. The recursion over all 64 columns at once was a chain of 64 dot products of up to 63
+// terms in one thread each: 121 us in FP64 and 46 us in FP32, this 49 and 29.
 template <class T>
 static __global__ void __launch_bounds__(256) larft_kernel(const T *part, int nparts, const T *tau, int kb, T *Tm) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T (*G)[65] = reinterpret_cast<T (*)[65]>(smem_raw);  // 64 x 65 each
     T (*Ts)[65] = G + 64;
-    __shared__ T w[64];
-    const int t = threadIdx.x;
-    for (int idx = t; idx < 64 * 64; idx += blockDim.x) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    for (int idx = t; idx < 64 * 64; idx += 256) {
+        const int i = idx >> 6, j = idx & 63;
         T sum = T(0);
-        for (int c = 0; c < nparts; c++) sum += part[(size_t)c * 64 * 64 + idx];
-        G[idx >> 6][idx & 63] = sum;
-        Ts[idx >> 6][idx & 63] = T(0);
+        if (i < j && j < kb)
+            for (int c = 0; c < nparts; c++) sum += part[(size_t)c * 64 * 64 + idx];
+        G[i][j] = sum;
+        Ts[i][j] = T(0);
     }
     __syncthreads();
-    for (int j = 0; j < kb; j++) {
-        const T tj = tau[j];
-        if (t < j) {
-            T s = T(0);
-            for (int q = t; q < j; q++) s = fma(Ts[t][q], G[q][j], s);
-            w[t] = -tj * s;
+    if (warp < 4) {
+        const int o = warp * 16;
+        for (int j = 0; j < 16 && o + j < kb; j++) {
+            const T tj = tau[o + j];
+            if (lane < j) {
+                T s = T(0);
+                for (int q = lane; q < j; q++) s = fma(Ts[o + lane][o + q], G[o + q][o + j], s);
+                Ts[o + lane][o + j] = -tj * s;
+            }
+            if (lane == j) Ts[o + j][o + j] = tj;
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    for (int h = 16; h <= 32; h *= 2) {  // T12 of the pairs of h x h blocks
+        const int pairs = 32 / h, total = pairs * h * h;
+        T p[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {  // P = Gm12 T2 (T2 upper triangular)
+            const int idx = t + e * 256;
+            p[e] = T(0);
+            if (idx < total) {
+                const int o = idx / (h * h) * 2 * h, i = idx / h % h, j = idx % h;
+                for (int q = 0; q <= j; q++) p[e] = fma(G[o + i][o + h + q], Ts[o + h + q][o + h + j], p[e]);
+            }
         }
         __syncthreads();
-        if (t < j) Ts[t][j] = w[t];
-        if (t == 0) Ts[j][j] = tj;
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int idx = t + e * 256;
+            if (idx < total) G[idx / (h * h) * 2 * h + idx / h % h][idx / (h * h) * 2 * h + h + idx % h] = p[e];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 4; e++) {  // T12 = -T1 P (T1 upper triangular)
+            const int idx = t + e * 256;
+            if (idx < total) {
+                const int o = idx / (h * h) * 2 * h, i = idx / h % h, j = idx % h;
+                T s = T(0);
+                for (int q = i; q < h; q++) s = fma(Ts[o + i][o + q], G[o + q][o + h + j], s);
+                Ts[o + i][o + h + j] = -s;
+            }
+        }
         __syncthreads();
     }
-    for (int idx = t; idx < kb * kb; idx += blockDim.x) Tm[idx] = Ts[idx / kb][idx % kb];
+    for (int idx = t; idx < kb * kb; idx += 256) Tm[idx] = Ts[idx / kb][idx % kb];
 }
 
 // Identity-like start for first_k_columns: Q (m x k) = I[:, 0:k].

@@ -357,11 +357,23 @@ rl_status block_t_factor(const T *V, int mrows, int kb, const T *tau, T *part, i
                          cudaStream_t s) {
     const int nparts = ceil_div(mrows, kGramRows);
     if (nparts > max_parts) return RL_ERR_INVALID_ARG;
-    RL_LAUNCH(gram_partial_kernel<T>, nparts, 256, 0, s, V, mrows, kb, part);
+    RL_LAUNCH(gram_partial_kernel<T>, dim3(nparts, 10), 128, 0, s, V, mrows, kb, part);
     const size_t smem = 2 * 64 * 65 * sizeof(T);
     RL_TRY(set_smem(larft_kernel<T>, smem));
     RL_LAUNCH(larft_kernel<T>, 1, 256, smem, s, part, nparts, tau, kb, Tm);
     return RL_OK;
+}
+
+// X (mrows x q) -= V W with V the mrows x kb reflectors of a panel, W kb x q. FP64: the
+// unit-triangular rows of V apart, whose few entries would send the first row of tiles of the
+// tensor-core product to the FP64 unit (its accuracy check is per tile, gemm_f64tc.cuh).
+template <class T>
+rl_status block_update(const T *V, int mrows, int kb, const T *W, T *X, long long ldx, int q, cudaStream_t s) {
+    const int head = sizeof(T) == 8 && mrows > kb ? kb : 0;
+    if (head)
+        RL_TRY((gemm<T, false, false>(head, q, kb, T(-1), V, kb, W, q, T(1), X, ldx, s)));
+    return gemm<T, false, false>(mrows - head, q, kb, T(-1), V + (long long)head * kb, kb, W, q, T(1), X + (long long)head * ldx,
+                                 ldx, s);
 }
 
 // Blocked Householder QR with compact-WY trailing updates; nrefl reflectors
@@ -412,7 +424,7 @@ rl_status qr_factor_dev(T *A, long long lda, int m, int n, int nrefl, T *tau, cu
         T *A2 = P + kb;
         RL_TRY((gemm<T, true, false>(kb, n2, mrows, T(1), V.p, kb, A2, lda, T(0), W1.p, n2, s)));
         RL_TRY((gemm<T, true, false>(kb, n2, kb, T(1), Tm.p, kb, W1.p, n2, T(0), W2.p, n2, s)));
-        RL_TRY((gemm<T, false, false>(mrows, n2, kb, T(-1), V.p, kb, W2.p, n2, T(1), A2, lda, s)));
+        RL_TRY(block_update<T>(V.p, mrows, kb, W2.p, A2, lda, n2, s));
     }
     int err = 0;
     RL_TRY_CUDA(cudaMemcpyAsync(&err, &sync.p->err, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -421,7 +433,10 @@ rl_status qr_factor_dev(T *A, long long lda, int m, int n, int nrefl, T *tau, cu
 }
 
 // Q[:, 0:k] of a compact QR (HouseholderComposition::first_k_columns): reflector panels
-// applied in reverse order to I[:, 0:k], each as Q2 -= V (T (V^T Q2)).
+// applied in reverse order to I[:, 0:k], each as Q2 -= V (T (V^T Q2)). The rows and columns of
+// a panel's own reflectors are still those of the identity, Q2 = [I 0; 0 Q3] (Q3 an identity
+// too for the first panel applied), so V^T Q2 = [V1^T, V2^T Q3] takes a product for the
+// columns of Q3 only.
 template <class T>
 rl_status qr_first_k_dev(const T *QR, long long lda, int m, int n, const T *tau, int k, T *Q, long long ldq,
                          cudaStream_t s) {
@@ -445,9 +460,13 @@ rl_status qr_first_k_dev(const T *QR, long long lda, int m, int n, const T *tau,
         RL_LAUNCH(extract_v_kernel<T>, (int)((mkb + 255) / 256), 256, 0, s, P, lda, mrows, kb, V.p);
         RL_TRY(block_t_factor<T>(V.p, mrows, kb, tau + k0, Gp.p, max_parts, Tm.p, s));
         T *Q2 = Q + (long long)k0 * ldq + k0;
-        RL_TRY((gemm<T, true, false>(kb, nc, mrows, T(1), V.p, kb, Q2, ldq, T(0), W1.p, nc, s)));
+        const int copied = k0 + kb == jmax ? nc : kb;  // columns of V^T Q2 that are columns of V^T
+        RL_LAUNCH(v_transpose_kernel<T>, ceil_div((long long)kb * copied, 256), 256, 0, s, V.p, kb, copied, W1.p, (long long)nc);
+        if (copied < nc)
+            RL_TRY((gemm<T, true, false>(kb, nc - kb, mrows - kb, T(1), V.p + (long long)kb * kb, kb,
+                                         Q2 + (long long)kb * ldq + kb, ldq, T(0), W1.p + kb, nc, s)));
         RL_TRY((gemm<T, false, false>(kb, nc, kb, T(1), Tm.p, kb, W1.p, nc, T(0), W2.p, nc, s)));
-        RL_TRY((gemm<T, false, false>(mrows, nc, kb, T(-1), V.p, kb, W2.p, nc, T(1), Q2, ldq, s)));
+        RL_TRY(block_update<T>(V.p, mrows, kb, W2.p, Q2, ldq, nc, s));
     }
     return RL_OK;
 }
@@ -485,7 +504,7 @@ rl_status qr_apply_q_dev(const T *QR, long long lda, int m, int n, const T *tau,
             RL_TRY((gemm<T, true, false>(kb, q, kb, T(1), Tm.p, kb, W1.p, q, T(0), W2.p, q, s)));
         else
             RL_TRY((gemm<T, false, false>(kb, q, kb, T(1), Tm.p, kb, W1.p, q, T(0), W2.p, q, s)));
-        RL_TRY((gemm<T, false, false>(mrows, q, kb, T(-1), V.p, kb, W2.p, q, T(1), X2, ldx, s)));
+        RL_TRY(block_update<T>(V.p, mrows, kb, W2.p, X2, ldx, q, s));
     }
     return RL_OK;
 }

@@ -206,6 +206,79 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
     }
 }
 
+// The same product for few outputs: 32 x 32 (FP32) or 16 x 16 (FP64) outputs per CTA of 128
+// threads, K in chunks of 32 through shared memory, so that a product of a few 64 x 64 tiles
+// (T^T W and W = V^T A of a Householder block, the solves' small updates) spreads over the
+// SMs: on this part a 64 x 64 x 64 FP64 product is 70 us of one SM's FP64 unit. T^T W of a
+// 1201 x 499 QR (64 x n2 x 64) went from ~270 to 8 us, in FP32 (2999 x 1501) from 17 to 4. Sums
+// run over k in order, as in gemm_kernel.
+template <class T>
+constexpr int gemm_few_tile() {
+    return sizeof(T) == 4 ? 32 : 16;
+}
+template <class T, bool TA, bool TB>
+static __global__ void __launch_bounds__(128)
+    gemm_few_kernel(int m, int n, int k, T alpha, const T *__restrict__ A, long long lda, const T *__restrict__ B, long long ldb,
+                    T beta, T *__restrict__ C, long long ldc) {
+    constexpr int BT = gemm_few_tile<T>(), BK = 32, R = BT * BT / 128, RS = 128 / BT;  // outputs a thread: rows ty + RS i
+    __shared__ T As[BK][BT + 1], Bs[BK][BT + 1];
+    const int tid = threadIdx.x, tx = tid % BT, ty = tid / BT;
+    const int row0 = blockIdx.y * BT, col0 = blockIdx.x * BT;
+    constexpr int PER = BK * BT / 128;
+    T ra[PER], rb[PER], acc[R];
+#pragma unroll
+    for (int i = 0; i < R; i++) acc[i] = T(0);
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int e = 0; e < PER; e++) {
+            const int idx = tid + e * 128;
+            const int ia = TA ? idx % BT : idx / BK, pa = TA ? idx / BT : idx % BK;
+            ra[e] = (row0 + ia < m && k0 + pa < k)
+                        ? (TA ? A[(long long)(k0 + pa) * lda + row0 + ia] : A[(long long)(row0 + ia) * lda + k0 + pa])
+                        : T(0);
+            const int jb = TB ? idx / BK : idx % BT, pb = TB ? idx % BK : idx / BT;
+            rb[e] = (col0 + jb < n && k0 + pb < k)
+                        ? (TB ? B[(long long)(col0 + jb) * ldb + k0 + pb] : B[(long long)(k0 + pb) * ldb + col0 + jb])
+                        : T(0);
+        }
+    };
+    load(0);
+    for (int k0 = 0; k0 < k; k0 += BK) {
+#pragma unroll
+        for (int e = 0; e < PER; e++) {
+            const int idx = tid + e * 128;
+            if (TA)
+                As[idx / BT][idx % BT] = ra[e];
+            else
+                As[idx % BK][idx / BK] = ra[e];
+            if (TB)
+                Bs[idx % BK][idx / BK] = rb[e];
+            else
+                Bs[idx / BT][idx % BT] = rb[e];
+        }
+        __syncthreads();
+        if (k0 + BK < k) load(k0 + BK);
+        const int lim = min(BK, k - k0);
+#pragma unroll 8
+        for (int p = 0; p < lim; p++) {
+            const T b = Bs[p][tx];
+#pragma unroll
+            for (int i = 0; i < R; i++) acc[i] = fma(As[p][ty + RS * i], b, acc[i]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const int gi = row0 + ty + RS * i, gj = col0 + tx;
+        if (gi < m && gj < n) {
+            T *cp = C + (long long)gi * ldc + gj;
+            T v = alpha * acc[i];
+            if (beta != T(0)) v = fma(beta, *cp, v);
+            *cp = v;
+        }
+    }
+}
+
 // Launches C = alpha * op(A) op(B) + beta * C on `stream`. FP32 products with at least
 // a 128 x 128 tile's worth of C and K >= 256 go to the tcgen05 kernel (gemm_tc.cuh).
 // A product with fewer tiles than SMs and a long K (the V^T A2 and V^T V products of a
@@ -225,6 +298,17 @@ rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T 
             int ks = 1;
             if (!LOWER && tc_tiles < sms / 2 && k >= 1024) ks = std::min({16, ceil_div(sms, tc_tiles), k / 256});
             return sgemm_tc<TA, TB>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, LOWER, stream, ks);
+        }
+    }
+    if constexpr (!LOWER) {
+        // Few outputs, short K: small tiles over the SMs. gemm_kernel's tiles take BM BN K
+        // multiply-adds of one SM each; here every SM takes a share.
+        constexpr int BT = gemm_few_tile<T>();
+        const bool tc = std::is_same<T, double>::value && dgemm_tc_eligible(m, n, k);
+        if (tiles * 4 <= sms && k <= 512 && !tc) {
+            RL_LAUNCH((gemm_few_kernel<T, TA, TB>), dim3(ceil_div(n, BT), ceil_div(m, BT)), 128, 0, stream, m, n, k, alpha, A, lda,
+                      B, ldb, beta, C, ldc);
+            return RL_OK;
         }
     }
     DevBuf<unsigned char> ws;
