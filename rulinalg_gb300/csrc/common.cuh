@@ -39,6 +39,11 @@ inline cudaStream_t resolve_stream(void *s) { return s ? static_cast<cudaStream_
         if (rl_s_ != RL_OK) return rl_s_;     \
     } while (0)
 
+// Kernels in the headers are static, one per translation unit. A host function that keeps
+// something about a kernel in a static local (its shared-memory attribute, its cluster size) is
+// static as well: an inline one would share that local over the units while the kernel that
+// each of them launches is its own.
+
 // Launch bookkeeping: every kernel launch in the library goes through this macro so
 // that rl_launch_count() and the launch-error check stay exact.
 #define RL_LAUNCH(kernel, grid, block, smem, stream, ...)                  \

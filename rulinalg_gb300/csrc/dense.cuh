@@ -1174,7 +1174,7 @@ static __global__ void __launch_bounds__(256) laswp_kernel(T *A, long long lda, 
 
 // Launch of laswp_kernel over the columns outside [c_skip0, c_skip1).
 template <class T>
-rl_status laswp(T *A, long long lda, int ncols, int c_skip0, int c_skip1, const int *ipiv, int j0, int j1,
+static rl_status laswp(T *A, long long lda, int ncols, int c_skip0, int c_skip1, const int *ipiv, int j0, int j1,
                 cudaStream_t s) {
     const int nother = ncols - (c_skip1 - c_skip0);
     if (nother <= 0 || j1 <= j0) return RL_OK;
@@ -1264,7 +1264,7 @@ static __global__ void __launch_bounds__(kRowMapThreads) pivots_to_rows_kernel(c
     }
 }
 
-inline rl_status pivots_to_rows(const int *ipiv, int n, int *rows, uint64_t *stored, cudaStream_t s) {
+static inline rl_status pivots_to_rows(const int *ipiv, int n, int *rows, uint64_t *stored, cudaStream_t s) {
     DevBuf<int2> moves;
     RL_TRY(moves.alloc((size_t)ceil_div(n, kSwapBlock) * 2 * kSwapBlock, s));
     const size_t smem = n <= kRowMapSmem ? sizeof(int) * n : 0;

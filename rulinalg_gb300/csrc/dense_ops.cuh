@@ -137,7 +137,7 @@ rl_status launch_cluster(K kern, int C, size_t smem, cudaStream_t s, Args... arg
 // The LU panel on one cluster when it fits (launched = true), else nothing. Threads per row
 // and rows per thread follow the rows a CTA holds (256 threads).
 template <class T, int TPR, int RPT>
-rl_status lu_panel_cluster_launch(T *P, long long lda, int mrows, int kb, int k0, int C, int rows_per, int *ipiv, int *err,
+static rl_status lu_panel_cluster_launch(T *P, long long lda, int mrows, int kb, int k0, int C, int rows_per, int *ipiv, int *err,
                                   T tiny, cudaStream_t s) {
     static const int cmax = probe_cluster(lu_panel_cluster_kernel<T, TPR, RPT>, kPanelSmem<T>);
     if (C > cmax) return RL_ERR_CUDA;
@@ -146,7 +146,7 @@ rl_status lu_panel_cluster_launch(T *P, long long lda, int mrows, int kb, int k0
 }
 
 template <class T>
-rl_status lu_panel_cluster(T *P, long long lda, int mrows, int kb, int k0, int *ipiv, int *err, T tiny, cudaStream_t s,
+static rl_status lu_panel_cluster(T *P, long long lda, int mrows, int kb, int k0, int *ipiv, int *err, T tiny, cudaStream_t s,
                            bool &launched) {
     constexpr int NB = PanelNB<T>::value;
     launched = false;
@@ -186,7 +186,7 @@ rl_status lu_panel_cluster(T *P, long long lda, int mrows, int kb, int k0, int *
 
 // The Householder panel on one cluster when it fits (launched = true), else nothing.
 template <class T>
-rl_status qr_panel_cluster(T *P, long long lda, int mrows, int kb, T *tau, cudaStream_t s, bool &launched) {
+static rl_status qr_panel_cluster(T *P, long long lda, int mrows, int kb, T *tau, cudaStream_t s, bool &launched) {
     constexpr int NB = PanelNB<T>::value;
     launched = false;
     auto kern = qr_panel_cluster_kernel<T>;
@@ -513,7 +513,7 @@ rl_status qr_apply_q_dev(const T *QR, long long lda, int m, int n, const T *tau,
 // 8-wide one would issue 8 FMAs per element, 7 of them predicated off, each a full issue of
 // the FP64 pipe for T = double). ws as trsv_sweep_kernel takes it.
 template <class T, class TA, int RW>
-rl_status sweep_launch_w(const TA *A, long long lda, int n, const T *Dinv, T *Y, long long ldy, int nrhs, int mode, int *dstatus,
+static rl_status sweep_launch_w(const TA *A, long long lda, int n, const T *Dinv, T *Y, long long ldy, int nrhs, int mode, int *dstatus,
                          cudaStream_t s, T tiny, void *ws) {
     using cfg = SweepCfg<T, RW>;
     auto kern = trsv_sweep_kernel<T, TA, RW>;

@@ -574,7 +574,7 @@ struct DgemmTcTiles {  // the tiles left to the FP64 unit
 // names the tiles that the caller still has to compute, on the same stream, with buffers that
 // live in `ws`.
 template <int BN>
-rl_status dgemm_tc_launch(int m, int n, int nkc, const CUtensorMap &mA, const __nv_bfloat16 *Sb, int kp,
+static rl_status dgemm_tc_launch(int m, int n, int nkc, const CUtensorMap &mA, const __nv_bfloat16 *Sb, int kp,
                           const unsigned *keyA, const unsigned *keyB, double alpha, double beta, double *C, long long ldc,
                           bool lower, int *flags, double *part, int ks, cudaStream_t s) {
     using namespace tc64;

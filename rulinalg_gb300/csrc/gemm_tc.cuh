@@ -358,7 +358,7 @@ __global__ void splitk_reduce_kernel(int m, int n, int nz, T alpha, const T *__r
 // ksplit > 1 (not with `lower`) runs K in that many slices at once into partial tiles,
 // added in slice order afterwards: for products with few output tiles and a long K.
 template <bool TA, bool TB>
-rl_status sgemm_tc(int m, int n, int k, float alpha, const float *A, long long lda, const float *B, long long ldb,
+static rl_status sgemm_tc(int m, int n, int k, float alpha, const float *A, long long lda, const float *B, long long ldb,
                    float beta, float *C, long long ldc, bool lower, cudaStream_t s, int ksplit = 1) {
     static const cudaError_t attr =
         cudaFuncSetAttribute(sgemm_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
@@ -409,7 +409,7 @@ rl_status sgemm_tc(int m, int n, int k, float alpha, const float *A, long long l
 }
 
 // Reads and clears the sticky timeout word (synchronises the stream).
-inline rl_status sgemm_tc_status(cudaStream_t s) {
+static inline rl_status sgemm_tc_status(cudaStream_t s) {
     int *err = nullptr;
     RL_TRY_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&err), g_sgemm_tc_err));
     int h = 0;
