@@ -4,6 +4,7 @@
 // default stream and copy the results back. Matrices with n <= 512 are factored by one
 // CTA (factor_cta.cuh); larger ones by the blocked multi-CTA path (dense.cuh + GEMM).
 #include <algorithm>
+#include <cstring>
 #include <type_traits>
 #include <vector>
 
@@ -325,6 +326,39 @@ rl_status qr_lstsq_host(size_t m, size_t n, T *a, size_t lda, const T *b, T *x) 
     return r;
 }
 
+// A calling thread's page-locked buffer for one system of at most kSmallN rows (33 KB, kept
+// until the thread ends): the kernel reads and writes it in place, so that a small solve is
+// one launch and one wait, without allocations or copies.
+struct SmallStage {
+    void *p = nullptr;
+    ~SmallStage() {
+        if (p) cudaFreeHost(p);
+    }
+    rl_status get(void *&out) {
+        if (!p) RL_TRY_CUDA(cudaHostAlloc(&p, (kSmallN * kSmallN + kSmallN) * sizeof(double) + 16, cudaHostAllocDefault));
+        out = p;
+        return RL_OK;
+    }
+};
+
+template <class T>
+rl_status matrix_solve_small(size_t n, T *a, size_t lda, T *b, cudaStream_t s) {
+    static thread_local SmallStage stage;
+    void *p = nullptr;
+    RL_TRY(stage.get(p));
+    volatile int *st = static_cast<int *>(p);
+    T *sa = reinterpret_cast<T *>(static_cast<unsigned char *>(p) + 16), *sb = sa + n * n;
+    *st = 0;
+    for (size_t i = 0; i < n; i++) memcpy(sa + i * n, a + i * lda, n * sizeof(T));
+    memcpy(sb, b, n * sizeof(T));
+    RL_LAUNCH(small_lu_kernel<T>, 1, 256, 0, s, sa, (int)n, (int)n, (int *)nullptr, sb, const_cast<int *>(st), Eps<T>::value);
+    RL_TRY_CUDA(cudaStreamSynchronize(s));
+    if (*st != RL_OK) return *st;
+    for (size_t i = 0; i < n; i++) memcpy(a + i * lda, sa + i * n, n * sizeof(T));
+    memcpy(b, sb, n * sizeof(T));
+    return RL_OK;
+}
+
 // Matrix::solve (impl_mat.rs:354-356): decompose + one solve, factors stay on the GPU.
 template <class T>
 rl_status matrix_solve_host(size_t n, T *a, size_t lda, T *b) {
@@ -332,6 +366,7 @@ rl_status matrix_solve_host(size_t n, T *a, size_t lda, T *b) {
     if (!a || !b || lda < n || !fits_int(n)) return RL_ERR_INVALID_ARG;
     RL_TRY(ensure_device());
     cudaStream_t s = cudaStreamPerThread;
+    if (n <= kSmallN) return matrix_solve_small<T>(n, a, lda, b, s);
     DevBuf<T> dA, dB;
     DevBuf<int> dpiv, rows;
     DevBuf<uint64_t> dperm;

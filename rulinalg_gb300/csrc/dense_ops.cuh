@@ -12,6 +12,7 @@
 #include "dense.cuh"
 #include "gemm.cuh"
 #include "mixed.cuh"
+#include "small.cuh"
 
 namespace rl {
 
@@ -32,15 +33,44 @@ inline rl_status set_smem(K kern, size_t bytes) {
     return RL_OK;
 }
 
-// One CTA factors a matrix with n <= CTA_NMAX; kind 0 LU (ipiv out), 1 Cholesky.
+// Sizes up to which one CTA factors a single matrix (the batched kernels keep CTA_NMAX). A
+// panel of a cluster costs ~1.5 us a column whatever its height; one CTA's FP64 unit makes
+// 2 multiply-adds a cycle, so FP64 leaves it beyond the 64 rows of small_lu_kernel (LU, host
+// call, one CTA against blocked: n = 64 416 and 196 us, 128 951 and 400, 512 16,016 and
+// 1,798). FP32 LU crosses at n = 256 (536 and 515; 512: 1,827 and 1,083), FP32 Cholesky
+// between 384 and 512 (547 and 636; 919 and 793), FP64 Cholesky at once with its diagonal
+// blocks on small_chol_kernel.
+template <class T>
+constexpr int one_cta_lu() {
+    return sizeof(T) == 8 ? kSmallN : 240;
+}
+template <class T>
+constexpr int one_cta_chol() {
+    return sizeof(T) == 8 ? kSmallN : 448;
+}
+
+// One CTA factors a matrix with n <= CTA_NMAX; kind 0 LU (ipiv out), 1 Cholesky. The status
+// word is set, not read.
+template <class T>
+rl_status factor_small_async(T *A, long long lda, int n, int kind, int *ipiv, int *st, cudaStream_t s, T tiny) {
+    if (n <= kSmallN) {
+        if (kind)
+            RL_LAUNCH(small_chol_kernel<T>, 1, 256, 0, s, A, (int)lda, n, st, tiny);
+        else
+            RL_LAUNCH(small_lu_kernel<T>, 1, 256, 0, s, A, (int)lda, n, ipiv, (T *)nullptr, st, tiny);
+        return RL_OK;
+    }
+    const size_t smem = cta_smem_bytes<T>();
+    RL_TRY(set_smem(factor_one_kernel<T>, smem));
+    RL_LAUNCH(factor_one_kernel<T>, 1, CTA_THREADS, smem, s, A, (int)lda, n, kind, ipiv, st, tiny);
+    return RL_OK;
+}
 template <class T>
 rl_status factor_small(T *A, long long lda, int n, int kind, int *ipiv, cudaStream_t s, T tiny = Eps<T>::value) {
     DevBuf<int> st;
     RL_TRY(st.alloc(1, s));
     RL_TRY_CUDA(cudaMemsetAsync(st.p, 0, sizeof(int), s));
-    const size_t smem = cta_smem_bytes<T>();
-    RL_TRY(set_smem(factor_one_kernel<T>, smem));
-    RL_LAUNCH(factor_one_kernel<T>, 1, CTA_THREADS, smem, s, A, (int)lda, n, kind, ipiv, st.p, tiny);
+    RL_TRY(factor_small_async<T>(A, lda, n, kind, ipiv, st.p, s, tiny));
     return read_status<T>(st.p, s);
 }
 
@@ -227,7 +257,7 @@ template <class T>
 rl_status lu_factor_dev(T *A, long long lda, int n, int *ipiv, cudaStream_t s, T tiny = Eps<T>::value) {
     NvtxRange nvtx_("rl.lu.factor");
     if (n <= 0) return RL_OK;
-    if (n <= CTA_NMAX) return factor_small<T>(A, lda, n, 0, ipiv, s, tiny);
+    if (n <= one_cta_lu<T>()) return factor_small<T>(A, lda, n, 0, ipiv, s, tiny);
     constexpr int NB = PanelNB<T>::value;
     int Gmax, rp;
     panel_geometry<T>(n, Gmax, rp);
@@ -310,7 +340,7 @@ template <class T>
 rl_status chol_factor_dev(T *A, long long lda, int n, cudaStream_t s, T tiny = Eps<T>::value) {
     NvtxRange nvtx_("rl.cholesky.factor");
     if (n <= 0) return RL_OK;
-    if (n <= CTA_NMAX) return factor_small<T>(A, lda, n, 1, nullptr, s, tiny);
+    if (n <= one_cta_chol<T>()) return factor_small<T>(A, lda, n, 1, nullptr, s, tiny);
     if constexpr (outer_nb<T>() > 0) {
         constexpr int NBO = outer_nb<T>();
         DevBuf<T> Linv, T21;
@@ -336,19 +366,24 @@ rl_status chol_factor_dev(T *A, long long lda, int n, cudaStream_t s, T tiny = E
         return read_status<T>(st.p, s);
     }
     constexpr int NB = PanelNB<T>::value;
+    // One sticky status word, read once: a block that fails leaves finite garbage behind for
+    // the launches after it.
+    DevBuf<int> st;
+    RL_TRY(st.alloc(1, s));
+    RL_TRY_CUDA(cudaMemsetAsync(st.p, 0, sizeof(int), s));
     for (int k0 = 0; k0 < n; k0 += NB) {
         const int kb = std::min(NB, n - k0), mrows = n - k0;
         T *P = A + (long long)k0 * lda + k0;
-        RL_TRY(factor_small<T>(P, lda, kb, 1, nullptr, s, tiny));
+        RL_TRY(factor_small_async<T>(P, lda, kb, 1, nullptr, st.p, s, tiny));
         const int m2 = mrows - kb;
         if (m2 > 0) {
-            RL_LAUNCH(trsm_right_lt_kernel<T>, ceil_div(m2, 128), 128, 0, s, P, lda, kb, P + (long long)kb * lda, lda,
+            RL_LAUNCH(trsm_right_lt_kernel<T>, ceil_div(m2, kTrsmCols), 128, 0, s, P, lda, kb, P + (long long)kb * lda, lda,
                       m2);
             T *L21 = P + (long long)kb * lda;
             RL_TRY((gemm<T, false, true, true>(m2, m2, kb, T(-1), L21, lda, L21, lda, T(1), L21 + kb, lda, s)));
         }
     }
-    return RL_OK;
+    return read_status<T>(st.p, s);
 }
 
 // Tm of a reflector block V (mrows x kb): partial Gram matrices, then the T recursion.
@@ -671,7 +706,12 @@ rl_status factor_solve_dev(const T *F, long long lda, int n, int kind, const uin
     DevBuf<int> st;
     RL_TRY(st.alloc(1, s));
     RL_TRY_CUDA(cudaMemsetAsync(st.p, 0, sizeof(int), s));
-    if (n <= CTA_NMAX) {
+    // Up to CTA_NMAX rows a CTA per right-hand side, or one sweep for a single one from the
+    // size where its chain of blocks is shorter (host calls, FP64 n = 96 128 and 113 us, 512
+    // 602 and 226; FP32 n = 256 122 and 120, 512 191 and 147). Many right-hand sides stay a
+    // CTA each (inverse, FP64 n = 512: 1,470 and 1,667 us).
+    const bool sweep = nrhs == 1 && !g_shared_gpu && n > (sizeof(T) == 8 ? 88 : 256);
+    if (n <= CTA_NMAX && !sweep) {
         const size_t smem = cta_smem_bytes<T>();
         RL_TRY(set_smem(solve_one_kernel<T>, smem));
         RL_LAUNCH(solve_one_kernel<T>, nrhs, CTA_THREADS, smem, s, F, (int)lda, n, kind, kind ? nullptr : dperm, B, ldb,
