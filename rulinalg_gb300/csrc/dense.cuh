@@ -13,6 +13,16 @@
 
 namespace rl {
 
+// a / p from r = 1 / p: the rounded product corrected by its exact remainder (Markstein, IBM
+// J. Res. Dev. 34, 1990).
+template <class T>
+__device__ __forceinline__ T quotient(T a, T p, T r) {
+    const T q = a * r;
+    const T e = fma(-q, p, a);
+    const T c = fma(e, r, q);
+    return e == e ? c : q;  // an infinite product has no remainder
+}
+
 // Largest panel width of the blocked paths.
 template <class T>
 struct PanelNB {
@@ -984,110 +994,167 @@ static __global__ void __launch_bounds__(256) qr_panel_kernel(T *P, long long ld
     }
 }
 
-// Householder panel on one thread-block cluster (up to 16 CTAs): qr_panel_kernel's
-// algorithm with the two cross-CTA sums per column (sigma, then u = A^T v) exchanged on
-// chip. Each CTA pushes its partial sums (and x0, from the CTA holding row j) into every
-// CTA's tables by remote shared-memory stores before a cluster barrier; after it every
-// CTA adds the C partials from its own tables in rank order, so all compute the same tau
-// and u with no remote read on the critical path. v_r = a_rj / v0 is formed once per
-// row (it was formed again for every column of the u sums). The tables are written for
-// column j + 1 only after the barrier that every CTA reaches once it has read them for
-// column j. A column with sigma = 0 still passes the second barrier, so every CTA runs
-// the same barrier sequence.
+// Householder panel on one thread-block cluster (up to 16 CTAs), one exchange per column. With
+// x the column below row j, the sums s_c = sum_r x_r a_rc for c >= j give everything at once:
+// sigma = s_j and, as v = (1, x / v0), u_c = a_jc + s_c / v0. Per column:
+//   1. the warps take up to 8 columns each, a lane the rows lane + 32 i, and reduce them
+//      together (warp_reduce_scatter: 9 additions for 8 columns; in FP64 an addition is 64
+//      cycles of a scheduler's unit, like a multiply-add);
+//   2. every partial sum, and row j from the CTA that holds it, goes to all CTAs by st.async,
+//      counted on their mbarriers (no cluster barrier, no CTA barrier);
+//   3. each CTA adds the partials in rank order, one warp forms tau and 1 / v0, and w_c =
+//      tau u_c is shared;
+//   4. a_rc -= v_r w_c, `tpr` threads per row; v takes the column's place.
+// Tables are double-buffered by column parity: a CTA pushes column j + 2 only after it has all
+// partials of column j + 1, which the others push after their last read of column j's tables.
+// Two exchanges behind cluster barriers (sigma, then u) and a butterfly per column sum took
+// 302 us per 64-column panel of a 2999 x 1501 FP32 QR, this 163; the whole 1201 x 499 FP64 QR
+// with its thin Q (8 panels) went from 11.05 to 9.0 ms. Bound by a column's chain: two CTA
+// barriers, the exchange, and tau's square root and divisions in one thread.
+template <class T>
+struct QrTables {
+    T tab[2][16][64];  // partial sums of column c from CTA g
+    T rowj[2][64];
+    T w[64];
+    T tau, v0, inv_v0, diag;
+    int zero;
+    uint64_t full[2];
+    int fail[2];  // a wait ran out, by column parity
+};
+
+__device__ __forceinline__ void st_async(uint32_t dst, float v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst), "r"(__float_as_uint(v)),
+                 "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void st_async(uint32_t dst, double v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
+                 "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
+}
+
+// Sums of N columns c = first, first + 8, ... of a warp, pushed to every CTA's tables.
+template <class T, int N>
+__device__ __forceinline__ void qr_dots(const T *R, int LDR, int rbeg, int nr, int j, int first, int kb, const T *rowj, int C, int g,
+                                        uint32_t tab_a, uint32_t row_a, uint32_t bar_a) {
+    const int lane = threadIdx.x & 31;
+    T acc[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) acc[k] = T(0);
+    for (int r = rbeg + lane; r < nr; r += 32) {
+        const T *row = R + (size_t)r * LDR;
+        const T x = row[j];
+#pragma unroll
+        for (int k = 0; k < N; k++)
+            if (first + 8 * k < kb) acc[k] = fma(x, row[first + 8 * k], acc[k]);
+    }
+    int k;
+    const T sum = warp_reduce_scatter<N>(acc, lane, k);
+    constexpr int PER = 32 / N;  // lanes that hold a column's sum
+    const int c = first + 8 * k;
+    if (c >= kb) return;
+    for (int to = lane % PER; to < C; to += PER) {
+        const uint32_t bar = cluster_addr(bar_a, to);
+        st_async(cluster_addr(tab_a + (unsigned)((g * 64 + c) * sizeof(T)), to), sum, bar);
+        if (rowj) st_async(cluster_addr(row_a + (unsigned)(c * sizeof(T)), to), rowj[c], bar);
+    }
+}
+
 template <class T>
 static __global__ void __launch_bounds__(256) qr_panel_cluster_kernel(T *P, long long lda, int mrows, int kb,
-                                                              int rows_per, T *tau) {
+                                                              int rows_per, int tpr, T *tau, int *err,
+                                                              unsigned long long wait_ns) {
     namespace cg = cooperative_groups;
-    constexpr int NB = PanelNB<T>::value;
-    constexpr int LDR = NB + 1;
-    constexpr int CMAX = 16;
+    constexpr int NB = PanelNB<T>::value, LDR = NB + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *R = reinterpret_cast<T *>(smem_raw);  // rows_per x LDR
-    T *vb = R + (size_t)rows_per * LDR;      // rows_per: this column's v for the owned rows
-    T *u = vb + rows_per;                    // NB: this column's u
-    T *up_tab = u + NB;                      // CMAX x NB: every CTA's partial of u
-    T *sig_tab = up_tab + CMAX * NB;         // CMAX: every CTA's partial of sigma
-    T *x0_slot = sig_tab + CMAX;             // 1: x0 = a_jj from the CTA holding row j
-    __shared__ T s_red[8];
+    __shared__ __align__(16) QrTables<T> S;
     cg::cluster_group cluster = cg::this_cluster();
     const int C = (int)cluster.num_blocks(), g = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nw = blockDim.x >> 5;
     const int r0 = g * rows_per, r1 = min(mrows, r0 + rows_per), nr = max(0, r1 - r0);
-    for (int idx = tid; idx < nr * kb; idx += blockDim.x) {
+    const int q = tid & (tpr - 1), grp = tid / tpr, G = 256 / tpr, rpt = (rows_per + G - 1) / G;
+    for (int idx = tid; idx < nr * kb; idx += 256) {
         const int r = idx / kb, c = idx - r * kb;
         R[r * LDR + c] = P[(long long)(r0 + r) * lda + c];
     }
-    __syncthreads();
+    if (tid == 0) {
+        S.fail[0] = S.fail[1] = 0;
+        cl_mbar_init(&S.full[0], 1);
+        cl_mbar_init(&S.full[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    cluster.sync();
+    bool bad = false;
     for (int j = 0; j < kb; j++) {
-        // (1) sigma partial over rows > j, pushed (with x0) to every CTA
-        T sp = T(0);
-        for (int r = max(j + 1 - r0, 0) + tid; r < nr; r += blockDim.x) {
-            const T v = R[r * LDR + j];
-            sp = fma(v, v, sp);
+        const int slot = j & 1, ncol = (kb - j + 7) / 8, rbeg = max(j + 1 - r0, 0);
+        const bool hold = j >= r0 && j < r1;
+        if (tid == 0) cl_mbar_expect(&S.full[slot], (unsigned)((kb - j) * (C + 1) * sizeof(T)));
+        // 1, 2. partial sums of columns j + warp, j + warp + 8, ...
+        {
+            const T *rj = hold ? R + (size_t)(j - r0) * LDR : nullptr;
+            const uint32_t ta = smem_addr(&S.tab[slot][0][0]), ra = smem_addr(&S.rowj[slot][0]), ba = smem_addr(&S.full[slot]);
+            const int first = j + warp;
+            if (ncol > 4)
+                qr_dots<T, 8>(R, LDR, rbeg, nr, j, first, kb, rj, C, g, ta, ra, ba);
+            else if (ncol > 2)
+                qr_dots<T, 4>(R, LDR, rbeg, nr, j, first, kb, rj, C, g, ta, ra, ba);
+            else
+                qr_dots<T, 2>(R, LDR, rbeg, nr, j, first, kb, rj, C, g, ta, ra, ba);
         }
-        sp = warp_sum(sp);
-        if (lane == 0) s_red[warp] = sp;
-        __syncthreads();
-        if (tid < C) {
-            T t = T(0);
-            for (int w = 0; w < nw; w++) t += s_red[w];
-            *cluster.map_shared_rank(sig_tab + g, tid) = t;
-            if (j >= r0 && j < r1) *cluster.map_shared_rank(x0_slot, tid) = R[(j - r0) * LDR + j];
-        }
-        cluster.sync();
-        // sigma over the CTAs in rank order (lane q holds CTA q's partial)
-        if (warp == 0) {
-            T sigma = lane < C ? sig_tab[lane] : T(0);
-            sigma = warp_sum(sigma);
-            if (lane == 0) s_red[0] = sigma;
-        }
-        __syncthreads();
-        const T sigma = s_red[0];
-        const T x0 = *x0_slot;
-        if (sigma == T(0)) {  // already a multiple of e1: tau = 0, nothing changes
-            if (g == 0 && tid == 0) tau[j] = T(0);
-            cluster.sync();
-            continue;
-        }
-        const T x_norm = sqrt(x0 * x0 + sigma);
-        const T v0 = x0 > T(0) ? x0 + x_norm : x0 - x_norm;
-        const T two = T(2);
-        const T t = two * v0 * v0 / (v0 * v0 + sigma);
-        if (g == 0 && tid == 0) tau[j] = t;
-        // v of the owned rows below the diagonal (stored into the panel by the update)
-        for (int r = max(j + 1 - r0, 0) + tid; r < nr; r += blockDim.x) vb[r] = R[r * LDR + j] / v0;
-        __syncthreads();
-        // (2) u_c partial = sum_r v_r a[r][c] for c >= j over owned rows r >= j, pushed
-        for (int c = j + warp; c < kb; c += nw) {
-            T acc = T(0);
-            for (int r = max(j - r0, 0) + lane; r < nr; r += 32) {
-                const T vr = (r0 + r == j) ? T(1) : vb[r];
-                acc = fma(vr, R[r * LDR + c], acc);
+        if (!cl_mbar_wait(&S.full[slot], (j >> 1) & 1, wait_ns)) S.fail[slot] = 1;
+        // 3. warp 0: sigma, tau, 1 / v0
+        const int c = j + tid;
+        T sc = T(0);
+        if (c < kb)
+            for (int k = 0; k < C; k++) sc += S.tab[slot][k][c];  // CTAs in rank order
+        if (tid == 0) {
+            const T sigma = sc, x0 = S.rowj[slot][j];
+            S.zero = sigma == T(0);  // already a multiple of e1: tau = 0, nothing changes
+            T t = T(0), inv = T(0), d = x0, v0 = T(1);
+            if (!S.zero) {
+                const T x_norm = sqrt(x0 * x0 + sigma);
+                v0 = x0 > T(0) ? x0 + x_norm : x0 - x_norm;
+                t = T(2) * v0 * v0 / (v0 * v0 + sigma);
+                inv = T(1) / v0;
+                d = x0 - t * (x0 + sigma * inv);
             }
-            acc = __shfl_sync(0xffffffffu, warp_sum(acc), 0);  // lane 0's sum, in every lane
-            if (lane < C) *cluster.map_shared_rank(up_tab + g * NB + c, lane) = acc;
-        }
-        cluster.sync();
-        if (tid >= j && tid < kb) {
-            T a = T(0);
-            for (int q = 0; q < C; q++) a += up_tab[q * NB + tid];
-            u[tid] = a;
+            S.tau = t;
+            S.v0 = v0;
+            S.inv_v0 = inv;
+            S.diag = d;
+            if (g == 0) tau[j] = t;
         }
         __syncthreads();
-        // (3) a[r][c] += (-tau v_r) u_c for c > j; the diagonal becomes x0 - tau u_j and
-        // v[1..] stays below it
-        for (int r = max(j - r0, 0) + tid; r < nr; r += blockDim.x) {
-            T *row = R + r * LDR;
-            const bool diag = (r0 + r == j);
-            const T vr = diag ? T(1) : vb[r];
-            const T sc = -t * vr;
-            for (int c = j + 1; c < kb; c++) row[c] = fma(sc, u[c], row[c]);
-            row[j] = diag ? x0 - t * u[j] : vr;
+        if (*(volatile int *)&S.fail[slot]) {
+            bad = true;
+            break;
+        }
+        if (!S.zero) {
+            const T inv = S.inv_v0;
+            if (c < kb) S.w[c] = S.tau * (S.rowj[slot][c] + sc * inv);
+            __syncthreads();
+            // 4. a_rc -= v_r w_c for c > j (v_j = 1); the diagonal, and v below it
+            for (int k = 0; k < rpt; k++) {  // the same count in every thread
+                const int r = grp + k * G;
+                const bool mine = r < nr && r0 + r >= j, diag = r0 + r == j;
+                T *row = R + (size_t)(mine ? r : 0) * LDR;
+                const T v = mine ? (diag ? T(1) : quotient(row[j], S.v0, inv)) : T(0);
+                __syncwarp();
+                if (mine) {
+                    const int first = j + 1 + ((q - j - 1) & (tpr - 1));
+#pragma unroll 4
+                    for (int cc = first; cc < kb; cc += tpr) row[cc] = fma(-v, S.w[cc], row[cc]);
+                    if (q == 0) row[j] = diag ? S.diag : v;
+                }
+            }
         }
         __syncthreads();
     }
-    for (int idx = tid; idx < nr * kb; idx += blockDim.x) {
+    if (bad) {
+        if (tid == 0) atomicCAS(err, 0, RL_ERR_TIMEOUT);
+    }
+    for (int idx = tid; idx < nr * kb; idx += 256) {
         const int r = idx / kb, c = idx - r * kb;
         P[(long long)(r0 + r) * lda + c] = R[r * LDR + c];
     }

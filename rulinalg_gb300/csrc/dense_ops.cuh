@@ -216,17 +216,20 @@ static rl_status lu_panel_cluster(T *P, long long lda, int mrows, int kb, int k0
 
 // The Householder panel on one cluster when it fits (launched = true), else nothing.
 template <class T>
-static rl_status qr_panel_cluster(T *P, long long lda, int mrows, int kb, T *tau, cudaStream_t s, bool &launched) {
+static rl_status qr_panel_cluster(T *P, long long lda, int mrows, int kb, T *tau, int *err, cudaStream_t s, bool &launched) {
     constexpr int NB = PanelNB<T>::value;
+    constexpr size_t cap = kClusterSmem - sizeof(QrTables<T>);
     launched = false;
     auto kern = qr_panel_cluster_kernel<T>;
-    static const int cmax_hw = probe_cluster(kern, kClusterSmem);
+    static const int cmax_hw = probe_cluster(kern, cap);
     const int cmax = std::min<int>(cmax_hw, (int)tune(RL_TUNE_PANEL_CLUSTER_MAX));
-    const size_t row_bytes = (NB + 2) * sizeof(T), extra = (NB + 16 * NB + 16 + 1) * sizeof(T);
+    const size_t row_bytes = (NB + 1) * sizeof(T);
     int rows_per = 0;
-    const int C = cluster_shape(mrows, row_bytes, extra, cmax, panel_target_rows<T>(), rows_per);
+    const int C = cluster_shape(mrows, row_bytes, kClusterSmem - cap, cmax, panel_target_rows<T>(), rows_per);
     if (C == 0) return RL_OK;
-    RL_TRY(launch_cluster(kern, C, (size_t)rows_per * row_bytes + extra, s, P, lda, mrows, kb, rows_per, tau));
+    int tpr = 1;  // threads per row: every thread busy when the CTA holds few rows
+    while (tpr < 8 && rows_per * tpr * 2 <= 256) tpr *= 2;
+    RL_TRY(launch_cluster(kern, C, (size_t)rows_per * row_bytes, s, P, lda, mrows, kb, rows_per, tpr, tau, err, wait_ns()));
     launched = true;
     return RL_OK;
 }
@@ -445,7 +448,7 @@ rl_status qr_factor_dev(T *A, long long lda, int m, int n, int nrefl, T *tau, cu
         T *P = A + (long long)k0 * lda + k0;
         T *tk = tau + k0;
         bool clustered = false;
-        RL_TRY(qr_panel_cluster<T>(P, lda, mrows, kb, tk, s, clustered));
+        RL_TRY(qr_panel_cluster<T>(P, lda, mrows, kb, tk, &sync.p->err, s, clustered));
         if (!clustered) {
             if (k0 > 0) RL_TRY_CUDA(cudaMemsetAsync(&sync.p->ctr, 0, sizeof(unsigned), s));
             void *args[] = {&P, &lda, (void *)&mrows, (void *)&kb, &rows_per, &tk, &part.p, &x0buf.p, &sync.p, &wns};

@@ -16,15 +16,6 @@ namespace rl {
 
 constexpr int kSmallN = 64;
 
-// a / p from r = 1 / p: the rounded product corrected by its exact remainder.
-template <class T>
-__device__ __forceinline__ T quotient(T a, T p, T r) {
-    const T q = a * r;
-    const T e = fma(-q, p, a);
-    const T c = fma(e, r, q);
-    return e == e ? c : q;  // an infinite product has no remainder
-}
-
 // The next local column to a[0], the finished one to the end.
 template <class T>
 __device__ __forceinline__ void rotate4(T (&a)[16]) {
