@@ -1369,7 +1369,9 @@ rl_status gather_rows(const T *B, long long ldb, T *Y, long long ldy, int n, int
 // column each holding 4 of its rows in registers: step j broadcasts x_j within the
 // column's lanes by a shuffle and every lane updates its rows, y_i -= d_ij x_j in
 // increasing j (the order of the reference's substitution). The FP64 work of a U12
-// solve is spread over every scheduler of every SM instead of a few CTAs' threads.
+// solve is spread over every scheduler of every SM instead of a few CTAs' threads. The block is
+// loaded with all 32 loads of a thread in flight: an element at a time, with a division by bs
+// for its place, it was half of the kernel's time (FP32 20 -> 10.6 us a launch, FP64 33 -> 24).
 constexpr int kTrsmCols = 8;
 template <class T>
 static __global__ void __launch_bounds__(128) trsm_diag_kernel(const T *D, long long ldd, int bs, T *Y, long long ldy,
@@ -1380,13 +1382,22 @@ static __global__ void __launch_bounds__(128) trsm_diag_kernel(const T *D, long 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int c0 = blockIdx.x * kTrsmCols;
     if (tid == 0) s_bad = 0;
-    for (int idx = tid; idx < bs * bs; idx += blockDim.x) {
-        const int i = idx / bs, j = idx - i * bs;
-        Ds[i][j] = D[(long long)i * ldd + j];
-    }
-    for (int idx = tid; idx < 64 * kTrsmCols; idx += blockDim.x) {
-        const int i = idx / kTrsmCols, cc = idx - i * kTrsmCols;
-        Ys[i][cc] = (i < bs && c0 + cc < nrhs) ? Y[(long long)i * ldy + c0 + cc] : T(0);
+    {  // the block and the columns, every load in flight before the first store
+        T d[32], yv[64 * kTrsmCols / 128];
+#pragma unroll
+        for (int e = 0; e < 32; e++) {
+            const int i = 2 * e + (tid >> 6), j = tid & 63;
+            d[e] = (i < bs && j < bs) ? D[(long long)i * ldd + j] : T(0);
+        }
+#pragma unroll
+        for (int e = 0; e < 64 * kTrsmCols / 128; e++) {
+            const int i = (tid + 128 * e) / kTrsmCols, cc = tid % kTrsmCols;
+            yv[e] = (i < bs && c0 + cc < nrhs) ? Y[(long long)i * ldy + c0 + cc] : T(0);
+        }
+#pragma unroll
+        for (int e = 0; e < 32; e++) Ds[2 * e + (tid >> 6)][tid & 63] = d[e];
+#pragma unroll
+        for (int e = 0; e < 64 * kTrsmCols / 128; e++) Ys[(tid + 128 * e) / kTrsmCols][tid % kTrsmCols] = yv[e];
     }
     __syncthreads();
     if (mode != 0 && tid < bs && absT(Ds[tid][tid]) < tiny) s_bad = 1;
@@ -1874,9 +1885,15 @@ static __global__ void __launch_bounds__(128) trsm_right_lt_kernel(const T *D, l
                                                             int m) {
     __shared__ T Ds[64][65];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int idx = tid; idx < bs * bs; idx += 128) {
-        const int i = idx / bs, j = idx - i * bs;
-        Ds[i][j] = D[(long long)i * ldd + j];
+    {
+        T d[32];
+#pragma unroll
+        for (int e = 0; e < 32; e++) {
+            const int i = 2 * e + (tid >> 6), j = tid & 63;
+            d[e] = (i < bs && j < bs) ? D[(long long)i * ldd + j] : T(0);
+        }
+#pragma unroll
+        for (int e = 0; e < 32; e++) Ds[2 * e + (tid >> 6)][tid & 63] = d[e];
     }
     __syncthreads();
     const int row = blockIdx.x * kTrsmCols + 2 * warp + (lane >> 4), r16 = lane & 15;

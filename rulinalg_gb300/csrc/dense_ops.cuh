@@ -243,8 +243,8 @@ rl_status tri_solve_dev(const TA *A, long long lda, int n, T *Y, long long ldy, 
 // Matrix<f32>): 256-column blocks, each factored with the 64-column panels confined to
 // the block, then ONE trailing update of K = 256 on the tensor cores (tcgen05, 3xTF32;
 // the K = 64 updates of the inner panels measured slower there and stay on the SIMT
-// kernel). FP64: 0, one block spanning the matrix (every update is a K = 64 DFMA GEMM,
-// already at the FP64 rate). The FP32 LU takes its width from RL_TUNE_LU_OUTER_NB.
+// kernel). FP64: 0, one block spanning the matrix (K = 64 updates). The LU has its own
+// widths (lu_factor_dev).
 template <class T>
 constexpr int outer_nb() {
     return std::is_same<T, float>::value ? 256 : 0;
@@ -277,7 +277,7 @@ rl_status lu_factor_dev(T *A, long long lda, int n, int *ipiv, cudaStream_t s, T
     // after it runs on in-range indices, and every later panel stops at its first barrier.
     RL_TRY_CUDA(cudaMemsetAsync(sync.p, 0, sizeof(PanelSync), s));
     unsigned long long wns = wait_ns();
-    int NBO = n;  // FP32: outer blocks of RL_TUNE_LU_OUTER_NB columns (a multiple of NB)
+    int NBO = n;  // outer block width (FP32: RL_TUNE_LU_OUTER_NB, a multiple of NB)
     if constexpr (std::is_same<T, float>::value) {
         // automatic: at n = 2048 / 4096 one level measured 9.4 / 20.5 ms against 10.5 / 24.2
         // with 256-column blocks; at 8192 / 16384 1024-column blocks 58.2 / 171 ms against
@@ -286,6 +286,12 @@ rl_status lu_factor_dev(T *A, long long lda, int n, int *ipiv, cudaStream_t s, T
         const long long v = tune(RL_TUNE_LU_OUTER_NB);
         const int w = v < 0 ? (n < 6144 ? 0 : 1024) : (int)(v / NB) * NB;
         if (w >= NB) NBO = w;
+    } else if (n >= 3072) {
+        // FP64: the trailing products run on the tensor cores, where K = 64 is dominated by C's
+        // traffic and a tile's fixed cost. FP64 solves with one level / 256 / 512 / 1024-column
+        // blocks: n = 2048 8.6 / 9.6 / 9.8 / 9.6 ms, 4096 28.9 / 26.6 / 26.3 / 26.5, 8192 139 /
+        // 94.6 / 88.5 / 89.2.
+        NBO = 512;
     }
     for (int K0 = 0; K0 < n; K0 += NBO) {
         const int K1 = std::min(n, K0 + NBO), KB = K1 - K0;

@@ -66,3 +66,17 @@ def test_failing_pivot_and_nan_column(gpu, col):
         assert np.array_equal(p, p2) and np.array_equal(np.isnan(f), np.isnan(f2))
         ok = ~np.isnan(f)
         assert np.array_equal(f[ok], f2[ok])
+
+
+@pytest.mark.parametrize("n", [3071, 3072, 3600])
+def test_fp64_outer_blocks(gpu, n):
+    """FP64 LU around the size where 512-column outer blocks start: P A = L U on sampled rows
+    within n u |L||U|."""
+    rng = np.random.default_rng(n)
+    a = rng.uniform(-1, 1, (n, n))
+    t = gpu.PartialPivLu.decompose(a).unpack()
+    rows = rng.permutation(n)[:40]
+    pa = np.empty_like(a)
+    pa[t.p.perm.astype(np.int64)] = a
+    bound = n * 2.0 ** -53 * (np.abs(t.l[rows]) @ np.abs(t.u))
+    assert (np.abs(t.l[rows] @ t.u - pa[rows]) <= bound).all()
