@@ -200,6 +200,14 @@ static __device__ __noinline__ int dequeue(const BatchDesc &d, int count, int &g
     return it;
 }
 
+// The three CTAs of an SM are in different phases of systems of different kinds, so the code
+// they run together decides how often a warp waits for instructions: with one copy of the
+// solve, of the one-warp path and of the pivot search (two or three inlined before) the
+// 40,000-system mix went from 45.0 to 42.2 ms and the 20,000 FP32 Cholesky systems from 12.8
+// to 12.0. Calls around the factorisations, the copy and the residual as well were slower
+// (45.5 and 13.3 ms: their registers then go through the stack), and so was replacing the
+// 32-step diagonal solves by inverted diagonal blocks (48.2 ms: more code, and the inversion).
+//
 // GATED: the host path's single launch over chunks that are still arriving (dequeue()
 // waits on the chunk flags); a separate instantiation, so the device path's kernel
 // carries none of it.

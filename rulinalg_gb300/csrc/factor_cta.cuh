@@ -440,9 +440,8 @@ __device__ int cta_lu_factor(T *__restrict__ A, int lda, int n, CtaSmem<T> &S, T
         }
         if (tid == 0) S.nmoved = 0;
         // One barrier per column, the column loop rolled: every row is kept rotated so
-        // that row[k][0] holds the current column j. Step j combines the warps' argmax
-        // candidates for column j (published at the end of the previous step, rotated
-        // the same way), turns the active rows' row[k][0] into multipliers, updates
+        // that row[k][0] holds the current column j. Step j publishes the warps' argmax
+        // candidates for column j (double-buffered by parity) and combines them, turns the active rows' row[k][0] into multipliers, updates
         // their columns j + 1 .. NB - 1 (indices 1 .. NB - 1 - j) with the pivot row,
         // and rotates every row left by one, the finished column-j entry going to the
         // end. After NB steps the rows are back in column order.
@@ -488,9 +487,9 @@ __device__ int cta_lu_factor(T *__restrict__ A, int lda, int n, CtaSmem<T> &S, T
                 row[k][NB - 1] = first;
             }
         };
-        publish(0, 0);
         for (int j = 0; j < kb; j++) {
             const int par = j & 1;
+            publish(j, par);
             __syncthreads();
             T bv = S.redv[par][0];
             int bi = S.redi[par][0], bq = S.redq[par][0], bw = 0;
@@ -542,7 +541,6 @@ __device__ int cta_lu_factor(T *__restrict__ A, int lda, int n, CtaSmem<T> &S, T
                 }
             }
             rotate();
-            if (j + 1 < kb) publish(j + 1, par ^ 1);
         }
         for (int j = kb; j < NB; j++) rotate();  // a narrow last panel: back to column order
         __syncthreads();
@@ -970,9 +968,11 @@ __device__ void cta_apply_pivots(int n, CtaSmem<T> &S) {
     __syncthreads();
 }
 
-// Full solve with a factor: kind 0 = LU (row permutation in S.rowperm), 1 = Cholesky.
+// Full solve with a factor: kind 0 = LU (row permutation in S.rowperm), 1 = Cholesky. Out of
+// line, one copy for the first solve and the corrections: with CTAs of one SM in different
+// phases the kernels run at the instruction cache's pace (batch.cuh).
 template <class T>
-__device__ int cta_factor_solve(const T *A, int lda, int n, int kind, CtaSmem<T> &S, T tiny) {
+__device__ __noinline__ int cta_factor_solve(const T *A, int lda, int n, int kind, CtaSmem<T> &S, T tiny) {
     if (kind == 1) {
         int st = cta_lower_solve(A, lda, n, S, tiny);
         if (st != RL_OK) return st;

@@ -118,11 +118,11 @@ __device__ double warp_residual(const TI *__restrict__ A, int n, double bl, doub
     return warp_max(fabs(r));
 }
 
-// One system by one warp; `tile` is the warp's WARP_NMAX x WARP_LDT slice of shared
+// One system by one warp (out of line: two call sites in the kernel); `tile` is the warp's WARP_NMAX x WARP_LDT slice of shared
 // memory. Writes x, info, iters, berr like batch_solve_one; mixed-precision failures go
 // to the FP64 fallback list.
 template <class TI, class TF, bool MIXED>
-__device__ void warp_solve_small(const BatchDesc &d, int sys, const TI *__restrict__ A, const TI *__restrict__ B,
+__device__ __noinline__ void warp_solve_small(const BatchDesc &d, int sys, const TI *__restrict__ A, const TI *__restrict__ B,
                                  TI *__restrict__ X, TF *tile) {
     const int lane = threadIdx.x & 31;
     const int n = d.n[sys], kind = d.kind[sys];
