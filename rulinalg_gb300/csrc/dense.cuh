@@ -1462,7 +1462,10 @@ static __global__ void __launch_bounds__(128) trsm_diag_kernel(const T *D, long 
 //     blocks and are reduced once, after the last one;
 //   * the diagonal block is in shared memory from the start: as its inverse (Dinv, from
 //     diag_inverse: the solve is one more BR x BR product) or scaled by its reciprocal
-//     diagonal, so that a substitution step is one shuffle and one multiply-add.
+//     diagonal, so that a substitution step is one shuffle and one multiply-add;
+//   * with Link (diag_link: Dinv_b times the tile of A that meets the block solved just
+//     before b) that product is off the chain too: Dinv_b times everything else is ready when
+//     the last solution arrives, x_b = c_b - Link_b x.
 // BR = 128 for FP32; 64 for FP64, where the products of a tile are bound by the FP64 unit.
 // The form before (64-row blocks, a flag per block behind a fence, the folded sums through
 // shared memory) against this one, per sweep: FP32 with inverses n = 3000 132 and 52 us,
@@ -1547,7 +1550,7 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
                                                              int n, T *__restrict__ Y, long long ldy, int nrhs, int mode,
                                                              T *ws, int *tickets, int *status, T tiny,
                                                              unsigned long long wait_ns, int withhold,
-                                                             const T *__restrict__ Dinv) {
+                                                             const T *__restrict__ Dinv, const T *__restrict__ Link) {
     using cfg = SweepCfg<T, RW>;
     constexpr int BR = cfg::BR, CPL = cfg::CPL, LDD = cfg::LDD, THREADS = cfg::THREADS, WARPS = cfg::WARPS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1577,19 +1580,24 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
         if (!trans)
 #pragma unroll
             for (int c = 0; c < RW; c++) y[c] = (mrow < bs && c < nrhs) ? Y[(long long)(r0 + mrow) * ldy + c] : T(0);
-        if (Dinv) {
-            const T *Db = Dinv + (long long)b * BR * BR;
-            for (int e = tid; e < BR * BR; e += THREADS) Ds[(e / BR) * LDD + e % BR] = Db[e];
-        } else {
-            for (int e = tid; e < BR * BR; e += THREADS) {
-                const int i = e / BR, j = e % BR;
-                T d = T(0);
-                if (i < bs && j < bs) d = T(A[(long long)(r0 + i) * lda + r0 + j]);
-                if (trans)
-                    Ds[j * LDD + i] = d;
-                else
-                    Ds[i * LDD + j] = d;
-            }
+        // The diagonal block, every load in flight before the first store (element by element the
+        // staging alone was ~20 us of a sweep).
+        constexpr int DP = BR * BR / THREADS;
+        T dv[DP];
+#pragma unroll
+        for (int q = 0; q < DP; q++) {
+            const int e = tid + q * THREADS, i = e / BR, j = e % BR;
+            if (Dinv)
+                dv[q] = Dinv[(long long)b * BR * BR + e];
+            else
+                dv[q] = (i < bs && j < bs) ? T(A[(long long)(r0 + i) * lda + r0 + j]) : T(0);
+        }
+#pragma unroll
+        for (int q = 0; q < DP; q++) {
+            const int e = tid + q * THREADS, i = e / BR, j = e % BR;
+            Ds[!Dinv && trans ? j * LDD + i : i * LDD + j] = dv[q];
+        }
+        if (!Dinv) {
             __syncthreads();
             if (tid < BR) {
                 const T d = tid < bs ? Ds[tid * LDD + tid] : T(1);
@@ -1623,11 +1631,27 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
                         t[i][u] = (wr < bs && lc < ks) ? A[(long long)(r0 + wr) * lda + c0 + lc] : TA(0);
                 }
         };
-        if (nk > 0) load(0, cur);
-        for (int kk = 0; kk < nk; kk++) {
+        const int nf = Link && nk > 0 ? nk - 1 : nk;  // blocks folded before the diagonal block's product
+        auto link = [&](TA (&t)[NA][CPL]) {
+#pragma unroll
+            for (int i = 0; i < NA; i++)
+#pragma unroll
+                for (int u = 0; u < CPL; u++)
+                    t[i][u] = (TA)Link[((long long)b * BR + warp * 8 + i) * BR + lane + 32 * u];
+        };
+        if (nf > 0)
+            load(0, cur);
+        else if (nk > 0)
+            link(cur);
+        for (int kk = 0; kk < nf; kk++) {
             // One right-hand side: the next tile is under way while this one waits. With 8
             // the sums take those registers.
-            if (RW == 1 && kk + 1 < nk) load(kk + 1, nxt);
+            if (RW == 1) {
+                if (kk + 1 < nf)
+                    load(kk + 1, nxt);
+                else if (nf < nk)
+                    link(nxt);
+            }
             const int k = fwd ? kk : nb - 1 - kk, c0 = k * BR, ks = min(BR, n - c0);
             if (RW == 1) {
                 if (!trans) {
@@ -1669,7 +1693,10 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
                             for (int c = 0; c < RW; c++) acc[i][c] = fma(T(cur[i][w0 & (CPL - 1)]), x[c], acc[i][c]);
                     }
                 }
-                if (kk + 1 < nk) load(kk + 1, cur);
+                if (kk + 1 < nf)
+                    load(kk + 1, cur);
+                else if (nf < nk)
+                    link(cur);
             }
             if (RW == 1)
 #pragma unroll
@@ -1729,14 +1756,51 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
                     for (int c = 0; c < RW; c++) o[i][c] = fma(d, x[c], o[i][c]);
                 }
             }
-#pragma unroll
-            for (int c = 0; c < RW; c++) {
+            auto reduce = [&](int c) {
                 T s8[8];
 #pragma unroll
                 for (int i = 0; i < 8; i++) s8[i] = o[i][c];
                 int row;
-                const T x = warp_reduce_scatter<8>(s8, lane, row);
-                if ((lane & 3) == 0) publish(mrow, c, x);
+                return warp_reduce_scatter<8>(s8, lane, row);
+            };
+            if (nf == nk) {
+#pragma unroll
+                for (int c = 0; c < RW; c++) {
+                    const T x = reduce(c);
+                    if ((lane & 3) == 0) publish(mrow, c, x);
+                }
+            } else {
+                T cb[RW];
+#pragma unroll
+                for (int c = 0; c < RW; c++) cb[c] = reduce(c);
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+#pragma unroll
+                    for (int c = 0; c < RW; c++) o[i][c] = T(0);
+                const int k = fwd ? b - 1 : b + 1, c0 = k * BR, ks = min(BR, n - c0);
+                if (RW > 1) {
+                    for (int e = tid; e < BR * RW; e += THREADS)
+                        xs[e] = e < ks * RW && e % RW < nrhs ? sweep_get(ws + (size_t)c0 * RW + e, &s_fail, wait_ns) : T(0);
+                    __syncthreads();
+                }
+#pragma unroll
+                for (int u = 0; u < CPL; u++) {
+                    const int lc = lane + 32 * u;
+                    T x[RW];
+                    if constexpr (RW == 1)
+                        x[0] = lc < ks ? sweep_get(ws + c0 + lc, &s_fail, wait_ns) : T(0);
+                    else
+                        ldv<RW>(xs + lc * RW, x);
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+#pragma unroll
+                        for (int c = 0; c < RW; c++) o[i][c] = fma(T(cur[i][u]), x[c], o[i][c]);
+                }
+#pragma unroll
+                for (int c = 0; c < RW; c++) {
+                    const T x = cb[c] - reduce(c);
+                    if ((lane & 3) == 0) publish(mrow, c, x);
+                }
             }
         } else if (warp < RW) {
             // substitution with the scaled rows: warp c solves right-hand side c, lane l
@@ -1874,6 +1938,55 @@ static __global__ void __launch_bounds__(256) diag_join_kernel(const TA *__restr
             out[r * 128 + c] = X[r * 65 + c];
             out[(64 + r) * 128 + 64 + c] = Z[r * 65 + c];
         }
+}
+
+// Link_b = Dinv_b op(A)_{b, b'} for the sweep, b' the block solved just before b (b - 1 for the
+// lower modes, b + 1 for the upper ones); 128 x 128 row-major per block, zero beyond n. Grid
+// (blocks, 4): a 64 x 64 quadrant per CTA, the K = 128 products in two halves.
+template <class T, class TA>
+static __global__ void __launch_bounds__(256) diag_link_kernel(const TA *__restrict__ A, long long lda, int n, int mode,
+                                                           const T *__restrict__ Dinv, T *__restrict__ Link) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *X = reinterpret_cast<T *>(smem_raw), *M = X + 64 * 65;
+    const int nb = (n + 127) / 128, b = blockIdx.x, bp = mode <= 1 ? b - 1 : b + 1;
+    if (bp < 0 || bp >= nb) return;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int i0 = (blockIdx.y >> 1) * 64, j0 = (blockIdx.y & 1) * 64, r0 = b * 128, c0 = bp * 128;
+    T o[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) o[i][j] = T(0);
+    for (int h = 0; h < 128; h += 64) {
+        __syncthreads();
+#pragma unroll 8
+        for (int e = tid; e < 64 * 64; e += 256) {
+            const int i = e >> 6, j = e & 63;
+            X[i * 65 + j] = Dinv[((long long)b * 128 + i0 + i) * 128 + h + j];
+            if (mode == 3) {  // op(A)[r][c] = A[c][r]: consecutive threads along r
+                const int r = r0 + h + j, c = c0 + j0 + i;
+                M[j * 65 + i] = (r < n && c < n) ? T(A[(long long)c * lda + r]) : T(0);
+            } else {
+                const int r = r0 + h + i, c = c0 + j0 + j;
+                M[i * 65 + j] = (r < n && c < n) ? T(A[(long long)r * lda + c]) : T(0);
+            }
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int k = 0; k < 64; k++) {
+            T li[4], rj[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) li[i] = X[(ty + 16 * i) * 65 + k], rj[i] = M[k * 65 + tx + 16 * i];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) o[i][j] = fma(li[i], rj[j], o[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) Link[((long long)b * 128 + i0 + ty + 16 * i) * 128 + j0 + tx + 16 * j] = o[i][j];
 }
 
 // Row-wise solve X D^T = Y for the rows of Y (m x bs, stride ldy), D lower bs x bs: the
