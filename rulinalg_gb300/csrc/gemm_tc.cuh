@@ -3,9 +3,9 @@
 //     C = alpha * A * B + beta * C,  A (m x k), B (k x n), C (m x n), row-major.
 //
 // Every operand x is split once into hi = tf32(x) (round to nearest) and lo = x - hi
-// (split_rows_kernel for A, split_transpose_kernel for B, which also transposes B to
-// K-major), and each product is accumulated as a_lo b_hi + a_hi b_lo + a_hi b_hi in FP32
-// in tensor memory (the a_lo b_lo term is below FP32 rounding).
+// (split_kernel, which also makes both operands K-major), and each product is accumulated as
+// a_lo b_hi + a_hi b_lo + a_hi b_hi in FP32 in tensor memory (the a_lo b_lo term is below FP32
+// rounding).
 //
 // sgemm_tma_kernel: one CTA (4 warps) per 128 x 128 tile of C, accumulator in 128
 // columns of tensor memory. K advances in chunks of 32 through a 3-stage ring of shared
@@ -133,41 +133,80 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 
 }  // namespace tc
 
-// hi/lo of A (rows x k, row stride ldx) into rows x kp buffers (kp = k rounded up to 32,
-// zero beyond k).
-static __global__ void split_rows_kernel(const float *__restrict__ X, long long ldx, int rows, int k, int kp,
-                                         float *__restrict__ hi, float *__restrict__ lo) {
-    const long long total = (long long)rows * kp;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-        const int r = (int)(e / kp), c = (int)(e - (long long)r * kp);
-        const float x = c < k ? X[(long long)r * ldx + c] : 0.f;
-        const float h = tc::tf32_rna(x);
-        hi[e] = h;
-        lo[e] = x - h;
-    }
-}
+// One operand of a product as rows x k, K-major: element (r, p) at X[r ld + p], or X[p ld + r]
+// with trans; hi and lo are rows x kp (kp = k rounded up to 32, zero beyond k).
+struct SplitOperand {
+    const float *X;
+    long long ld;
+    int rows, trans, vec;  // vec: 16-byte loads are aligned (trans = 0)
+    float *hi, *lo;
+    int blocks;            // of the launch's grid
+};
 
-// hi/lo of B^T: B is k x n (row stride ldb); outputs are n x kp (K-major), zero beyond k.
-// 32 x 32 tiles through shared memory; block (32, 8).
-static __global__ void split_transpose_kernel(const float *__restrict__ B, long long ldb, int k, int n, int kp,
-                                              float *__restrict__ hi, float *__restrict__ lo) {
-    __shared__ float t[32][33];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+// hi / lo of both operands in one launch, bound by memory (4 bytes in, 8 out per element). A
+// thread moves 4 consecutive p (16-byte stores; trans goes through 64 x 32 tiles of shared
+// memory). An element per thread and a launch per operand took 90 us for two 4096 x 4096
+// operands; this takes 59.
+static __global__ void __launch_bounds__(256) split_kernel(SplitOperand a, SplitOperand b, int k, int kp) {
+    __shared__ float t[32][65];
+    const bool second = (int)blockIdx.x >= a.blocks;
+    const SplitOperand o = second ? b : a;
+    const int blk = (int)blockIdx.x - (second ? a.blocks : 0), tid = threadIdx.x;
+    auto put = [&](long long at, const float (&x)[4]) {
+        float4 h, l;
+        float *hp = reinterpret_cast<float *>(&h), *lp = reinterpret_cast<float *>(&l);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const int kk = k0 + ty + 8 * j, nn = n0 + tx;
-        t[ty + 8 * j][tx] = (kk < k && nn < n) ? B[(long long)kk * ldb + nn] : 0.f;
+        for (int u = 0; u < 4; u++) {
+            hp[u] = tc::tf32_rna(x[u]);
+            lp[u] = x[u] - hp[u];
+        }
+        *reinterpret_cast<float4 *>(o.hi + at) = h;
+        *reinterpret_cast<float4 *>(o.lo + at) = l;
+    };
+    if (!o.trans) {
+        const int per = kp / 4;
+        const long long total = (long long)o.rows * per, step = (long long)o.blocks * 256;
+        for (long long e0 = (long long)blk * 256 + tid; e0 < total; e0 += 4 * step) {
+            float x[4][4];
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                const long long e = e0 + v * step;
+                const int r = (int)(e / per), p = (int)(e - (long long)r * per) * 4;
+                const float *src = o.X + (long long)r * o.ld + p;
+                if (e < total && o.vec && p + 4 <= k) {
+                    const float4 q = *reinterpret_cast<const float4 *>(src);
+                    x[v][0] = q.x, x[v][1] = q.y, x[v][2] = q.z, x[v][3] = q.w;
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 4; u++) x[v][u] = e < total && p + u < k ? src[u] : 0.f;
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < 4; v++)
+                if (e0 + v * step < total) put((e0 + v * step) * 4, x[v]);
+        }
+        return;
     }
-    __syncthreads();
+    const int rb = (o.rows + 63) / 64, kb = kp / 32;
+    for (long long t0 = blk; t0 < (long long)rb * kb; t0 += o.blocks) {
+        const int r0 = (int)(t0 % rb) * 64, p0 = (int)(t0 / rb) * 32;
+        __syncthreads();
+        float x[8];
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const int nn = n0 + ty + 8 * j, kk = k0 + tx;
-        if (nn < n) {
-            const float x = t[tx][ty + 8 * j];
-            const float h = tc::tf32_rna(x);
-            hi[(long long)nn * kp + kk] = h;
-            lo[(long long)nn * kp + kk] = x - h;
+        for (int j = 0; j < 8; j++) {  // 64 consecutive r of one p per 64 threads
+            const int p = p0 + (tid >> 6) + 4 * j, r = r0 + (tid & 63);
+            x[j] = (p < k && r < o.rows) ? o.X[(long long)p * o.ld + r] : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) t[(tid >> 6) + 4 * j][tid & 63] = x[j];
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int r = (tid >> 3) + 32 * j, p = (tid & 7) * 4;
+            if (r0 + r < o.rows) {
+                const float y[4] = {t[p][r], t[p + 1][r], t[p + 2][r], t[p + 3][r]};
+                put((long long)(r0 + r) * kp + p0 + p, y);
+            }
         }
     }
 }
@@ -267,6 +306,7 @@ static __global__ void __launch_bounds__(tc::THREADS, 1)
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int r = row0 + warp * 32 + lane;
+    const bool vec = !lower && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
 #pragma unroll 1
     for (int c0 = 0; c0 < BN; c0 += 16) {
         float v[16];
@@ -278,6 +318,20 @@ static __global__ void __launch_bounds__(tc::THREADS, 1)
         }
         if (r < m) {
             float *dst = C + (long long)r * ldc + col0 + c0;
+            if (vec && col0 + c0 + 16 <= n) {  // 16-byte stores: 564 -> 518 us at 4096^3
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) {
+                    float4 *p4 = reinterpret_cast<float4 *>(dst + j);
+                    float4 out = make_float4(alpha * v[j], alpha * v[j + 1], alpha * v[j + 2], alpha * v[j + 3]);
+                    if (ok && beta != 0.f) {
+                        const float4 old = *p4;
+                        out = make_float4(fmaf(beta, old.x, out.x), fmaf(beta, old.y, out.y), fmaf(beta, old.z, out.z),
+                                          fmaf(beta, old.w, out.w));
+                    }
+                    *p4 = out;
+                }
+                continue;
+            }
 #pragma unroll
             for (int j = 0; j < 16; j++) {
                 if (col0 + c0 + j < n && !(lower && col0 + c0 + j > r)) {
@@ -364,29 +418,23 @@ static rl_status sgemm_tc(int m, int n, int k, float alpha, const float *A, long
         cudaFuncSetAttribute(sgemm_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
     RL_TRY_CUDA(attr);
     const int kp = (k + tc::BK - 1) / tc::BK * tc::BK;
-    DevBuf<float> Ah, Al, Bh, Bl;
-    RL_TRY(Ah.alloc((size_t)m * kp, s));
-    RL_TRY(Al.alloc((size_t)m * kp, s));
-    RL_TRY(Bh.alloc((size_t)n * kp, s));
-    RL_TRY(Bl.alloc((size_t)n * kp, s));
-    auto split_rows = [&](const float *X, long long ldx, int rows, float *hi, float *lo) -> rl_status {
-        const long long t = (long long)rows * kp;
-        RL_LAUNCH(split_rows_kernel, (int)std::min<long long>(8LL * num_sms(), (t + 255) / 256), 256, 0, s, X, ldx,
-                  rows, k, kp, hi, lo);
-        return RL_OK;
+    const size_t ae = (size_t)m * kp, be = (size_t)n * kp;  // multiples of 32 elements
+    DevBuf<float> ws;
+    RL_TRY(ws.alloc(2 * (ae + be), s));
+    float *Ah = ws.p, *Al = Ah + ae, *Bh = Al + ae, *Bl = Bh + be;
+    auto operand = [&](const float *X, long long ld, int rows, bool trans, float *hi, float *lo) {
+        const bool vec = !trans && ld % 4 == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0;
+        const long long work = trans ? (long long)ceil_div(rows, 64) * (kp / 32) : ceil_div((long long)rows * (kp / 4), 1024);
+        return SplitOperand{X, ld, rows, trans ? 1 : 0, vec ? 1 : 0, hi, lo,
+                            (int)std::min<long long>(8LL * num_sms(), std::max(1LL, work))};
     };
-    auto split_t = [&](const float *X, long long ldx, int rows, float *hi, float *lo) -> rl_status {
-        RL_LAUNCH(split_transpose_kernel, dim3((rows + 31) / 32, kp / 32), dim3(32, 8), 0, s, X, ldx, k, rows, kp, hi,
-                  lo);
-        return RL_OK;
-    };
-    RL_TRY(TA ? split_t(A, lda, m, Ah.p, Al.p) : split_rows(A, lda, m, Ah.p, Al.p));
-    RL_TRY(TB ? split_rows(B, ldb, n, Bh.p, Bl.p) : split_t(B, ldb, n, Bh.p, Bl.p));
+    const SplitOperand oa = operand(A, lda, m, TA, Ah, Al), ob = operand(B, ldb, n, !TB, Bh, Bl);
+    RL_LAUNCH(split_kernel, oa.blocks + ob.blocks, 256, 0, s, oa, ob, k, kp);
     CUtensorMap mAh, mAl, mBh, mBl;
-    RL_TRY(make_tile_map(mAh, Ah.p, m, kp));
-    RL_TRY(make_tile_map(mAl, Al.p, m, kp));
-    RL_TRY(make_tile_map(mBh, Bh.p, n, kp));
-    RL_TRY(make_tile_map(mBl, Bl.p, n, kp));
+    RL_TRY(make_tile_map(mAh, Ah, m, kp));
+    RL_TRY(make_tile_map(mAl, Al, m, kp));
+    RL_TRY(make_tile_map(mBh, Bh, n, kp));
+    RL_TRY(make_tile_map(mBl, Bl, n, kp));
     int *err = nullptr;
     RL_TRY_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&err), g_sgemm_tc_err));
     dim3 grid((n + tc::BN - 1) / tc::BN, (m + tc::BM - 1) / tc::BM);
