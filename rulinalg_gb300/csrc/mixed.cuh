@@ -94,6 +94,18 @@ static __global__ void colnorm_kernel(const double *__restrict__ V, long long ld
     }
 }
 
+// The same for two matrices (the refinement's residual and solution) in one launch: out[c] for
+// R, out[nrhs + c] for X.
+static __global__ void colnorm2_kernel(const double *__restrict__ R, long long ldr, const double *__restrict__ X, long long ldx,
+                                int n, int nrhs, unsigned long long *out) {
+    const long long total = (long long)n * nrhs;
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
+        const int i = (int)(e / nrhs), c = (int)(e - (long long)i * nrhs);
+        atomic_max_nonneg(out + c, fabs(R[(long long)i * ldr + c]));
+        atomic_max_nonneg(out + nrhs + c, fabs(X[(long long)i * ldx + c]));
+    }
+}
+
 // W = (float)(R / scale[c]) (scale given as bits of a double), row i of W from row
 // rows[i] of R when a row map is given (the pivoting of an LU factor).
 static __global__ void scale_to_f32_kernel(const double *__restrict__ R, long long ldr, int n, int nrhs,

@@ -466,19 +466,20 @@ struct MixedFactor {
         if (!f32_ok) return solve_with_fp64(B, ldb, X, ldx, nrhs, out, s);
         DevBuf<float> W;
         DevBuf<double> R;
-        DevBuf<int> dstatus, active;
-        DevBuf<unsigned long long> nb;  // bnorm, rnorm, xnorm per column
+        DevBuf<int> active;
+        // bnorm, rnorm, xnorm per column and the two status words, read back together
+        DevBuf<unsigned long long> nb;
         RL_TRY(W.alloc((size_t)n * nrhs, s));
         RL_TRY(R.alloc((size_t)n * nrhs, s));
-        RL_TRY(dstatus.alloc(2, s));
         RL_TRY(active.alloc(nrhs + 1, s));
-        RL_TRY(nb.alloc(3 * nrhs, s));
-        unsigned long long *bn_b = nb.p, *rn_b = nb.p + nrhs, *xn_b = nb.p + 2 * nrhs;
-        RL_TRY_CUDA(cudaMemsetAsync(dstatus.p, 0, 2 * sizeof(int), s));
+        RL_TRY(nb.alloc(3 * nrhs + 1, s));
+        unsigned long long *bn_b = nb.p, *rn_b = nb.p + nrhs;
+        int *dstatus = reinterpret_cast<int *>(nb.p + 3 * nrhs);
+        RL_TRY_CUDA(cudaMemsetAsync(dstatus, 0, 2 * sizeof(int), s));
         SweepInv inv;
         DevBuf<unsigned char> sweep_ws;
         if (tune(RL_TUNE_MIXED_SWEEP_INV) && sweep_groups(nrhs) > 0 && n > CTA_NMAX && !g_shared_gpu) {
-            RL_TRY(ensure_dinv(dstatus.p, s));
+            RL_TRY(ensure_dinv(dstatus, s));
             RL_TRY(sweep_ws.alloc(2 * sweep_ws_bytes<float>(n, nrhs), s));
             const size_t de = dinv_elems();
             inv = SweepInv{Dinv, Dinv + de, Dinv + 2 * de, Dinv + 3 * de, sweep_ws.p};
@@ -492,25 +493,26 @@ struct MixedFactor {
         std::vector<double> prev(nrhs, INFINITY), bnorm(nrhs, 0.0);
         // x0 = M^-1 b
         RL_LAUNCH(scale_to_f32_kernel, ge, 256, 0, s, B, ldb, n, nrhs, bn_b, rows, W.p, (long long)nrhs);
-        RL_TRY(precond_solve(F, n, kind, W.p, nrhs, nrhs, dstatus.p, s, inv));
+        RL_TRY(precond_solve(F, n, kind, W.p, nrhs, nrhs, dstatus, s, inv));
         RL_TRY_CUDA(cudaMemset2DAsync(X, ldx * sizeof(double), 0, nrhs * sizeof(double), n, s));
         RL_LAUNCH(update_x_kernel, ge, 256, 0, s, X, ldx, W.p, (long long)nrhs, n, nrhs, bn_b, active.p);
-        std::vector<unsigned long long> hb(3 * nrhs);
+        std::vector<unsigned long long> hb(3 * nrhs + 1);
         bool stalled = false, need_fp64 = false, diverged = false;
         const int max_steps = (int)tune(RL_TUNE_MIXED_REFINE_STEPS);
         for (int it = 0;; it++) {
             RL_TRY(residual_dev(A, lda, n, X, ldx, B, ldb, R.p, nrhs, nrhs, s));
-            RL_TRY(colnorm_dev(R.p, nrhs, n, nrhs, rn_b, s));
-            RL_TRY(colnorm_dev(X, ldx, n, nrhs, xn_b, s));
-            int dst = 0;
+            RL_TRY_CUDA(cudaMemsetAsync(rn_b, 0, 2 * nrhs * sizeof(unsigned long long), s));
+            RL_LAUNCH(colnorm2_kernel, ge, 256, 0, s, R.p, (long long)nrhs, X, ldx, n, nrhs, rn_b);
             RL_TRY_CUDA(cudaMemcpyAsync(hb.data(), nb.p, hb.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-            RL_TRY_CUDA(cudaMemcpyAsync(&dst, dstatus.p, sizeof(int), cudaMemcpyDeviceToHost, s));
             RL_TRY_CUDA(cudaStreamSynchronize(s));
+            int dst = 0;
+            memcpy(&dst, &hb[3 * nrhs], sizeof dst);
             if (dst != 0) {  // the FP32 factor met a pivot below FLT_MIN in a solve
                 need_fp64 = true;
                 break;
             }
             int all = 1;
+            bool changed = false;  // a column of `active` to be switched
             double berr = 0;
             for (int c = 0; c < nrhs; c++) {
                 bnorm[c] = bits_to_double(hb[c]);
@@ -529,6 +531,7 @@ struct MixedFactor {
                 if (!std::isfinite(rn)) stalled = diverged = true;
                 prev[c] = rn;
                 all &= conv[c];
+                changed |= act[c] != !conv[c];
                 act[c] = !conv[c];
             }
             out.berr = berr;
@@ -540,10 +543,11 @@ struct MixedFactor {
                 for (int c = 0; c < nrhs; c++) conv[c] |= near[c];
                 break;
             }
-            RL_TRY_CUDA(cudaMemcpyAsync(active.p, act.data(), nrhs * sizeof(int), cudaMemcpyHostToDevice, s));
+            if (changed)
+                RL_TRY_CUDA(cudaMemcpyAsync(active.p, act.data(), nrhs * sizeof(int), cudaMemcpyHostToDevice, s));
             RL_LAUNCH(scale_to_f32_kernel, ge, 256, 0, s, R.p, (long long)nrhs, n, nrhs, rn_b, rows, W.p,
                       (long long)nrhs);
-            RL_TRY(precond_solve(F, n, kind, W.p, nrhs, nrhs, dstatus.p, s, inv));
+            RL_TRY(precond_solve(F, n, kind, W.p, nrhs, nrhs, dstatus, s, inv));
             RL_LAUNCH(update_x_kernel, ge, 256, 0, s, X, ldx, W.p, (long long)nrhs, n, nrhs, rn_b, active.p);
         }
         if (!need_fp64) {
@@ -566,7 +570,7 @@ struct MixedFactor {
             DevBuf<double> xb, bb;
             RL_TRY(xb.alloc(n, s));
             RL_TRY(bb.alloc(n, s));
-            Minv M{F, n, kind, rows, dstatus.p + 1, {}, {}, {}};
+            Minv M{F, n, kind, rows, dstatus + 1, {}, {}, {}};
             RL_TRY(M.init(s));
             for (int c = 0; c < nrhs && !need_fp64; c++) {
                 if (conv[c]) continue;
@@ -578,7 +582,7 @@ struct MixedFactor {
                 bool ok = false;
                 RL_TRY(gmres_ir(A, lda, n, M, bb.p, xb.p, anorm, bnorm[c], deadline, o, ok, s));
                 int dst = 0;
-                RL_TRY_CUDA(cudaMemcpyAsync(&dst, dstatus.p + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+                RL_TRY_CUDA(cudaMemcpyAsync(&dst, dstatus + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
                 RL_TRY_CUDA(cudaStreamSynchronize(s));
                 if (!ok || dst) {
                     need_fp64 = true;
