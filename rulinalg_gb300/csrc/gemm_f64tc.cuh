@@ -551,9 +551,11 @@ inline rl_status make_slice_map(CUtensorMap &map, const __nv_bfloat16 *S, int ro
 // Shapes worth the tensor cores: the slicing passes (34 bytes an element of A and B), five
 // launches and a tile's fixed cost against m n k on the FP64 unit. 256 x 256 with K = 64
 // measured 67-83 us against 92 on the FP64 unit, 512 x 512 with K = 256 87 against 289,
-// 2048^3 0.66 ms against 14.3 (26 TFLOP/s); below 6e6 multiply-adds the FP64 unit stays.
+// 2048^3 0.66 ms against 14.3 (26 TFLOP/s); below 6e6 multiply-adds the FP64 unit stays, or
+// below 1e6 for a long K, where it has few outputs to spread (V^T A of a panel, 64 x 50 with
+// K = 800: ~120 us and ~40).
 inline bool dgemm_tc_eligible(int m, int n, int k) {
-    return m >= 64 && n >= 32 && k >= 32 && (double)m * n * k >= 6e6;
+    return m >= 64 && n >= 32 && k >= 32 && (double)m * n * k >= (k > 512 ? 1e6 : 6e6);
 }
 
 // One CTA per tile, 1 per SM: the tile width with the smaller cost in waves of tiles.
