@@ -71,10 +71,11 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
     const int tx = tid % NTX, ty = tid / NTX;
     const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
     if (LOWER && col0 > row0 + BM - 1) return;  // tile strictly above the diagonal
+    constexpr bool FLAGS = std::is_same<T, double>::value;  // compiled into FP32 the test cost 4% at 2000 x 100 x 2000
     const int *flag_row = nullptr;
-    if (only.flags) {
+    if (FLAGS && only.flags) {
         if (*only.nfail == 0) return;
-        static_assert(!std::is_same<T, double>::value || tc64::BM % BM == 0, "one flag row per tile");
+        static_assert(!FLAGS || tc64::BM % BM == 0, "one flag row per tile");
         flag_row = only.flags + (row0 / tc64::BM) * only.gx;
         const int c1 = min(n, col0 + BN) - 1;
         int any = 0;
@@ -197,7 +198,7 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
             const int gj = col0 + (j / 4) * (BN / SN_) + tx * 4 + (j % 4);
             if (gj >= n) continue;
             if (LOWER && gj > gi) continue;
-            if (flag_row && !flag_row[gj / only.bn]) continue;
+            if (FLAGS && flag_row && !flag_row[gj / only.bn]) continue;
             T *cp = C + (long long)gi * ldc + gj;
             T v = alpha * acc[i][j];
             if (beta != T(0)) v = fma(beta, *cp, v);
