@@ -275,7 +275,7 @@ def event_times(fn, steps, warmup, stream, flush=None):
     return out
 
 
-FP64_PEAK_TFLOPS = 1.25  # GB300's FP64 rate (nominal; rl_dgemm_dev sustains it at n = 8192)
+FP64_PEAK_TFLOPS = 1.25  # GB300's FP64 unit (nominal)
 
 
 def peaks():
@@ -347,7 +347,7 @@ def config1(dev):
 
 def config2(dev, sizes=(1024, 2048, 4096, 8192), steps=3, warm=3):
     """Square GEMM sweep (N(0,1), seeded), f32 and f64, and the plain FP64 LU solve at the
-    largest size: TFLOP/s, fraction of the FP64 rate / the 3xTF32 ceiling, cuBLAS beside
+    largest size: TFLOP/s, fraction of the BF16-slice / the 3xTF32 ceiling, cuBLAS beside
     it for context, and the normwise accuracy bound n eps ||A||_F ||B||_F against an FP64
     product."""
     import torch
@@ -357,6 +357,7 @@ def config2(dev, sizes=(1024, 2048, 4096, 8192), steps=3, warm=3):
     sh = stream.cuda_stream
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
     ceil32 = tf32x3_ceiling_tflops()
+    ceil64 = ceil32 * 6 / 28  # FP64 products as 28 exact BF16 slice products: BF16 rate / 28
     sweep = []
     for n in sizes:
         g = torch.Generator(device=dev)
@@ -374,7 +375,7 @@ def config2(dev, sizes=(1024, 2048, 4096, 8192), steps=3, warm=3):
             bound = n * eps * float(torch.linalg.norm(a.double())) * float(torch.linalg.norm(b.double()))
             cub = statistics.median(event_times(lambda: torch.matmul(a, b, out=c), steps, warm, stream, flush))
             tf = 2.0 * n ** 3 / (ms / 1e3) / 1e12
-            peak = FP64_PEAK_TFLOPS if dt == torch.float64 else ceil32
+            peak = ceil64 if dt == torch.float64 else ceil32
             sweep.append({"n": n, "dtype": "f64" if dt == torch.float64 else "f32", "ms": ms, "tflops": tf,
                           "frac": tf / peak, "peak_tflops": peak, "cublas_tflops": 2.0 * n ** 3 / (cub / 1e3) / 1e12,
                           "err_over_bound": err / bound, "within": err <= bound})
@@ -390,8 +391,10 @@ def config2(dev, sizes=(1024, 2048, 4096, 8192), steps=3, warm=3):
     r = (b - a @ x).abs().max().item()
     berr = r / (a.abs().sum(1).max().item() * x.abs().max().item() + b.abs().max().item())
     tf = (2.0 * n ** 3 / 3.0 + 2.0 * n * n) / (ms / 1e3) / 1e12
-    return {"workload": "square GEMM C = A B, N(0,1), f32 (tcgen05 3xTF32) and f64 (DFMA); plain FP64 LU solve",
-            "peaks": {"f64_tflops": FP64_PEAK_TFLOPS, "f64_source": "GB300 FP64 rate (nominal)",
+    return {"workload": "square GEMM C = A B, N(0,1), f32 (tcgen05 3xTF32) and f64 (tcgen05, exact BF16 slices); "
+                        "plain FP64 LU solve",
+            "peaks": {"f64_tflops": ceil64, "f64_source": "MEASURED_PEAKS bf16 burst / 28 slice products, of measured",
+                      "f64_unit_tflops": FP64_PEAK_TFLOPS, "f64_unit_source": "GB300 FP64 unit (nominal)",
                       "f32_tflops": ceil32, "f32_source": "MEASURED_PEAKS bf16 burst / 2 (TF32) / 3 (3xTF32), of measured"},
             "gemm": sweep,
             "fp64_lu_solve": {"n": n, "ms": ms, "tflops": tf, "frac_of_fp64_rate": tf / FP64_PEAK_TFLOPS,
