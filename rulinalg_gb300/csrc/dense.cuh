@@ -1460,17 +1460,12 @@ static __global__ void __launch_bounds__(128) trsm_diag_kernel(const T *D, long 
 //   * the tile of A that meets the awaited block is in registers before the wait, a warp
 //     holding 8 rows and a lane the columns lane + 32 u; the products stay per lane over all
 //     blocks and are reduced once, after the last one;
-//   * the diagonal block is in shared memory from the start: as its inverse (Dinv, from
-//     diag_inverse: the solve is one more BR x BR product) or scaled by its reciprocal
-//     diagonal, so that a substitution step is one shuffle and one multiply-add;
-//   * with Link (diag_link: Dinv_b times the tile of A that meets the block solved just
-//     before b) that product is off the chain too: Dinv_b times everything else is ready when
-//     the last solution arrives, x_b = c_b - Link_b x.
+//   * the diagonal block is in shared memory from the start: as its inverse (Dinv, FP64 and one
+//     right-hand side: the solve is one more BR x BR product) or scaled by its reciprocal
+//     diagonal, so that a substitution step is one shuffle and one multiply-add.
 // BR = 128 for FP32; 64 for FP64, where the products of a tile are bound by the FP64 unit.
 // The form before (64-row blocks, a flag per block behind a fence, the folded sums through
-// shared memory) against this one, per sweep: FP32 with inverses n = 3000 132 and 52 us,
-// n = 4096 220 and 74; n = 8192 with 64 right-hand sides 2216 and 1022; FP64 by substitution
-// n = 4096 992 and 461; FP32 n = 1501 176 (substitution) and 22 (inverses).
+// shared memory) against this one, per sweep: FP64 by substitution n = 4096 992 and 461 us.
 // A CTA waits only on tickets taken before its own, by CTAs that are running, so the sweep
 // always progresses; every wait is bounded by wait_ns (RL_TUNE_WAIT_TIMEOUT_NS,
 // RL_ERR_TIMEOUT), after which the CTA goes on with zeros and publishes, so no later block
@@ -1494,7 +1489,8 @@ inline int sweep_groups(int nrhs) {
 inline int sweep_width(int nrhs) { return nrhs == 1 ? 1 : kSweepRhs; }
 template <class T>
 inline size_t sweep_ws_bytes(int n, int nrhs) {
-    return (size_t)sweep_groups(nrhs) * ((size_t)n * sweep_width(nrhs) * sizeof(T) + 16);
+    const size_t b = (size_t)sweep_groups(nrhs) * ((size_t)n * sweep_width(nrhs) * sizeof(T) + 16);
+    return (b + 15) & ~(size_t)15;  // a second workspace behind this one is aligned as well
 }
 
 __device__ __forceinline__ float sweep_peek(const float *p) {
@@ -1529,6 +1525,26 @@ __device__ __forceinline__ T sweep_get(const T *p, volatile int *fail, unsigned 
     }
     return v;
 }
+// The published values at p and p + 1 (8-byte aligned) with one load a poll; of the two the
+// first `have` are awaited, the others are 0.
+__device__ __forceinline__ float2 sweep_get2(const float *p, int have, volatile int *fail, unsigned long long limit) {
+    if (have <= 0) return make_float2(0.f, 0.f);
+    unsigned long long t0 = 0;
+    for (unsigned spin = 0;; spin++) {
+        unsigned a, b;
+        asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "l"(p) : "memory");
+        if (have < 2) b = 0u;
+        if (a != 0xffffffffu && b != 0xffffffffu) return make_float2(__uint_as_float(a), __uint_as_float(b));
+        if ((spin & 63u) == 63u) {
+            const unsigned long long t = global_ns();
+            if (t0 == 0) t0 = t;
+            if (*fail || t - t0 > limit) {
+                *fail = 1;
+                return make_float2(0.f, 0.f);
+            }
+        }
+    }
+}
 __device__ __forceinline__ void sweep_put(float *p, float v) {
     const unsigned u = __float_as_uint(v);
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(u == 0xffffffffu ? 0x7fffffffu : u) : "memory");
@@ -1550,9 +1566,10 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
                                                              int n, T *__restrict__ Y, long long ldy, int nrhs, int mode,
                                                              T *ws, int *tickets, int *status, T tiny,
                                                              unsigned long long wait_ns, int withhold,
-                                                             const T *__restrict__ Dinv, const T *__restrict__ Link) {
+                                                             const T *__restrict__ Dinv) {
     using cfg = SweepCfg<T, RW>;
     constexpr int BR = cfg::BR, CPL = cfg::CPL, LDD = cfg::LDD, THREADS = cfg::THREADS, WARPS = cfg::WARPS;
+    constexpr bool INV = sizeof(T) == 8 && RW == 1;  // the instance that is called with Dinv
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *Ds = reinterpret_cast<T *>(smem_raw);  // BR x LDD: the inverse, or the scaled diagonal block
     T *v = Ds + BR * LDD;                     // BR x RW: right-hand side minus the folded sums
@@ -1587,7 +1604,7 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
 #pragma unroll
         for (int q = 0; q < DP; q++) {
             const int e = tid + q * THREADS, i = e / BR, j = e % BR;
-            if (Dinv)
+            if (INV && Dinv)
                 dv[q] = Dinv[(long long)b * BR * BR + e];
             else
                 dv[q] = (i < bs && j < bs) ? T(A[(long long)(r0 + i) * lda + r0 + j]) : T(0);
@@ -1595,9 +1612,9 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
 #pragma unroll
         for (int q = 0; q < DP; q++) {
             const int e = tid + q * THREADS, i = e / BR, j = e % BR;
-            Ds[!Dinv && trans ? j * LDD + i : i * LDD + j] = dv[q];
+            Ds[!(INV && Dinv) && trans ? j * LDD + i : i * LDD + j] = dv[q];
         }
-        if (!Dinv) {
+        if (!(INV && Dinv)) {
             __syncthreads();
             if (tid < BR) {
                 const T d = tid < bs ? Ds[tid * LDD + tid] : T(1);
@@ -1631,27 +1648,11 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
                         t[i][u] = (wr < bs && lc < ks) ? A[(long long)(r0 + wr) * lda + c0 + lc] : TA(0);
                 }
         };
-        const int nf = Link && nk > 0 ? nk - 1 : nk;  // blocks folded before the diagonal block's product
-        auto link = [&](TA (&t)[NA][CPL]) {
-#pragma unroll
-            for (int i = 0; i < NA; i++)
-#pragma unroll
-                for (int u = 0; u < CPL; u++)
-                    t[i][u] = (TA)Link[((long long)b * BR + warp * 8 + i) * BR + lane + 32 * u];
-        };
-        if (nf > 0)
-            load(0, cur);
-        else if (nk > 0)
-            link(cur);
-        for (int kk = 0; kk < nf; kk++) {
+        if (nk > 0) load(0, cur);
+        for (int kk = 0; kk < nk; kk++) {
             // One right-hand side: the next tile is under way while this one waits. With 8
             // the sums take those registers.
-            if (RW == 1) {
-                if (kk + 1 < nf)
-                    load(kk + 1, nxt);
-                else if (nf < nk)
-                    link(nxt);
-            }
+            if (RW == 1 && kk + 1 < nk) load(kk + 1, nxt);
             const int k = fwd ? kk : nb - 1 - kk, c0 = k * BR, ks = min(BR, n - c0);
             if (RW == 1) {
                 if (!trans) {
@@ -1693,10 +1694,7 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
                             for (int c = 0; c < RW; c++) acc[i][c] = fma(T(cur[i][w0 & (CPL - 1)]), x[c], acc[i][c]);
                     }
                 }
-                if (kk + 1 < nf)
-                    load(kk + 1, cur);
-                else if (nf < nk)
-                    link(cur);
+                if (kk + 1 < nk) load(kk + 1, cur);
             }
             if (RW == 1)
 #pragma unroll
@@ -1736,7 +1734,7 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
                 Y[(long long)(r0 + i) * ldy + c] = x;
             }
         };
-        if (Dinv) {
+        if (INV && Dinv) {
             T o[8][RW];
 #pragma unroll
             for (int i = 0; i < 8; i++)
@@ -1756,51 +1754,14 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
                     for (int c = 0; c < RW; c++) o[i][c] = fma(d, x[c], o[i][c]);
                 }
             }
-            auto reduce = [&](int c) {
+#pragma unroll
+            for (int c = 0; c < RW; c++) {
                 T s8[8];
 #pragma unroll
                 for (int i = 0; i < 8; i++) s8[i] = o[i][c];
                 int row;
-                return warp_reduce_scatter<8>(s8, lane, row);
-            };
-            if (nf == nk) {
-#pragma unroll
-                for (int c = 0; c < RW; c++) {
-                    const T x = reduce(c);
-                    if ((lane & 3) == 0) publish(mrow, c, x);
-                }
-            } else {
-                T cb[RW];
-#pragma unroll
-                for (int c = 0; c < RW; c++) cb[c] = reduce(c);
-#pragma unroll
-                for (int i = 0; i < 8; i++)
-#pragma unroll
-                    for (int c = 0; c < RW; c++) o[i][c] = T(0);
-                const int k = fwd ? b - 1 : b + 1, c0 = k * BR, ks = min(BR, n - c0);
-                if (RW > 1) {
-                    for (int e = tid; e < BR * RW; e += THREADS)
-                        xs[e] = e < ks * RW && e % RW < nrhs ? sweep_get(ws + (size_t)c0 * RW + e, &s_fail, wait_ns) : T(0);
-                    __syncthreads();
-                }
-#pragma unroll
-                for (int u = 0; u < CPL; u++) {
-                    const int lc = lane + 32 * u;
-                    T x[RW];
-                    if constexpr (RW == 1)
-                        x[0] = lc < ks ? sweep_get(ws + c0 + lc, &s_fail, wait_ns) : T(0);
-                    else
-                        ldv<RW>(xs + lc * RW, x);
-#pragma unroll
-                    for (int i = 0; i < 8; i++)
-#pragma unroll
-                        for (int c = 0; c < RW; c++) o[i][c] = fma(T(cur[i][u]), x[c], o[i][c]);
-                }
-#pragma unroll
-                for (int c = 0; c < RW; c++) {
-                    const T x = cb[c] - reduce(c);
-                    if ((lane & 3) == 0) publish(mrow, c, x);
-                }
+                const T x = warp_reduce_scatter<8>(s8, lane, row);
+                if ((lane & 3) == 0) publish(mrow, c, x);
             }
         } else if (warp < RW) {
             // substitution with the scaled rows: warp c solves right-hand side c, lane l
@@ -1833,6 +1794,179 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
 #pragma unroll
             for (int h = 0; h < CPL; h++) publish(lane + 32 * h, c, z[h]);
         }
+        if (tid == 0 && *(volatile int *)&s_fail) atomicCAS(status, 0, RL_ERR_TIMEOUT);
+    }
+}
+
+// The FP32 sweep with inverted 64 x 64 diagonal blocks (Dinv, from diag_inverse_kernel): the
+// refinement of the mixed single-system solvers, RW = 1 or 8 right-hand sides a group. Which
+// step of a refinement passes its test hangs on the last bits of every correction at the edge
+// of the test, and whether it converges on how far the inverses are from the triangle's, so the
+// block size and the order of the sums are part of the results and are fixed here: thread (row,
+// quarter) of a block adds the products with its 16 columns of every block solved before, in
+// solve order; the quarters are added as (0 + 1) + (2 + 3), in the L^T mode as
+// ((0 + 1) + 2) + 3; v = y - sums; x_b = Dinv_b v in the same quarters. (With 128-row blocks and
+// the sums spread over the lanes 2 of 8 systems of kappa = 1e6, n = 4096, ended a step sooner,
+// with an error of 5e-9 in place of 5e-10, and systems made of Hadamard factors, which converge
+// here in 10 to 16 steps, went to the FP64 fallback.)
+// The chain from one block's solutions to the next one's is what it takes: the solutions are
+// polled in place (ws as in trsv_sweep_kernel), two values a lane in one load, by each warp for
+// itself without a CTA barrier (RW = 1) or once per CTA; the tiles of A are in registers
+// kInvDepth blocks ahead; a thread's share of Dinv and of the right-hand side is loaded before
+// the fold.
+// Per sweep, with the 128-row form before: n = 3000 47 us (45), 4096 64 (61.5), 16384 333 (296);
+// n = 2048 with 8 right-hand sides 62 (65), n = 8192 with 64 508 (665; the CTAs of all 8 groups
+// resident from the start, with the grid in group order 970). Tiles 4 blocks ahead: the same for
+// one right-hand side, 658 for 64 (registers).
+constexpr int kInvRows = 64, kInvDepth = 2;
+template <int RW>
+static __global__ void __launch_bounds__(256) trsv_inv_kernel(const float *__restrict__ A, long long lda, int n,
+                                                              float *__restrict__ Y, long long ldy, int nrhs, int mode,
+                                                              float *ws, int *tickets, int *status,
+                                                              unsigned long long wait_ns, int withhold,
+                                                              const float *__restrict__ Dinv) {
+    constexpr int BR = kInvRows, DEPTH = kInvDepth, OWN = RW == 1 ? 1 : 2;  // OWN: columns a thread ends with
+    // A quarter's 16 x RW values, 16 bytes further for each quarter: the four quarters of a warp
+    // read from different banks.
+    constexpr int QS = 16 * RW + 4;
+    __shared__ __align__(16) float xs[RW == 1 ? 8 : 1][2][4 * QS];  // the awaited solutions (RW = 1: a warp's copy)
+    __shared__ __align__(16) float v[4 * QS];
+    __shared__ float red[4][BR][RW];  // the quarters' sums (L^T)
+    __shared__ int s_t, s_fail;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nb = (n + BR - 1) / BR;
+    const bool fwd = mode <= 1, trans = mode == 3;
+    const bool vec = !trans && (lda & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+    const int rr = tid >> 2, qq = tid & 3;                                 // row and quarter of the block's product
+    const int r = trans ? tid & (BR - 1) : rr, q = trans ? tid >> 6 : qq;  // and of the fold
+    Y += (long long)blockIdx.y * RW;
+    nrhs = min(RW, nrhs - (int)blockIdx.y * RW);
+    ws += (size_t)blockIdx.y * n * RW;
+    const int c0y = RW == 1 ? 0 : 2 * qq, own = RW == 1 ? (qq == 0 ? 1 : 0) : min(2, nrhs - c0y);
+    if (tid == 0) s_fail = 0;
+    for (;;) {
+        __syncthreads();  // the previous block's shared state is no longer read
+        if (tid == 0) s_t = atomicAdd(tickets + blockIdx.y, 1) + 1;  // preset to -1
+        __syncthreads();
+        if (s_t >= nb) break;
+        const int b = fwd ? s_t : nb - 1 - s_t, r0 = b * BR, bs = min(BR, n - r0);
+        const int nk = fwd ? b : nb - 1 - b;  // blocks solved before this one
+        float d[16], t[DEPTH][16], acc[RW], y[OWN];
+        ldv<16>(Dinv + ((long long)b * BR + rr) * BR + qq * 16, d);
+#pragma unroll
+        for (int c = 0; c < OWN; c++) y[c] = c < own && rr < bs ? Y[(long long)(r0 + rr) * ldy + c0y + c] : 0.f;
+        auto load = [&](int kk, float (&o)[16]) {
+            const int c0 = (fwd ? kk : nb - 1 - kk) * BR, ks = min(BR, n - c0);
+            if (vec && ks == BR) {
+                if (r < bs) {
+                    ldv<16>(A + (long long)(r0 + r) * lda + c0 + q * 16, o);
+                } else {
+#pragma unroll
+                    for (int jj = 0; jj < 16; jj++) o[jj] = 0.f;
+                }
+                return;
+            }
+#pragma unroll
+            for (int jj = 0; jj < 16; jj++) {
+                const int j = q * 16 + jj;
+                o[jj] = (r < bs && j < ks) ? (trans ? A[(long long)(c0 + j) * lda + r0 + r] : A[(long long)(r0 + r) * lda + c0 + j])
+                                           : 0.f;
+            }
+        };
+        // 16 terms of every column's sum: a times the quarter's values at p
+        auto dot16 = [&](const float (&a)[16], const float *p, float (&o)[RW]) {
+            if constexpr (RW == 1) {
+                float x[16];
+                ldv<16>(p, x);
+#pragma unroll
+                for (int jj = 0; jj < 16; jj++) o[0] = fmaf(a[jj], x[jj], o[0]);
+            } else {
+#pragma unroll
+                for (int jj = 0; jj < 16; jj++) {
+                    float x[RW];
+                    ldv<RW>(p + jj * RW, x);
+#pragma unroll
+                    for (int c = 0; c < RW; c++) o[c] = fmaf(a[jj], x[c], o[c]);
+                }
+            }
+        };
+#pragma unroll
+        for (int u = 0; u < DEPTH; u++)
+            if (u < nk) load(u, t[u]);
+#pragma unroll
+        for (int c = 0; c < RW; c++) acc[c] = 0.f;
+        for (int k0 = 0; k0 < nk; k0 += DEPTH) {
+#pragma unroll
+            for (int u = 0; u < DEPTH; u++) {
+                const int kk = k0 + u;
+                if (kk >= nk) break;
+                const int c0 = (fwd ? kk : nb - 1 - kk) * BR, ks = min(BR, n - c0);
+                // A buffer of the two is written again only after the barrier that follows the
+                // reads of the other.
+                float *w = xs[RW == 1 ? warp : 0][u & 1];
+                if constexpr (RW == 1) {
+                    const int p = 2 * lane + (trans ? 16 * q : 0);  // L^T: the quarter's 16 are enough
+                    if (!trans || lane < 8)
+                        *reinterpret_cast<float2 *>(w + (p >> 4) * QS + (p & 15)) =
+                            sweep_get2(ws + c0 + p, ks - p, &s_fail, wait_ns);
+                    __syncwarp();
+                } else {
+                    *reinterpret_cast<float2 *>(w + (rr >> 4) * QS + (rr & 15) * RW + c0y) =
+                        sweep_get2(ws + (size_t)(c0 + rr) * RW + c0y, rr < ks ? own : 0, &s_fail, wait_ns);
+                    __syncthreads();
+                }
+                dot16(t[u], w + q * QS, acc);
+                if (kk + DEPTH < nk) load(kk + DEPTH, t[u]);
+            }
+        }
+        // the quarters' sums of this thread's columns: (0 + 1) + (2 + 3)
+        auto quarters = [&](float (&o)[RW], float (&out)[OWN]) {
+            if constexpr (RW == 1) {
+                o[0] += __shfl_xor_sync(0xffffffffu, o[0], 1);
+                out[0] = o[0] + __shfl_xor_sync(0xffffffffu, o[0], 2);
+            } else {  // lane q keeps the columns 2 q, 2 q + 1 and gives the others away
+                const bool odd = qq & 1, high = qq & 2;
+                float h[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int e = (i & 1) + 4 * (i >> 1);  // columns 0 1 4 5, and 2 3 6 7 of an odd lane
+                    const float keep = odd ? o[e + 2] : o[e], give = odd ? o[e] : o[e + 2];
+                    h[i] = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+                }
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const float keep = high ? h[i + 2] : h[i], give = high ? h[i] : h[i + 2];
+                    out[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+                }
+            }
+        };
+        float *vo = v + (rr >> 4) * QS + (rr & 15) * RW + c0y, sum[OWN];
+        if (!trans) {
+            quarters(acc, sum);
+        } else {
+#pragma unroll
+            for (int c = 0; c < RW; c++) red[q][r][c] = acc[c];
+            __syncthreads();
+#pragma unroll
+            for (int c = 0; c < OWN; c++)
+                sum[c] = (((0.f + red[0][rr][c0y + c]) + red[1][rr][c0y + c]) + red[2][rr][c0y + c]) + red[3][rr][c0y + c];
+        }
+        if (RW > 1 || qq == 0)
+#pragma unroll
+            for (int c = 0; c < OWN; c++) vo[c] = y[c] - sum[c];
+        __syncthreads();
+        float x[RW], xo[OWN];
+#pragma unroll
+        for (int c = 0; c < RW; c++) x[c] = 0.f;
+        dot16(d, v + qq * QS, x);
+        quarters(x, xo);
+        if (rr < bs)
+#pragma unroll
+            for (int c = 0; c < OWN; c++)
+                if (c < own) {
+                    if (b != withhold) sweep_put(ws + (size_t)(r0 + rr) * RW + c0y + c, xo[c]);
+                    Y[(long long)(r0 + rr) * ldy + c0y + c] = xo[c];
+                }
         if (tid == 0 && *(volatile int *)&s_fail) atomicCAS(status, 0, RL_ERR_TIMEOUT);
     }
 }
@@ -1878,115 +2012,6 @@ static __global__ void __launch_bounds__(64) diag_inverse_kernel(const TA *__res
     __syncthreads();
     T *out = Dinv + (long long)b * BR * BR;
     for (int idx = j; idx < BR * BR; idx += blockDim.x) out[idx] = X[idx / BR][idx % BR];
-}
-
-// The inverses of 128 x 128 diagonal blocks from those of their 64 x 64 halves (D64, from
-// diag_inverse_kernel): [X1 0; -X2 M X1, X2] for a lower op(D), [X1, -X1 M X2; 0 X2] for an
-// upper one, M the off-diagonal 64 x 64 block. One CTA per block.
-template <class T, class TA>
-static __global__ void __launch_bounds__(256) diag_join_kernel(const TA *__restrict__ A, long long lda, int n, int mode,
-                                                           const T *__restrict__ D64, T *__restrict__ Dinv) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *X = reinterpret_cast<T *>(smem_raw), *Z = X + 64 * 65, *M = Z + 64 * 65, *P = M + 64 * 65;
-    const int b = blockIdx.x, r0 = b * 128, tid = threadIdx.x;
-    const bool lower = mode <= 1;
-    const int nb64 = (n + 63) / 64;
-    for (int e = tid; e < 64 * 64; e += 256) {
-        const int i = e / 64, j = e % 64;
-        X[i * 65 + j] = D64[(long long)(2 * b) * 4096 + e];
-        Z[i * 65 + j] = 2 * b + 1 < nb64 ? D64[(long long)(2 * b + 1) * 4096 + e] : T(0);
-        // op(D) at (64 + i, j) (lower) or (i, 64 + j) (upper)
-        const int oi = r0 + (lower ? 64 + i : i), oj = r0 + (lower ? j : 64 + j);
-        T m = T(0);
-        if (oi < n && oj < n) m = T(mode == 3 ? A[(long long)oj * lda + oi] : A[(long long)oi * lda + oj]);
-        M[i * 65 + j] = m;
-    }
-    __syncthreads();
-    const T *first = lower ? X : Z, *second = lower ? Z : X;  // -second (M first)
-    const int tx = tid & 15, ty = tid >> 4;
-    auto product = [&](const T *l, const T *r, T (&o)[4][4]) {
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) o[i][j] = T(0);
-        for (int k = 0; k < 64; k++) {
-            T li[4], rj[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) li[i] = l[(ty + 16 * i) * 65 + k], rj[i] = r[k * 65 + tx + 16 * i];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) o[i][j] = fma(li[i], rj[j], o[i][j]);
-        }
-    };
-    T o[4][4];
-    product(M, first, o);
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) P[(ty + 16 * i) * 65 + tx + 16 * j] = o[i][j];
-    __syncthreads();
-    product(second, P, o);
-    T *out = Dinv + (long long)b * 128 * 128;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int r = ty + 16 * i, c = tx + 16 * j;
-            out[(lower ? 64 + r : r) * 128 + (lower ? c : 64 + c)] = -o[i][j];
-            out[(lower ? r : 64 + r) * 128 + (lower ? 64 + c : c)] = T(0);
-            out[r * 128 + c] = X[r * 65 + c];
-            out[(64 + r) * 128 + 64 + c] = Z[r * 65 + c];
-        }
-}
-
-// Link_b = Dinv_b op(A)_{b, b'} for the sweep, b' the block solved just before b (b - 1 for the
-// lower modes, b + 1 for the upper ones); 128 x 128 row-major per block, zero beyond n. Grid
-// (blocks, 4): a 64 x 64 quadrant per CTA, the K = 128 products in two halves.
-template <class T, class TA>
-static __global__ void __launch_bounds__(256) diag_link_kernel(const TA *__restrict__ A, long long lda, int n, int mode,
-                                                           const T *__restrict__ Dinv, T *__restrict__ Link) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *X = reinterpret_cast<T *>(smem_raw), *M = X + 64 * 65;
-    const int nb = (n + 127) / 128, b = blockIdx.x, bp = mode <= 1 ? b - 1 : b + 1;
-    if (bp < 0 || bp >= nb) return;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int i0 = (blockIdx.y >> 1) * 64, j0 = (blockIdx.y & 1) * 64, r0 = b * 128, c0 = bp * 128;
-    T o[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) o[i][j] = T(0);
-    for (int h = 0; h < 128; h += 64) {
-        __syncthreads();
-#pragma unroll 8
-        for (int e = tid; e < 64 * 64; e += 256) {
-            const int i = e >> 6, j = e & 63;
-            X[i * 65 + j] = Dinv[((long long)b * 128 + i0 + i) * 128 + h + j];
-            if (mode == 3) {  // op(A)[r][c] = A[c][r]: consecutive threads along r
-                const int r = r0 + h + j, c = c0 + j0 + i;
-                M[j * 65 + i] = (r < n && c < n) ? T(A[(long long)c * lda + r]) : T(0);
-            } else {
-                const int r = r0 + h + i, c = c0 + j0 + j;
-                M[i * 65 + j] = (r < n && c < n) ? T(A[(long long)r * lda + c]) : T(0);
-            }
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int k = 0; k < 64; k++) {
-            T li[4], rj[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) li[i] = X[(ty + 16 * i) * 65 + k], rj[i] = M[k * 65 + tx + 16 * i];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) o[i][j] = fma(li[i], rj[j], o[i][j]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) Link[((long long)b * 128 + i0 + ty + 16 * i) * 128 + j0 + tx + 16 * j] = o[i][j];
 }
 
 // Row-wise solve X D^T = Y for the rows of Y (m x bs, stride ldy), D lower bs x bs: the

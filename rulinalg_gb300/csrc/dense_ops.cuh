@@ -553,11 +553,12 @@ rl_status qr_apply_q_dev(const T *QR, long long lda, int m, int n, const T *tau,
     return RL_OK;
 }
 
-// One launch of the triangular sweep: the 1-wide instance for one right-hand side (the
-// 8-wide one would issue 8 FMAs per element, 7 of them predicated off, each a full issue of
-// the FP64 pipe for T = double). ws as trsv_sweep_kernel takes it.
+// One launch of the triangular sweep by substitution, or (FP64, one right-hand side) with the
+// inverted diagonal blocks Dinv: the 1-wide instance for one right-hand side (the 8-wide one would
+// issue 8 FMAs per element, 7 of them predicated off, each a full issue of the FP64 pipe for T =
+// double). ws as trsv_sweep_kernel takes it.
 template <class T, class TA, int RW>
-static rl_status sweep_launch_w(const TA *A, long long lda, int n, const T *Dinv, const T *Link, T *Y, long long ldy, int nrhs, int mode,
+static rl_status sweep_launch_w(const TA *A, long long lda, int n, const T *Dinv, T *Y, long long ldy, int nrhs, int mode,
                                 int *dstatus, cudaStream_t s, T tiny, void *ws) {
     using cfg = SweepCfg<T, RW>;
     auto kern = trsv_sweep_kernel<T, TA, RW>;
@@ -572,14 +573,31 @@ static rl_status sweep_launch_w(const TA *A, long long lda, int n, const T *Dinv
     int *tickets = reinterpret_cast<int *>(x + (size_t)groups * n * RW);
     const dim3 grid(std::min(nb, std::max(1, per_sm) * num_sms()), groups);
     RL_LAUNCH(kern, grid, cfg::THREADS, cfg::SMEM, s, A, lda, n, Y, ldy, nrhs, mode, x, tickets, dstatus, tiny, wait_ns(),
-              (int)tune(RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK), Dinv, Link);
+              (int)tune(RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK), Dinv);
     return RL_OK;
 }
 template <class T, class TA>
-rl_status sweep_launch(const TA *A, long long lda, int n, const T *Dinv, const T *Link, T *Y, long long ldy, int nrhs, int mode, int *dstatus,
-                       cudaStream_t s, T tiny, void *ws) {
-    return sweep_width(nrhs) == 1 ? sweep_launch_w<T, TA, 1>(A, lda, n, Dinv, Link, Y, ldy, nrhs, mode, dstatus, s, tiny, ws)
-                                  : sweep_launch_w<T, TA, kSweepRhs>(A, lda, n, Dinv, Link, Y, ldy, nrhs, mode, dstatus, s, tiny, ws);
+static rl_status sweep_launch(const TA *A, long long lda, int n, const T *Dinv, T *Y, long long ldy, int nrhs, int mode,
+                              int *dstatus, cudaStream_t s, T tiny, void *ws) {
+    return sweep_width(nrhs) == 1 ? sweep_launch_w<T, TA, 1>(A, lda, n, Dinv, Y, ldy, nrhs, mode, dstatus, s, tiny, ws)
+                                  : sweep_launch_w<T, TA, kSweepRhs>(A, lda, n, Dinv, Y, ldy, nrhs, mode, dstatus, s, tiny, ws);
+}
+
+// One launch of trsv_inv_kernel (FP32, inverted diagonal blocks); ws as above.
+template <int RW>
+static rl_status sweep_inv_launch(const float *A, long long lda, int n, const float *Dinv, float *Y, long long ldy, int nrhs,
+                                  int mode, int *dstatus, cudaStream_t s, void *ws) {
+    static int per_sm = 0;
+    static const cudaError_t q = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trsv_inv_kernel<RW>, 256, 0);
+    RL_TRY_CUDA(q);
+    const int groups = sweep_groups(nrhs), nb = ceil_div(n, kInvRows);
+    float *x = static_cast<float *>(ws);
+    int *tickets = reinterpret_cast<int *>(x + (size_t)groups * n * RW);
+    // every group's chain runs from the start: the CTAs that fit are shared out over the groups
+    const dim3 grid(std::min(nb, std::max(1, std::max(1, per_sm) * num_sms() / groups)), groups);
+    RL_LAUNCH(trsv_inv_kernel<RW>, grid, 256, 0, s, A, lda, n, Y, ldy, nrhs, mode, x, tickets, dstatus, wait_ns(),
+              (int)tune(RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK), Dinv);
+    return RL_OK;
 }
 
 // Blocked triangular solve op(A) X = Y in place (A n x n, Y n x nrhs).
@@ -633,7 +651,7 @@ rl_status tri_solve_dev(const TA *A, long long lda, int n, T *Y, long long ldy, 
         DevBuf<unsigned char> ws;
         RL_TRY(ws.alloc(sweep_ws_bytes<T>(n, nrhs), s));
         RL_TRY_CUDA(cudaMemsetAsync(ws.p, 0xff, sweep_ws_bytes<T>(n, nrhs), s));
-        return sweep_launch<T, TA>(A, lda, n, nullptr, nullptr, Y, ldy, nrhs, mode, dstatus, s, tiny, ws.p);
+        return sweep_launch<T, TA>(A, lda, n, nullptr, Y, ldy, nrhs, mode, dstatus, s, tiny, ws.p);
     }
     if constexpr (!std::is_same<T, TA>::value) {
         return RL_ERR_INVALID_ARG;  // mixed storage: few right-hand sides only
@@ -669,50 +687,32 @@ rl_status tri_solve_dev(const TA *A, long long lda, int n, T *Y, long long ldy, 
     }
 }
 
-// Inverses of op(A)'s diagonal blocks of sweep_rows<T>() rows, formed in T (row-major blocks
-// in Dinv, diag_inverse_elems<T>(n) values; zero beyond a partial last block).
-template <class T>
-inline size_t diag_inverse_elems(int n) {
-    return (size_t)ceil_div(n, sweep_rows<T>()) * sweep_rows<T>() * sweep_rows<T>();
-}
+// Inverses of op(A)'s 64 x 64 diagonal blocks, formed in T (ceil(n / 64) row-major blocks in Dinv,
+// zero beyond a partial last one; diag_inverse_kernel).
+inline size_t diag_inverse_elems(int n) { return (size_t)ceil_div(n, kInvRows) * kInvRows * kInvRows; }
 template <class T, class TA>
 rl_status diag_inverse(const TA *A, long long lda, int n, int mode, T *Dinv, int *dstatus, cudaStream_t s, T tiny) {
     if (n <= 0) return RL_OK;
-    const int nb64 = ceil_div(n, 64);
-    if constexpr (sweep_rows<T>() == 64) {
-        RL_LAUNCH((diag_inverse_kernel<T, TA>), nb64, 64, 0, s, A, lda, n, mode, Dinv, dstatus, tiny);
-    } else {
-        DevBuf<T> half;
-        RL_TRY(half.alloc((size_t)nb64 * 64 * 64, s));
-        RL_LAUNCH((diag_inverse_kernel<T, TA>), nb64, 64, 0, s, A, lda, n, mode, half.p, dstatus, tiny);
-        const size_t smem = 4 * 64 * 65 * sizeof(T);
-        RL_TRY(set_smem(diag_join_kernel<T, TA>, smem));
-        RL_LAUNCH((diag_join_kernel<T, TA>), ceil_div(n, 128), 256, smem, s, A, lda, n, mode, half.p, Dinv);
-    }
+    RL_LAUNCH((diag_inverse_kernel<T, TA>), ceil_div(n, kInvRows), 64, 0, s, A, lda, n, mode, Dinv, dstatus, tiny);
     return RL_OK;
 }
 
-// Link of a triangle whose diagonal blocks are inverted (FP32: 128-row blocks), as many values.
-template <class TA>
-rl_status diag_link(const TA *A, long long lda, int n, int mode, const float *Dinv, float *Link, cudaStream_t s) {
-    const size_t smem = 2 * 64 * 65 * sizeof(float);
-    RL_LAUNCH((diag_link_kernel<float, TA>), dim3(ceil_div(n, 128), 4), 256, smem, s, A, lda, n, mode, Dinv, Link);
-    return RL_OK;
-}
-
-// op(A) Y = Y' for at most kSweepGroups x kSweepRhs right-hand sides in one sweep launch
-// whose block solves are products with the diagonal blocks' inverses Dinv
-// (diag_inverse; Link: their products with the tiles of A before them, diag_link, or null).
-// ws: sweep_ws_bytes<T>(n, nrhs) bytes with all bits set. More right-hand
-// sides, or a GPU shared with other streams of this library (the serving workers, see
-// tri_solve_dev), take tri_solve_dev's substitution paths instead.
+// op(A) Y = Y' in one sweep launch whose block solves are products with the diagonal blocks'
+// inverses Dinv (diag_inverse): FP32 with at most kSweepGroups x kSweepRhs right-hand sides, or FP64
+// with one. ws: sweep_ws_bytes<T>(n, nrhs) bytes with all bits set. More right-hand sides, or a GPU
+// shared with other streams of this library (the serving workers, see tri_solve_dev), take
+// tri_solve_dev's substitution paths instead.
 template <class T, class TA>
-rl_status tri_solve_inv_dev(const TA *A, long long lda, int n, const T *Dinv, const T *Link, T *Y, long long ldy, int nrhs,
-                            int mode, int *dstatus, cudaStream_t s, T tiny, void *ws) {
+rl_status tri_solve_inv_dev(const TA *A, long long lda, int n, const T *Dinv, T *Y, long long ldy, int nrhs, int mode,
+                            int *dstatus, cudaStream_t s, T tiny, void *ws) {
     if (sweep_groups(nrhs) == 0 || g_shared_gpu)
         return tri_solve_dev<T, TA>(A, lda, n, Y, ldy, nrhs, mode, dstatus, s, tiny);
     if (n <= 0 || nrhs <= 0) return RL_OK;
-    return sweep_launch<T, TA>(A, lda, n, Dinv, Link, Y, ldy, nrhs, mode, dstatus, s, tiny, ws);
+    if constexpr (std::is_same<T, double>::value)
+        return sweep_launch_w<T, TA, 1>(A, lda, n, Dinv, Y, ldy, nrhs, mode, dstatus, s, tiny, ws);
+    else
+        return nrhs == 1 ? sweep_inv_launch<1>(A, lda, n, Dinv, Y, ldy, nrhs, mode, dstatus, s, ws)
+                         : sweep_inv_launch<kSweepRhs>(A, lda, n, Dinv, Y, ldy, nrhs, mode, dstatus, s, ws);
 }
 
 // Solve with factors already on the device. kind 0 = LU (dperm: stored permutation),

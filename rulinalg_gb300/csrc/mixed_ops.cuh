@@ -62,7 +62,7 @@ inline rl_status colnorm_dev(const double *V, long long ldv, int n, int nrhs, un
 // Inverted diagonal blocks of the two triangles of an FP32 factor (FP32, formed once) and
 // the workspace of the sweeps that use them: the form of RL_TUNE_MIXED_SWEEP_INV.
 struct SweepInv {
-    const float *D1 = nullptr, *D2 = nullptr, *L1 = nullptr, *L2 = nullptr;  // inverses, links
+    const float *D1 = nullptr, *D2 = nullptr;
     unsigned char *ws = nullptr;  // 2 x sweep_ws_bytes<float>(n, nrhs), set before each pair of sweeps
 };
 
@@ -78,8 +78,8 @@ inline rl_status precond_solve(const float *F, int n, int kind, float *W, long l
     if (inv.D1 && sweep_groups(nrhs) > 0) {
         const size_t bytes = sweep_ws_bytes<float>(n, nrhs);
         RL_TRY_CUDA(cudaMemsetAsync(inv.ws, 0xff, 2 * bytes, s));
-        RL_TRY((tri_solve_inv_dev<float, float>(F, n, n, inv.D1, inv.L1, W, ldw, nrhs, m1, dstatus, s, tiny, inv.ws)));
-        return tri_solve_inv_dev<float, float>(F, n, n, inv.D2, inv.L2, W, ldw, nrhs, m2, dstatus, s, tiny, inv.ws + bytes);
+        RL_TRY((tri_solve_inv_dev<float, float>(F, n, n, inv.D1, W, ldw, nrhs, m1, dstatus, s, tiny, inv.ws)));
+        return tri_solve_inv_dev<float, float>(F, n, n, inv.D2, W, ldw, nrhs, m2, dstatus, s, tiny, inv.ws + bytes);
     }
     RL_TRY(tri_solve_dev<float>(F, n, n, W, ldw, nrhs, m1, dstatus, s, tiny));
     return tri_solve_dev<float>(F, n, n, W, ldw, nrhs, m2, dstatus, s, tiny);
@@ -123,8 +123,8 @@ struct Minv {
     int mode1() const { return kind == RL_KIND_LU ? 0 : 1; }
     int mode2() const { return kind == RL_KIND_LU ? 2 : 3; }
     rl_status init(cudaStream_t s) {
-        RL_TRY(D1.alloc(diag_inverse_elems<double>(n), s));
-        RL_TRY(D2.alloc(diag_inverse_elems<double>(n), s));
+        RL_TRY(D1.alloc(diag_inverse_elems(n), s));
+        RL_TRY(D2.alloc(diag_inverse_elems(n), s));
         RL_TRY(ws.alloc(2 * sweep_ws_bytes<double>(n, 1), s));
         RL_TRY((diag_inverse<double, float>(F, n, n, mode1(), D1.p, dstatus, s, FLT_MIN)));
         return diag_inverse<double, float>(F, n, n, mode2(), D2.p, dstatus, s, FLT_MIN);
@@ -137,8 +137,8 @@ struct Minv {
             RL_TRY_CUDA(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
         const size_t bytes = sweep_ws_bytes<double>(n, 1);
         RL_TRY_CUDA(cudaMemsetAsync(ws.p, 0xff, 2 * bytes, s));
-        RL_TRY((tri_solve_inv_dev<double, float>(F, n, n, D1.p, (const double *)nullptr, dst, 1, 1, mode1(), dstatus, s, tiny, ws.p)));
-        return tri_solve_inv_dev<double, float>(F, n, n, D2.p, (const double *)nullptr, dst, 1, 1, mode2(), dstatus, s, tiny, ws.p + bytes);
+        RL_TRY((tri_solve_inv_dev<double, float>(F, n, n, D1.p, dst, 1, 1, mode1(), dstatus, s, tiny, ws.p)));
+        return tri_solve_inv_dev<double, float>(F, n, n, D2.p, dst, 1, 1, mode2(), dstatus, s, tiny, ws.p + bytes);
     }
 };
 
@@ -351,26 +351,23 @@ struct MixedFactor {
         F64 = nullptr, ipiv64 = nullptr, rows64 = nullptr, Dinv = nullptr;
     }
 
-    size_t dinv_elems() const { return diag_inverse_elems<float>(n); }
+    size_t dinv_elems() const { return diag_inverse_elems(n); }
 
     size_t bytes() const {
         size_t b = (size_t)n * n * sizeof(float) + 2 * (size_t)n * sizeof(int);
         if (A_own) b += (size_t)n * n * sizeof(double);
         if (F64) b += (size_t)n * n * sizeof(double) + 2 * (size_t)n * sizeof(int);
-        if (Dinv) b += 4 * dinv_elems() * sizeof(float);
+        if (Dinv) b += 2 * dinv_elems() * sizeof(float);
         return b;
     }
 
     // The inverted diagonal blocks for the sweeps (formed on first use).
     rl_status ensure_dinv(int *dstatus, cudaStream_t s) {
         if (Dinv) return RL_OK;
-        RL_TRY(alloc(Dinv, 4 * dinv_elems(), s));  // both triangles' inverses, then their links
+        RL_TRY(alloc(Dinv, 2 * dinv_elems(), s));
         const int m1 = kind == RL_KIND_LU ? 0 : 1, m2 = kind == RL_KIND_LU ? 2 : 3;
-        const size_t de = dinv_elems();
         RL_TRY((diag_inverse<float, float>(F, n, n, m1, Dinv, dstatus, s, FLT_MIN)));
-        RL_TRY((diag_inverse<float, float>(F, n, n, m2, Dinv + de, dstatus, s, FLT_MIN)));
-        RL_TRY(diag_link<float>(F, n, n, m1, Dinv, Dinv + 2 * de, s));
-        return diag_link<float>(F, n, n, m2, Dinv + de, Dinv + 3 * de, s);
+        return diag_inverse<float, float>(F, n, n, m2, Dinv + dinv_elems(), dstatus, s, FLT_MIN);
     }
 
     template <class T>
@@ -481,8 +478,7 @@ struct MixedFactor {
         if (tune(RL_TUNE_MIXED_SWEEP_INV) && sweep_groups(nrhs) > 0 && n > CTA_NMAX && !g_shared_gpu) {
             RL_TRY(ensure_dinv(dstatus, s));
             RL_TRY(sweep_ws.alloc(2 * sweep_ws_bytes<float>(n, nrhs), s));
-            const size_t de = dinv_elems();
-            inv = SweepInv{Dinv, Dinv + de, Dinv + 2 * de, Dinv + 3 * de, sweep_ws.p};
+            inv = SweepInv{Dinv, Dinv + dinv_elems(), sweep_ws.p};
         }
         std::vector<int> act(nrhs + 1, 1);
         RL_TRY_CUDA(cudaMemcpyAsync(active.p, act.data(), act.size() * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -690,14 +686,12 @@ inline rl_status lstsq_mixed(const double *A, long long lda, int m, int n, const
     DevBuf<unsigned char> sweep_ws;
     SweepInv inv;
     if (tune(RL_TUNE_MIXED_SWEEP_INV) && n > CTA_NMAX && !g_shared_gpu) {
-        const size_t de = diag_inverse_elems<float>(n);
-        RL_TRY(Dinv.alloc(4 * de, s));
+        const size_t de = diag_inverse_elems(n);
+        RL_TRY(Dinv.alloc(2 * de, s));
         RL_TRY(sweep_ws.alloc(2 * sweep_ws_bytes<float>(n, 1), s));
         RL_TRY((diag_inverse<float, float>(L.p, n, n, 1, Dinv.p, dstatus.p, s, FLT_MIN)));
         RL_TRY((diag_inverse<float, float>(L.p, n, n, 3, Dinv.p + de, dstatus.p, s, FLT_MIN)));
-        RL_TRY(diag_link<float>(L.p, n, n, 1, Dinv.p, Dinv.p + 2 * de, s));
-        RL_TRY(diag_link<float>(L.p, n, n, 3, Dinv.p + de, Dinv.p + 3 * de, s));
-        inv = SweepInv{Dinv.p, Dinv.p + de, Dinv.p + 2 * de, Dinv.p + 3 * de, sweep_ws.p};
+        inv = SweepInv{Dinv.p, Dinv.p + de, sweep_ws.p};
     }
     Minv32 M{L.p, n, w32.p, bits.p + 2, one.p, dstatus.p, inv};
     GemvT At{partial.p, chunks, rows_per};
