@@ -316,6 +316,14 @@ rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T 
     DgemmTcTiles left;
     if constexpr (std::is_same<T, double>::value) {  // FP64 with enough work: exact slices on the tensor cores
         bool taken = false;
+        const int max_k = dgemm_tc_eligible(m, n, k) ? dgemm_tc_max_k(m, n, LOWER) : k;
+        if (k > max_k) {  // equal parts of K, added into C in order
+            const int part = ceil_div(ceil_div(k, ceil_div(k, max_k)), tc64::BK) * tc64::BK;
+            for (int p = 0; p < k; p += part)
+                RL_TRY((gemm<T, TA, TB, LOWER>(m, n, std::min(part, k - p), alpha, A + (TA ? p * lda : (long long)p), lda,
+                                               B + (TB ? (long long)p : p * ldb), ldb, p ? T(1) : beta, C, ldc, stream)));
+            return RL_OK;
+        }
         if (dgemm_tc_eligible(m, n, k))
             RL_TRY((dgemm_tc<TA, TB>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, LOWER, stream, ws, left, taken)));
         // what follows computes the tiles that were left (usually none), or all of C

@@ -12,7 +12,9 @@
 // i + j <= 7, 36 of them (63 bits); group g = i + j carries the weight 2^(-14 - 8g).
 // Groups 0 .. 4 are sums of integers below 2^24 in magnitude as long as a tensor-memory
 // accumulator covers K <= 192 (5 pairs x 192 x 2^14 < 2^24), so FP32 accumulation is exact;
-// after each 192 they are read back and added exactly into 64-bit integers. The groups
+// after each 192 they are read back and added exactly into 64-bit integers, which hold the
+// 2^46 sum of a 2^-E b 2^-F over 65,536 columns (MAX_K, half of their range); a longer K is cut
+// into products of at most that many columns per CTA, added into C one after another. The groups
 // after them share one accumulator, read back with them and summed in FP32: the tensor
 // core's truncation leaves about 2^-55 2^(E_i + F_j) per 192 columns of K there, a seventh of
 // that with the 36 products' read-back after every 64.
@@ -50,6 +52,7 @@ constexpr int PLANES = NS + 1;                                // the digits and 
 constexpr int SUPER7 = 6, SUPER8 = 2;                         // K chunks per drain: 192 / 64
 constexpr int A_TILE = BM * BK * 2;                           // one slice tile: 8 KB
 constexpr int DRAIN_WARPS = 8, THREADS = 32 * (DRAIN_WARPS + 2);
+constexpr int MAX_K = 65536;                                  // columns a 64-bit accumulator covers
 constexpr int EXP_LIM = 400;
 constexpr float GUARD7 = 0x1p1f, GUARD8 = 0x1p-8f;  // least S_ij 2^(-E_i - F_j) for 7 / 8 digits
 template <int BN>
@@ -566,6 +569,16 @@ inline int dgemm_tc_bn(int m, int n) {
     return w64 < w80 ? 64 : 80;
 }
 
+// Slices of K that run at once (few tiles and a long K: at least one drain each, to fill the
+// SMs), and the longest K of one product, each slice within its accumulators' MAX_K columns.
+inline int dgemm_tc_ksplit(int m, int n, int nkc, bool lower) {
+    const int tiles = ceil_div(n, dgemm_tc_bn(m, n)) * ceil_div(m, tc64::BM);
+    return lower ? 1 : std::max(1, std::min({16, num_sms() / tiles, nkc / tc64::SUPER7}));
+}
+inline int dgemm_tc_max_k(int m, int n, bool lower) {
+    return tc64::MAX_K * dgemm_tc_ksplit(m, n, tc64::MAX_K, lower);
+}
+
 struct DgemmTcTiles {  // the tiles left to the FP64 unit
     const int *flags = nullptr, *nfail = nullptr;
     int bn = 0, gx = 0;
@@ -608,8 +621,8 @@ rl_status dgemm_tc(int m, int n, int k, double alpha, const double *A, long long
     if (cap != cudaStreamCaptureStatusNone) return RL_OK;
     const int sms = num_sms(), kp = ceil_div(k, BK) * BK, nkc = kp / BK;
     const int bn = dgemm_tc_bn(m, n), gx = ceil_div(n, bn), tiles = gx * ceil_div(m, BM);
-    // few tiles and a long K: slices of K (at least one drain each) fill the SMs
-    const int ks = lower ? 1 : std::max(1, std::min({16, sms / tiles, nkc / SUPER7}));
+    const int ks = dgemm_tc_ksplit(m, n, nkc, lower);
+    if (ceil_div(nkc, ks) * BK > MAX_K) return RL_ERR_INVALID_ARG;  // the caller cuts K (dgemm_tc_max_k)
     const bool same = (const void *)A == (const void *)B && lda == ldb && m == n && TA != TB;
     auto round = [](size_t v) { return (v + 255) & ~(size_t)255; };
     const size_t key_b = round(((size_t)m + n) * 4), flag_b = round(((size_t)tiles + 1) * 4);
