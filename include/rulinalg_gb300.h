@@ -99,11 +99,15 @@ RL_API uint64_t rl_launch_count(void);
                                            flag, so its wait runs out (RL_ERR_TIMEOUT): [-1, 255], default -1 */
 #define RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK 101 /* tests only: the one-launch triangular sweep never
                                                  publishes this 64-row block: [-1, 2^30], default -1 */
+#define RL_TUNE_TEST_WITHHOLD_PRODUCT_TILE 102 /* tests only: this tile of an FP64 product on the tensor cores
+                                                  never announces its accumulators: [-1, 2^30], default -1 */
 RL_API rl_status rl_tune_set(int key, int64_t value);
 RL_API rl_status rl_tune_get(int key, int64_t *value);
 
 /* ------------------------------------------------------------------------ GEMM -- */
-/* C = A * B with A m x k, B k x n, C m x n; alpha = 1, beta = 0.
+/* C = A * B with A m x k, B k x n, C m x n; alpha = 1, beta = 0. Large products wait on the
+ * tensor cores, bounded by RL_TUNE_WAIT_TIMEOUT_NS: a wait that runs out leaves NaN in its tile
+ * of C, and the host-pointer calls return RL_ERR_TIMEOUT.
  * Replaces the matrixmultiply::{sgemm,dgemm} calls of mat_mul_general!
  * (src/matrix/mat_mul.rs:33-43 and :57-67): rsa/rsb are the row strides that
  * `row_stride()` supplies there, rsc = n for a new Matrix. */

@@ -165,6 +165,7 @@ TUNE_PANEL_LOOKAHEAD = 9
 TUNE_FULLPIV_CTAS_PER_SM = 10
 TUNE_TEST_WITHHOLD_CHUNK = 100
 TUNE_TEST_WITHHOLD_SWEEP_BLOCK = 101
+TUNE_TEST_WITHHOLD_PRODUCT_TILE = 102
 
 for _name, (_res, _args) in SIGNATURES.items():
     _fn = getattr(lib, _name)

@@ -22,11 +22,9 @@ namespace {
 // slices; everything else on the SIMT kernel; both split a long K when the product has few output tiles (gemm()).
 template <class T>
 rl_status gemm_public(int m, int n, int k, const T *a, long long lda, const T *b, long long ldb, T *c, long long ldc,
-                      cudaStream_t s, bool &used_tc) {
+                      cudaStream_t s, int *err) {
     NvtxRange nvtx_("rl.gemm");
-    used_tc = false;
-    used_tc = std::is_same<T, float>::value ? sgemm_tc_eligible(m, n, k) : dgemm_tc_eligible(m, n, k);
-    return gemm<T, false, false>(m, n, k, T(1), a, lda, b, ldb, T(0), c, ldc, s);
+    return gemm<T, false, false>(m, n, k, T(1), a, lda, b, ldb, T(0), c, ldc, s, err);
 }
 
 template <class T>
@@ -43,12 +41,17 @@ rl_status gemm_host(size_t m, size_t k, size_t n, const T *a, size_t rsa, const 
     RL_TRY(dC.alloc(m * n, s));
     RL_TRY(copy_h2d(dA.p, k, a, rsa, m, k, s));
     RL_TRY(copy_h2d(dB.p, n, b, rsb, k, n, s));
-    bool used_tc = false;
-    RL_TRY(gemm_public<T>((int)m, (int)n, (int)k, dA.p, (long long)k, dB.p, (long long)n, dC.p, (long long)n, s,
-                          used_tc));
+    DevBuf<int> st;
+    const bool waits = std::is_same<T, float>::value ? sgemm_tc_eligible((int)m, (int)n, (int)k)
+                                                     : dgemm_tc_eligible((int)m, (int)n, (int)k);
+    if (waits) {
+        RL_TRY(st.alloc(1, s));
+        RL_TRY_CUDA(cudaMemsetAsync(st.p, 0, sizeof(int), s));
+    }
+    RL_TRY(gemm_public<T>((int)m, (int)n, (int)k, dA.p, (long long)k, dB.p, (long long)n, dC.p, (long long)n, s, st.p));
     RL_TRY(copy_d2h(c, rsc, dC.p, n, m, n, s));
+    if (waits) return read_status<T>(st.p, s);
     RL_TRY_CUDA(cudaStreamSynchronize(s));
-    if (used_tc) RL_TRY(sgemm_tc_status(s));
     return RL_OK;
 }
 
@@ -59,9 +62,8 @@ rl_status gemm_dev(size_t m, size_t k, size_t n, const T *a, size_t rsa, const T
     if (!c || (k && (!a || !b))) return RL_ERR_INVALID_ARG;
     if (!fits_int(m) || !fits_int(n) || !fits_int(k)) return RL_ERR_INVALID_ARG;
     RL_TRY(ensure_device());
-    bool used_tc = false;
     return gemm_public<T>((int)m, (int)n, (int)k, a, (long long)rsa, b, (long long)rsb, c, (long long)rsc,
-                          resolve_stream(stream), used_tc);
+                          resolve_stream(stream), nullptr);
 }
 
 template <class T>
@@ -246,10 +248,12 @@ rl_status qr_first_k_host(size_t m, size_t n, const T *qr, size_t lda, const T *
     RL_TRY(dQ.alloc(m * k, s));
     RL_TRY(copy_h2d(dA.p, n, qr, lda, m, n, s));
     if (p) RL_TRY_CUDA(cudaMemcpyAsync(dt.p, tau, p * sizeof(T), cudaMemcpyHostToDevice, s));
-    RL_TRY(qr_first_k_dev<T>(dA.p, (long long)n, (int)m, (int)n, dt.p, (int)k, dQ.p, (long long)k, s));
+    DevBuf<int> st;
+    RL_TRY(st.alloc(1, s));
+    RL_TRY_CUDA(cudaMemsetAsync(st.p, 0, sizeof(int), s));
+    RL_TRY(qr_first_k_dev<T>(dA.p, (long long)n, (int)m, (int)n, dt.p, (int)k, dQ.p, (long long)k, s, st.p));
     RL_TRY(copy_d2h(q, ldq, dQ.p, k, m, k, s));
-    RL_TRY_CUDA(cudaStreamSynchronize(s));
-    return RL_OK;
+    return read_status<T>(st.p, s);
 }
 
 template <class T>
@@ -268,10 +272,12 @@ rl_status qr_apply_q_host(size_t m, size_t n, const T *qr, size_t lda, const T *
     RL_TRY(copy_h2d(dA.p, n, qr, lda, m, n, s));
     if (p) RL_TRY_CUDA(cudaMemcpyAsync(dt.p, tau, p * sizeof(T), cudaMemcpyHostToDevice, s));
     RL_TRY(copy_h2d(dX.p, q, x, ldx, m, q, s));
-    RL_TRY(qr_apply_q_dev<T>(dA.p, (long long)n, (int)m, (int)n, dt.p, (int)q, dX.p, (long long)q, trans, s));
+    DevBuf<int> st;
+    RL_TRY(st.alloc(1, s));
+    RL_TRY_CUDA(cudaMemsetAsync(st.p, 0, sizeof(int), s));
+    RL_TRY(qr_apply_q_dev<T>(dA.p, (long long)n, (int)m, (int)n, dt.p, (int)q, dX.p, (long long)q, trans, s, st.p));
     RL_TRY(copy_d2h(x, ldx, dX.p, q, m, q, s));
-    RL_TRY_CUDA(cudaStreamSynchronize(s));
-    return RL_OK;
+    return read_status<T>(st.p, s);
 }
 
 // U X = B (upper = true, back_substitution) or L X = B (forward_substitution) for an

@@ -318,7 +318,7 @@ rl_status lu_factor_dev(T *A, long long lda, int n, int *ipiv, cudaStream_t s, T
                 RL_LAUNCH(trsm_diag_kernel<T>, ceil_div(n2, kTrsmCols), 128, 0, s, P, lda, kb, P + kb, lda, n2, 0,
                           (int *)nullptr, tiny);
                 RL_TRY((gemm<T, false, false>(m2, n2, kb, T(-1), P + (long long)kb * lda, lda, P + kb, lda, T(1),
-                                             P + (long long)kb * lda + kb, lda, s)));
+                                             P + (long long)kb * lda + kb, lda, s, &sync.p->err)));
             }
         }
         if (K1 < n) {
@@ -329,7 +329,7 @@ rl_status lu_factor_dev(T *A, long long lda, int n, int *ipiv, cudaStream_t s, T
             T *L11 = A + (long long)K0 * lda + K0;
             RL_TRY(tri_solve_dev<T>(L11, lda, KB, L11 + KB, lda, N2, 0, &sync.p->err, s, tiny));
             RL_TRY((gemm<T, false, false>(N2, N2, KB, T(-1), L11 + (long long)KB * lda, lda, L11 + KB, lda, T(1),
-                                         L11 + (long long)KB * lda + KB, lda, s)));
+                                         L11 + (long long)KB * lda + KB, lda, s, &sync.p->err)));
         } else if (K0 > 0) {
             RL_TRY(laswp<T>(A, lda, K0, 0, 0, ipiv, K0, K1, s));  // the last block's swaps on the left
         }
@@ -367,10 +367,10 @@ rl_status chol_factor_dev(T *A, long long lda, int n, cudaStream_t s, T tiny = E
             RL_LAUNCH(eye_kernel<T>, (int)((kk + 255) / 256), 256, 0, s, Linv.p, (long long)KB, KB, KB);
             RL_TRY(tri_solve_dev<T>(P, lda, KB, Linv.p, KB, KB, 1, st.p, s, tiny));
             T *A21 = P + (long long)KB * lda;
-            RL_TRY((gemm<T, false, true>(m2, KB, KB, T(1), A21, lda, Linv.p, KB, T(0), T21.p, KB, s)));
+            RL_TRY((gemm<T, false, true>(m2, KB, KB, T(1), A21, lda, Linv.p, KB, T(0), T21.p, KB, s, st.p)));
             RL_TRY_CUDA(cudaMemcpy2DAsync(A21, lda * sizeof(T), T21.p, KB * sizeof(T), KB * sizeof(T), m2,
                                           cudaMemcpyDeviceToDevice, s));
-            RL_TRY((gemm<T, false, true, true>(m2, m2, KB, T(-1), A21, lda, A21, lda, T(1), A21 + KB, lda, s)));
+            RL_TRY((gemm<T, false, true, true>(m2, m2, KB, T(-1), A21, lda, A21, lda, T(1), A21 + KB, lda, s, st.p)));
         }
         return read_status<T>(st.p, s);
     }
@@ -389,7 +389,7 @@ rl_status chol_factor_dev(T *A, long long lda, int n, cudaStream_t s, T tiny = E
             RL_LAUNCH(trsm_right_lt_kernel<T>, ceil_div(m2, kTrsmCols), 128, 0, s, P, lda, kb, P + (long long)kb * lda, lda,
                       m2);
             T *L21 = P + (long long)kb * lda;
-            RL_TRY((gemm<T, false, true, true>(m2, m2, kb, T(-1), L21, lda, L21, lda, T(1), L21 + kb, lda, s)));
+            RL_TRY((gemm<T, false, true, true>(m2, m2, kb, T(-1), L21, lda, L21, lda, T(1), L21 + kb, lda, s, st.p)));
         }
     }
     return read_status<T>(st.p, s);
@@ -412,12 +412,13 @@ rl_status block_t_factor(const T *V, int mrows, int kb, const T *tau, T *part, i
 // unit-triangular rows of V apart, whose few entries would send the first row of tiles of the
 // tensor-core product to the FP64 unit (its accuracy check is per tile, gemm_f64tc.cuh).
 template <class T>
-rl_status block_update(const T *V, int mrows, int kb, const T *W, T *X, long long ldx, int q, cudaStream_t s) {
+rl_status block_update(const T *V, int mrows, int kb, const T *W, T *X, long long ldx, int q, cudaStream_t s,
+                       int *err) {
     const int head = sizeof(T) == 8 && mrows > kb ? kb : 0;
     if (head)
-        RL_TRY((gemm<T, false, false>(head, q, kb, T(-1), V, kb, W, q, T(1), X, ldx, s)));
+        RL_TRY((gemm<T, false, false>(head, q, kb, T(-1), V, kb, W, q, T(1), X, ldx, s, err)));
     return gemm<T, false, false>(mrows - head, q, kb, T(-1), V + (long long)head * kb, kb, W, q, T(1), X + (long long)head * ldx,
-                                 ldx, s);
+                                 ldx, s, err);
 }
 
 // Blocked Householder QR with compact-WY trailing updates; nrefl reflectors
@@ -466,9 +467,9 @@ rl_status qr_factor_dev(T *A, long long lda, int m, int n, int nrefl, T *tau, cu
         RL_LAUNCH(extract_v_kernel<T>, (int)((mk + 255) / 256), 256, 0, s, P, lda, mrows, kb, V.p);
         RL_TRY(block_t_factor<T>(V.p, mrows, kb, tk, Gp.p, max_parts, Tm.p, s));
         T *A2 = P + kb;
-        RL_TRY((gemm<T, true, false>(kb, n2, mrows, T(1), V.p, kb, A2, lda, T(0), W1.p, n2, s)));
-        RL_TRY((gemm<T, true, false>(kb, n2, kb, T(1), Tm.p, kb, W1.p, n2, T(0), W2.p, n2, s)));
-        RL_TRY(block_update<T>(V.p, mrows, kb, W2.p, A2, lda, n2, s));
+        RL_TRY((gemm<T, true, false>(kb, n2, mrows, T(1), V.p, kb, A2, lda, T(0), W1.p, n2, s, &sync.p->err)));
+        RL_TRY((gemm<T, true, false>(kb, n2, kb, T(1), Tm.p, kb, W1.p, n2, T(0), W2.p, n2, s, &sync.p->err)));
+        RL_TRY(block_update<T>(V.p, mrows, kb, W2.p, A2, lda, n2, s, &sync.p->err));
     }
     int err = 0;
     RL_TRY_CUDA(cudaMemcpyAsync(&err, &sync.p->err, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -480,10 +481,10 @@ rl_status qr_factor_dev(T *A, long long lda, int m, int n, int nrefl, T *tau, cu
 // applied in reverse order to I[:, 0:k], each as Q2 -= V (T (V^T Q2)). The rows and columns of
 // a panel's own reflectors are still those of the identity, Q2 = [I 0; 0 Q3] (Q3 an identity
 // too for the first panel applied), so V^T Q2 = [V1^T, V2^T Q3] takes a product for the
-// columns of Q3 only.
+// columns of Q3 only. *err: a status word for the products' waits (gemm()), read by the caller.
 template <class T>
 rl_status qr_first_k_dev(const T *QR, long long lda, int m, int n, const T *tau, int k, T *Q, long long ldq,
-                         cudaStream_t s) {
+                         cudaStream_t s, int *err) {
     if (m <= 0 || k <= 0) return RL_OK;
     constexpr int NB = PanelNB<T>::value;
     const long long mk = (long long)m * k;
@@ -508,9 +509,9 @@ rl_status qr_first_k_dev(const T *QR, long long lda, int m, int n, const T *tau,
         RL_LAUNCH(v_transpose_kernel<T>, ceil_div((long long)kb * copied, 256), 256, 0, s, V.p, kb, copied, W1.p, (long long)nc);
         if (copied < nc)
             RL_TRY((gemm<T, true, false>(kb, nc - kb, mrows - kb, T(1), V.p + (long long)kb * kb, kb,
-                                         Q2 + (long long)kb * ldq + kb, ldq, T(0), W1.p + kb, nc, s)));
-        RL_TRY((gemm<T, false, false>(kb, nc, kb, T(1), Tm.p, kb, W1.p, nc, T(0), W2.p, nc, s)));
-        RL_TRY(block_update<T>(V.p, mrows, kb, W2.p, Q2, ldq, nc, s));
+                                         Q2 + (long long)kb * ldq + kb, ldq, T(0), W1.p + kb, nc, s, err)));
+        RL_TRY((gemm<T, false, false>(kb, nc, kb, T(1), Tm.p, kb, W1.p, nc, T(0), W2.p, nc, s, err)));
+        RL_TRY(block_update<T>(V.p, mrows, kb, W2.p, Q2, ldq, nc, s, err));
     }
     return RL_OK;
 }
@@ -520,10 +521,10 @@ rl_status qr_first_k_dev(const T *QR, long long lda, int m, int n, const T *tau,
 // HouseholderComposition::left_multiply_into (householder.rs:203-227) applies the
 // reflectors from the last to the first, Q^T takes them from the first to the last.
 // Per 64-reflector panel (compact WY, Q_i = I - V T V^T): X[k0:, :] -= V (op(T) (V^T X[k0:, :]))
-// with op(T) = T for Q, T^T for Q^T.
+// with op(T) = T for Q, T^T for Q^T. *err as in qr_first_k_dev.
 template <class T>
 rl_status qr_apply_q_dev(const T *QR, long long lda, int m, int n, const T *tau, int q, T *X, long long ldx, bool trans,
-                         cudaStream_t s) {
+                         cudaStream_t s, int *err) {
     const int p = std::min(m, n);
     if (m <= 0 || q <= 0 || p <= 0) return RL_OK;
     constexpr int NB = PanelNB<T>::value;
@@ -543,12 +544,12 @@ rl_status qr_apply_q_dev(const T *QR, long long lda, int m, int n, const T *tau,
         RL_LAUNCH(extract_v_kernel<T>, (int)((mkb + 255) / 256), 256, 0, s, P, lda, mrows, kb, V.p);
         RL_TRY(block_t_factor<T>(V.p, mrows, kb, tau + k0, Gp.p, max_parts, Tm.p, s));
         T *X2 = X + (long long)k0 * ldx;
-        RL_TRY((gemm<T, true, false>(kb, q, mrows, T(1), V.p, kb, X2, ldx, T(0), W1.p, q, s)));
+        RL_TRY((gemm<T, true, false>(kb, q, mrows, T(1), V.p, kb, X2, ldx, T(0), W1.p, q, s, err)));
         if (trans)
-            RL_TRY((gemm<T, true, false>(kb, q, kb, T(1), Tm.p, kb, W1.p, q, T(0), W2.p, q, s)));
+            RL_TRY((gemm<T, true, false>(kb, q, kb, T(1), Tm.p, kb, W1.p, q, T(0), W2.p, q, s, err)));
         else
-            RL_TRY((gemm<T, false, false>(kb, q, kb, T(1), Tm.p, kb, W1.p, q, T(0), W2.p, q, s)));
-        RL_TRY(block_update<T>(V.p, mrows, kb, W2.p, X2, ldx, q, s));
+            RL_TRY((gemm<T, false, false>(kb, q, kb, T(1), Tm.p, kb, W1.p, q, T(0), W2.p, q, s, err)));
+        RL_TRY(block_update<T>(V.p, mrows, kb, W2.p, X2, ldx, q, s, err));
     }
     return RL_OK;
 }
@@ -666,7 +667,7 @@ rl_status tri_solve_dev(const TA *A, long long lda, int n, T *Y, long long ldy, 
                 const int rest = n - b0 - bs;
                 if (rest > 0)
                     RL_TRY((gemm<T, false, false>(rest, nrhs, bs, T(-1), A + (long long)(b0 + bs) * lda + b0, lda, Yb, ldy,
-                                                  T(1), Yb + (long long)bs * ldy, ldy, s)));
+                                                  T(1), Yb + (long long)bs * ldy, ldy, s, dstatus)));
             }
         } else {
             for (int b1 = n; b1 > 0; b1 -= NB) {
@@ -676,10 +677,10 @@ rl_status tri_solve_dev(const TA *A, long long lda, int n, T *Y, long long ldy, 
                 RL_LAUNCH(trsm_diag_kernel<T>, gr, 128, 0, s, D, lda, bs, Yb, ldy, nrhs, mode, dstatus, tiny);
                 if (b0 > 0) {
                     if (mode == 2)
-                        RL_TRY((gemm<T, false, false>(b0, nrhs, bs, T(-1), A + b0, lda, Yb, ldy, T(1), Y, ldy, s)));
+                        RL_TRY((gemm<T, false, false>(b0, nrhs, bs, T(-1), A + b0, lda, Yb, ldy, T(1), Y, ldy, s, dstatus)));
                     else
                         RL_TRY((gemm<T, true, false>(b0, nrhs, bs, T(-1), A + (long long)b0 * lda, lda, Yb, ldy, T(1), Y,
-                                                     ldy, s)));
+                                                     ldy, s, dstatus)));
                 }
             }
         }

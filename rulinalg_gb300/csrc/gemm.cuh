@@ -284,10 +284,12 @@ static __global__ void __launch_bounds__(128)
 // a 128 x 128 tile's worth of C and K >= 256 go to the tcgen05 kernel (gemm_tc.cuh).
 // A product with fewer tiles than SMs and a long K (the V^T A2 and V^T V products of a
 // Householder block, K = the panel height) is split along K into partial tiles that
-// run at once, then added in slice order.
+// run at once, then added in slice order. The tensor-core forms wait (bounded): *err, a device
+// status word of the caller's (0 or its first error; null: none is kept), receives
+// RL_ERR_TIMEOUT when a wait runs out, and the tile of C NaN.
 template <class T, bool TA, bool TB, bool LOWER = false>
 rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T *B, long long ldb, T beta, T *C,
-               long long ldc, cudaStream_t stream) {
+               long long ldc, cudaStream_t stream, int *err) {
     if (m <= 0 || n <= 0) return RL_OK;
     constexpr int BM = GemmCfg<T>::BM, BN = GemmCfg<T>::BN, BK = GemmCfg<T>::BK;
     constexpr int NT = (BM / GemmCfg<T>::TM) * (BN / GemmCfg<T>::TN);
@@ -298,7 +300,7 @@ rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T 
             const int tc_tiles = ceil_div(n, tc::BN) * ceil_div(m, tc::BM);
             int ks = 1;
             if (!LOWER && tc_tiles < sms / 2 && k >= 1024) ks = std::min({16, ceil_div(sms, tc_tiles), k / 256});
-            return sgemm_tc<TA, TB>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, LOWER, stream, ks);
+            return sgemm_tc<TA, TB>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, LOWER, stream, err, ks);
         }
     }
     if constexpr (!LOWER) {
@@ -321,11 +323,11 @@ rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T 
             const int part = ceil_div(ceil_div(k, ceil_div(k, max_k)), tc64::BK) * tc64::BK;
             for (int p = 0; p < k; p += part)
                 RL_TRY((gemm<T, TA, TB, LOWER>(m, n, std::min(part, k - p), alpha, A + (TA ? p * lda : (long long)p), lda,
-                                               B + (TB ? (long long)p : p * ldb), ldb, p ? T(1) : beta, C, ldc, stream)));
+                                               B + (TB ? (long long)p : p * ldb), ldb, p ? T(1) : beta, C, ldc, stream, err)));
             return RL_OK;
         }
         if (dgemm_tc_eligible(m, n, k))
-            RL_TRY((dgemm_tc<TA, TB>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, LOWER, stream, ws, left, taken)));
+            RL_TRY((dgemm_tc<TA, TB>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, LOWER, stream, err, ws, left, taken)));
         // what follows computes the tiles that were left (usually none), or all of C
     }
     int ksplit = 1;

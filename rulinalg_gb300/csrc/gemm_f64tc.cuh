@@ -37,7 +37,7 @@
 // chunks of 32 through two stages of shared memory, each holding the slice tiles of both
 // operands (64-byte swizzle). A producer lane, an MMA lane (56 or 72 MMAs per chunk, all
 // from one load of the 14 or 16 tiles) and 8 warps that drain the accumulators. Every
-// wait is bounded (RL_ERR_TIMEOUT, NaN over the tile).
+// wait is bounded (RL_ERR_TIMEOUT in the caller's status word, NaN over the tile).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -267,7 +267,7 @@ template <int BN>
 static __global__ void __launch_bounds__(tc64::THREADS, 1)
     dgemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int m, int n, int nkc, const unsigned *__restrict__ keyA, const unsigned *__restrict__ keyB, double alpha,
                     double beta, double *C, long long ldc, int lower, int *flags, int *nfail, int kc_per,
-                    long long zstride, int *err, unsigned long long wait_ns) {
+                    long long zstride, int *err, unsigned long long wait_ns, int withhold) {
     using namespace tc64;
     using tc::mbar_expect_tx;
     using tc::mbar_wait;
@@ -284,7 +284,8 @@ static __global__ void __launch_bounds__(tc64::THREADS, 1)
     uint64_t *empty = full + STAGES;
     uint64_t *tfull = empty + STAGES;
     uint64_t *tempty = tfull + 1;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tempty + 1);
+    uint64_t *drained = tempty + 1;  // after a wait that ran out: every MMA issued has completed
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drained + 1);
     __shared__ int s_fail;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int c_begin = blockIdx.z * kc_per;
@@ -305,6 +306,7 @@ static __global__ void __launch_bounds__(tc64::THREADS, 1)
         }
         tc::mbar_init(tfull, 1);
         tc::mbar_init(tempty, DRAIN_WARPS);
+        tc::mbar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -348,7 +350,8 @@ static __global__ void __launch_bounds__(tc64::THREADS, 1)
                              (use > 0 || u > 0 || ks > 0) ? 1u : 0u);
             mma_commit(&empty[s]);
         }
-        mma_commit(tfull);
+        // withhold: a test setting, this tile's first accumulators are never announced
+        if ((int)(blockIdx.y * gridDim.x + blockIdx.x) != withhold) mma_commit(tfull);
     }
     __syncwarp();
     bool ok = true, seven = true;
@@ -498,7 +501,12 @@ static __global__ void __launch_bounds__(tc64::THREADS, 1)
     }
     __syncthreads();
     const bool dead = s_fail != 0;
-    if (dead && warp == DRAIN_WARPS && lane == 0)  // no copy may land after the CTA has left
+    // no copy may land and no MMA may run after the CTA has given up its memory
+    if (dead && warp == DRAIN_WARPS + 1 && lane == 0) {
+        mma_commit(drained);
+        mbar_wait(drained, 0, wait_ns);
+    }
+    if (dead && warp == DRAIN_WARPS && lane == 0)
         for (int c = max(0, issued - STAGES); c < issued; c++) mbar_wait(&full[c % STAGES], (c / STAGES) & 1, wait_ns);
     if (take || dead) {
         for (int e = tid; e < BM * BN; e += THREADS) {
@@ -511,7 +519,7 @@ static __global__ void __launch_bounds__(tc64::THREADS, 1)
             }
         }
     }
-    if (dead && tid == 0) atomicCAS(err, 0, RL_ERR_TIMEOUT);
+    if (dead && tid == 0 && err) atomicCAS(err, 0, RL_ERR_TIMEOUT);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == DRAIN_WARPS)
@@ -591,27 +599,26 @@ struct DgemmTcTiles {  // the tiles left to the FP64 unit
 template <int BN>
 static rl_status dgemm_tc_launch(int m, int n, int nkc, const CUtensorMap &mA, const __nv_bfloat16 *Sb, int kp,
                           const unsigned *keyA, const unsigned *keyB, double alpha, double beta, double *C, long long ldc,
-                          bool lower, int *flags, double *part, int ks, cudaStream_t s) {
+                          bool lower, int *flags, double *part, int ks, cudaStream_t s, int *err) {
     using namespace tc64;
     static const cudaError_t attr =
         cudaFuncSetAttribute(dgemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::SMEM);
     RL_TRY_CUDA(attr);
     CUtensorMap mB;
     RL_TRY(make_slice_map(mB, Sb, n, kp, BN));
-    int *err = nullptr;
-    RL_TRY_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&err), g_sgemm_tc_err));
     dim3 grid(ceil_div(n, BN), ceil_div(m, BM), ks);
     const bool split = ks > 1;
     RL_LAUNCH(dgemm_tc_kernel<BN>, grid, THREADS, Cfg<BN>::SMEM, s, mA, mB, m, n, nkc, keyA, keyB, split ? 1.0 : alpha,
               split ? 0.0 : beta, split ? part : C, split ? (long long)n : ldc, lower ? 1 : 0, flags + 1, flags,
-              ceil_div(nkc, ks), split ? (long long)m * n : 0ll, err, wait_ns());
+              ceil_div(nkc, ks), split ? (long long)m * n : 0ll, err, wait_ns(),
+              (int)tune(RL_TUNE_TEST_WITHHOLD_PRODUCT_TILE));
     return RL_OK;
 }
 
 template <bool TA, bool TB>
 rl_status dgemm_tc(int m, int n, int k, double alpha, const double *A, long long lda, const double *B, long long ldb, double beta,
-                   double *C, long long ldc, bool lower, cudaStream_t s, DevBuf<unsigned char> &ws, DgemmTcTiles &left,
-                   bool &taken) {
+                   double *C, long long ldc, bool lower, cudaStream_t s, int *err, DevBuf<unsigned char> &ws,
+                   DgemmTcTiles &left, bool &taken) {
     using namespace tc64;
     taken = false;
     const double aa = alpha < 0 ? -alpha : alpha;
@@ -651,8 +658,10 @@ rl_status dgemm_tc(int m, int n, int k, double alpha, const double *A, long long
     RL_LAUNCH(f64_slice_kernel, a.blocks + b.blocks, 256, 0, s, a, b, k, kp);
     CUtensorMap mA;
     RL_TRY(make_slice_map(mA, Sa, m, kp, BM));
-    RL_TRY(bn == 64 ? dgemm_tc_launch<64>(m, n, nkc, mA, Sb, kp, a.key, b.key, alpha, beta, C, ldc, lower, flags, part, ks, s)
-                    : dgemm_tc_launch<80>(m, n, nkc, mA, Sb, kp, a.key, b.key, alpha, beta, C, ldc, lower, flags, part, ks, s));
+    RL_TRY(bn == 64 ? dgemm_tc_launch<64>(m, n, nkc, mA, Sb, kp, a.key, b.key, alpha, beta, C, ldc, lower, flags, part, ks, s,
+                                               err)
+                    : dgemm_tc_launch<80>(m, n, nkc, mA, Sb, kp, a.key, b.key, alpha, beta, C, ldc, lower, flags, part, ks, s,
+                                               err));
     if (ks > 1)
         RL_LAUNCH(dgemm_tc_reduce_kernel, (int)std::min<long long>(4LL * sms, ((long long)m * n + 255) / 256), 256, 0, s, m, n, ks,
                   alpha, part, beta, C, ldc, flags + 1, flags, bn, gx, 0);

@@ -342,15 +342,12 @@ static __global__ void __launch_bounds__(tc::THREADS, 1)
             }
         }
     }
-    if (!ok && tid == 0) atomicCAS(err, 0, RL_ERR_TIMEOUT);
+    if (!ok && tid == 0 && err) atomicCAS(err, 0, RL_ERR_TIMEOUT);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
 }
-
-// Sticky timeout word of the tensor-core GEMM (one per translation unit that launches it).
-static __device__ int g_sgemm_tc_err;
 
 // Shapes worth the tensor cores: at least half a 128 x 128 tile of C in each direction
 // and K >= 256. Below that K the per-call split, tensor-map set-up and a pipeline that
@@ -410,10 +407,11 @@ __global__ void splitk_reduce_kernel(int m, int n, int nz, T alpha, const T *__r
 // alignment. op(A) = A (m x k, A[i * lda + p]) or A^T (A[p * lda + i]); op(B) = B (k x n,
 // B[p * ldb + j]) or B^T (B[j * ldb + p]). The split kernels repack both operands K-major.
 // ksplit > 1 (not with `lower`) runs K in that many slices at once into partial tiles,
-// added in slice order afterwards: for products with few output tiles and a long K.
+// added in slice order afterwards: for products with few output tiles and a long K. A wait
+// that runs out leaves NaN in its tile and RL_ERR_TIMEOUT in *err (may be null).
 template <bool TA, bool TB>
 static rl_status sgemm_tc(int m, int n, int k, float alpha, const float *A, long long lda, const float *B, long long ldb,
-                   float beta, float *C, long long ldc, bool lower, cudaStream_t s, int ksplit = 1) {
+                   float beta, float *C, long long ldc, bool lower, cudaStream_t s, int *err, int ksplit = 1) {
     static const cudaError_t attr =
         cudaFuncSetAttribute(sgemm_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
     RL_TRY_CUDA(attr);
@@ -435,8 +433,6 @@ static rl_status sgemm_tc(int m, int n, int k, float alpha, const float *A, long
     RL_TRY(make_tile_map(mAl, Al, m, kp));
     RL_TRY(make_tile_map(mBh, Bh, n, kp));
     RL_TRY(make_tile_map(mBl, Bl, n, kp));
-    int *err = nullptr;
-    RL_TRY_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&err), g_sgemm_tc_err));
     dim3 grid((n + tc::BN - 1) / tc::BN, (m + tc::BM - 1) / tc::BM);
     const int nkc = kp / tc::BK;
     if (ksplit > 1 && !lower) {
@@ -454,17 +450,6 @@ static rl_status sgemm_tc(int m, int n, int k, float alpha, const float *A, long
     RL_LAUNCH(sgemm_tma_kernel, grid, tc::THREADS, tc::SMEM_BYTES, s, mAh, mAl, mBh, mBl, m, n, kp, alpha, beta, C,
               ldc, lower ? 1 : 0, err, nkc, 0ll, wait_ns());
     return RL_OK;
-}
-
-// Reads and clears the sticky timeout word (synchronises the stream).
-static inline rl_status sgemm_tc_status(cudaStream_t s) {
-    int *err = nullptr;
-    RL_TRY_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&err), g_sgemm_tc_err));
-    int h = 0;
-    RL_TRY_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    RL_TRY_CUDA(cudaStreamSynchronize(s));
-    if (h) RL_TRY_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
-    return h ? RL_ERR_TIMEOUT : RL_OK;
 }
 
 }  // namespace rl

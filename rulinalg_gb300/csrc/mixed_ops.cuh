@@ -31,9 +31,9 @@ inline double bits_to_double(unsigned long long b) {
     return d;
 }
 
-// R = B - A X (B == nullptr: R = A X), FP64.
+// R = B - A X (B == nullptr: R = A X), FP64. *err: see gemm().
 inline rl_status residual_dev(const double *A, long long lda, int n, const double *X, long long ldx, const double *B,
-                       long long ldb, double *R, long long ldr, int nrhs, cudaStream_t s) {
+                       long long ldb, double *R, long long ldr, int nrhs, cudaStream_t s, int *err) {
     if (nrhs <= 4) {
         // instantiated for the exact count: the FP64 pipe spends its ~64 cycles on a warp
         // DFMA whose predicate is off as well, so a 4-column instance on one column costs 4x
@@ -49,7 +49,7 @@ inline rl_status residual_dev(const double *A, long long lda, int n, const doubl
     if (B)
         RL_TRY_CUDA(cudaMemcpy2DAsync(R, ldr * sizeof(double), B, ldb * sizeof(double), nrhs * sizeof(double), n,
                                       cudaMemcpyDeviceToDevice, s));
-    return gemm<double, false, false>(n, nrhs, n, B ? -1.0 : 1.0, A, lda, X, ldx, B ? 1.0 : 0.0, R, ldr, s);
+    return gemm<double, false, false>(n, nrhs, n, B ? -1.0 : 1.0, A, lda, X, ldx, B ? 1.0 : 0.0, R, ldr, s, err);
 }
 
 inline rl_status colnorm_dev(const double *V, long long ldv, int n, int nrhs, unsigned long long *out, cudaStream_t s) {
@@ -189,7 +189,7 @@ inline rl_status gmres_ir(const double *A, long long lda, int n, const Minv &M, 
     ok = false;
     double prev_rn = INFINITY;
     for (int outer = 0; outer < outer_max; outer++) {
-        RL_TRY(residual_dev(A, lda, n, x, 1, b, 1, r.p, 1, 1, s));
+        RL_TRY(residual_dev(A, lda, n, x, 1, b, 1, r.p, 1, 1, s, M.dstatus));
         RL_TRY(colnorm_dev(r.p, 1, n, 1, bits.p, s));
         RL_TRY(colnorm_dev(x, 1, n, 1, bits.p + 1, s));
         unsigned long long hb[2];
@@ -221,7 +221,7 @@ inline rl_status gmres_ir(const double *A, long long lda, int n, const Minv &M, 
         for (int k = 0; k < m; k++) {
             double *vk = V.p + (size_t)k * n;
             double *hk = H.p + (size_t)k * (m + 1);
-            RL_TRY(residual_dev(A, lda, n, vk, 1, nullptr, 0, r.p, 1, 1, s));  // r = A v_k
+            RL_TRY(residual_dev(A, lda, n, vk, 1, nullptr, 0, r.p, 1, 1, s, M.dstatus));  // r = A v_k
             RL_TRY(M.apply(r.p, w.p, s));                                    // w = M^-1 A v_k
             // CGS2: h = V^T w, w -= V h, twice
             RL_TRY(dots.run(V.p, n, k + 1, w.p, n, hk, 0, s));
@@ -298,16 +298,19 @@ inline rl_status backward_error_dev(const double *A, long long lda, int n, const
     DevBuf<double> R;
     DevBuf<unsigned long long> bits;
     RL_TRY(R.alloc((size_t)n * nrhs, s));
-    RL_TRY(bits.alloc(3 * nrhs + 1, s));
-    RL_TRY(residual_dev(A, lda, n, X, ldx, B, ldb, R.p, nrhs, nrhs, s));
+    RL_TRY(bits.alloc(3 * nrhs + 2, s));  // the columns' norms, ||A||, a status word
+    RL_TRY_CUDA(cudaMemsetAsync(bits.p + 3 * nrhs, 0, 2 * sizeof(unsigned long long), s));
+    RL_TRY(residual_dev(A, lda, n, X, ldx, B, ldb, R.p, nrhs, nrhs, s, reinterpret_cast<int *>(bits.p + 3 * nrhs + 1)));
     RL_TRY(colnorm_dev(R.p, nrhs, n, nrhs, bits.p, s));
     RL_TRY(colnorm_dev(X, ldx, n, nrhs, bits.p + nrhs, s));
     RL_TRY(colnorm_dev(B, ldb, n, nrhs, bits.p + 2 * nrhs, s));
-    RL_TRY_CUDA(cudaMemsetAsync(bits.p + 3 * nrhs, 0, sizeof(unsigned long long), s));
     RL_LAUNCH(rownorm_kernel, grid_rows(n, 8), 256, 0, s, A, lda, n, bits.p + 3 * nrhs);
-    std::vector<unsigned long long> hb(3 * nrhs + 1);
+    std::vector<unsigned long long> hb(3 * nrhs + 2);
     RL_TRY_CUDA(cudaMemcpyAsync(hb.data(), bits.p, hb.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     RL_TRY_CUDA(cudaStreamSynchronize(s));
+    int st = 0;
+    memcpy(&st, &hb[3 * nrhs + 1], sizeof st);
+    if (st) return st;
     const double anorm = bits_to_double(hb[3 * nrhs]);
     berr = 0.0;
     for (int c = 0; c < nrhs; c++) {
@@ -496,14 +499,14 @@ struct MixedFactor {
         bool stalled = false, need_fp64 = false, diverged = false;
         const int max_steps = (int)tune(RL_TUNE_MIXED_REFINE_STEPS);
         for (int it = 0;; it++) {
-            RL_TRY(residual_dev(A, lda, n, X, ldx, B, ldb, R.p, nrhs, nrhs, s));
+            RL_TRY(residual_dev(A, lda, n, X, ldx, B, ldb, R.p, nrhs, nrhs, s, dstatus));
             RL_TRY_CUDA(cudaMemsetAsync(rn_b, 0, 2 * nrhs * sizeof(unsigned long long), s));
             RL_LAUNCH(colnorm2_kernel, ge, 256, 0, s, R.p, (long long)nrhs, X, ldx, n, nrhs, rn_b);
             RL_TRY_CUDA(cudaMemcpyAsync(hb.data(), nb.p, hb.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
             RL_TRY_CUDA(cudaStreamSynchronize(s));
             int dst = 0;
             memcpy(&dst, &hb[3 * nrhs], sizeof dst);
-            if (dst != 0) {  // the FP32 factor met a pivot below FLT_MIN in a solve
+            if (dst != 0) {  // the FP32 factor met a pivot below FLT_MIN in a solve, or a wait ran out
                 need_fp64 = true;
                 break;
             }

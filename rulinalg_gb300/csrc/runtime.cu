@@ -84,6 +84,7 @@ TuneKey g_tune_keys[] = {
     {RL_TUNE_FULLPIV_CTAS_PER_SM, 1, 3, 3},
     {RL_TUNE_TEST_WITHHOLD_CHUNK, -1, 255, -1},
     {RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK, -1, 1LL << 30, -1},
+    {RL_TUNE_TEST_WITHHOLD_PRODUCT_TILE, -1, 1LL << 30, -1},
 };
 constexpr int kTuneCount = sizeof(g_tune_keys) / sizeof(g_tune_keys[0]);
 std::atomic<int64_t> g_tune_values[kTuneCount];

@@ -104,7 +104,7 @@ static __global__ void __launch_bounds__(256) small_lu_kernel(T *A, int lda, int
             if (tid == j) my_piv = wi;
             __syncthreads();
             if (S.bad) {
-                if (tid == 0) *status = RL_ERR_DIV_BY_ZERO;
+                if (tid == 0) atomicCAS(status, 0, RL_ERR_DIV_BY_ZERO);
                 return;
             }
             const T p = S.piv, inv = S.inv;
@@ -205,7 +205,7 @@ static __global__ void __launch_bounds__(256) small_chol_kernel(T *A, int lda, i
             }
             __syncthreads();
             if (S.bad) {
-                if (tid == 0) *status = RL_ERR_DECOMP_FAILURE;
+                if (tid == 0) atomicCAS(status, 0, RL_ERR_DECOMP_FAILURE);
                 return;
             }
             const T s = S.s, inv = S.inv, own = S.col[slot][r];
