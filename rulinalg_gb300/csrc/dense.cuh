@@ -2017,12 +2017,14 @@ static __global__ void __launch_bounds__(64) diag_inverse_kernel(const TA *__res
 // Row-wise solve X D^T = Y for the rows of Y (m x bs, stride ldy), D lower bs x bs: the
 // Cholesky panel L21 = A21 L11^-T. As trsm_diag_kernel: CTA per 8 rows, 16 lanes per row each
 // holding 4 of its entries, so that the FP64 work is on every SM (a thread per row put the
-// 64-step chain of 2,016 multiply-adds on 11 SMs at m = 1,400: 129 us).
+// 64-step chain of 2,016 multiply-adds on 11 SMs at m = 1,400: 129 us). With *status set (D's
+// factorisation, or an earlier one, has failed) nothing is done.
 template <class T>
 static __global__ void __launch_bounds__(128) trsm_right_lt_kernel(const T *D, long long ldd, int bs, T *Y, long long ldy,
-                                                            int m) {
+                                                            int m, const int *status) {
     __shared__ T Ds[64][65];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int failed = *status;  // read with D in flight
     {
         T d[32];
 #pragma unroll
@@ -2030,6 +2032,7 @@ static __global__ void __launch_bounds__(128) trsm_right_lt_kernel(const T *D, l
             const int i = 2 * e + (tid >> 6), j = tid & 63;
             d[e] = (i < bs && j < bs) ? D[(long long)i * ldd + j] : T(0);
         }
+        if (failed) return;
 #pragma unroll
         for (int e = 0; e < 32; e++) Ds[2 * e + (tid >> 6)][tid & 63] = d[e];
     }

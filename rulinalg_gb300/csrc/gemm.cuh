@@ -156,7 +156,11 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
 
     const int ktiles = (k + BK - 1) / BK;
     if (ktiles > 0) {
-        load_tile(0);
+        int stopped = 0;  // read with the first tile in flight
+    if constexpr (LOWER && FLAGS)
+        if (only.stop) stopped = *only.stop;
+    load_tile(0);
+    if (stopped) return;
         store_tile(0);
     }
     __syncthreads();
@@ -286,7 +290,8 @@ static __global__ void __launch_bounds__(128)
 // Householder block, K = the panel height) is split along K into partial tiles that
 // run at once, then added in slice order. The tensor-core forms wait (bounded): *err, a device
 // status word of the caller's (0 or its first error; null: none is kept), receives
-// RL_ERR_TIMEOUT when a wait runs out, and the tile of C NaN.
+// RL_ERR_TIMEOUT when a wait runs out, and the tile of C NaN. The FP64 SYRK form (LOWER) leaves C
+// as it is when *err is set already: a Cholesky that has failed does not run on.
 template <class T, bool TA, bool TB, bool LOWER = false>
 rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T *B, long long ldb, T beta, T *C,
                long long ldc, cudaStream_t stream, int *err) {
@@ -316,6 +321,7 @@ rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T 
     }
     DevBuf<unsigned char> ws;
     DgemmTcTiles left;
+    if (LOWER) left.stop = err;
     if constexpr (std::is_same<T, double>::value) {  // FP64 with enough work: exact slices on the tensor cores
         bool taken = false;
         const int max_k = dgemm_tc_eligible(m, n, k) ? dgemm_tc_max_k(m, n, LOWER) : k;

@@ -267,7 +267,7 @@ template <int BN>
 static __global__ void __launch_bounds__(tc64::THREADS, 1)
     dgemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int m, int n, int nkc, const unsigned *__restrict__ keyA, const unsigned *__restrict__ keyB, double alpha,
                     double beta, double *C, long long ldc, int lower, int *flags, int *nfail, int kc_per,
-                    long long zstride, int *err, unsigned long long wait_ns, int withhold) {
+                    long long zstride, int *err, const int *stop, unsigned long long wait_ns, int withhold) {
     using namespace tc64;
     using tc::mbar_expect_tx;
     using tc::mbar_wait;
@@ -286,8 +286,9 @@ static __global__ void __launch_bounds__(tc64::THREADS, 1)
     uint64_t *tempty = tfull + 1;
     uint64_t *drained = tempty + 1;  // after a wait that ran out: every MMA issued has completed
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drained + 1);
-    __shared__ int s_fail;
+    __shared__ int s_fail, s_stop;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 32) s_stop = stop ? *stop : 0;  // read while the tensor memory is allocated
     const int c_begin = blockIdx.z * kc_per;
     const int nk = max(0, min(nkc, c_begin + kc_per) - c_begin);
     C += blockIdx.z * zstride;
@@ -314,6 +315,11 @@ static __global__ void __launch_bounds__(tc64::THREADS, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
     constexpr uint32_t idesc = idesc_bf16(BM, BN);
+    if (s_stop) {  // the factorisation this product belongs to has failed
+        if (warp == DRAIN_WARPS)
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+        return;
+    }
 
     // Phase 1: the magnitudes' product over the whole K, a stage holding up to 8 chunks of
     // the one slice.
@@ -590,6 +596,7 @@ inline int dgemm_tc_max_k(int m, int n, bool lower) {
 struct DgemmTcTiles {  // the tiles left to the FP64 unit
     const int *flags = nullptr, *nfail = nullptr;
     int bn = 0, gx = 0;
+    const int *stop = nullptr;  // a status word: if set, nothing is left to do (the SYRK form)
 };
 
 // C = alpha op(A) op(B) + beta C. `taken` = false: nothing was done (no memory for the
@@ -610,7 +617,7 @@ static rl_status dgemm_tc_launch(int m, int n, int nkc, const CUtensorMap &mA, c
     const bool split = ks > 1;
     RL_LAUNCH(dgemm_tc_kernel<BN>, grid, THREADS, Cfg<BN>::SMEM, s, mA, mB, m, n, nkc, keyA, keyB, split ? 1.0 : alpha,
               split ? 0.0 : beta, split ? part : C, split ? (long long)n : ldc, lower ? 1 : 0, flags + 1, flags,
-              ceil_div(nkc, ks), split ? (long long)m * n : 0ll, err, wait_ns(),
+              ceil_div(nkc, ks), split ? (long long)m * n : 0ll, err, lower ? err : nullptr, wait_ns(),
               (int)tune(RL_TUNE_TEST_WITHHOLD_PRODUCT_TILE));
     return RL_OK;
 }
@@ -665,7 +672,7 @@ rl_status dgemm_tc(int m, int n, int k, double alpha, const double *A, long long
     if (ks > 1)
         RL_LAUNCH(dgemm_tc_reduce_kernel, (int)std::min<long long>(4LL * sms, ((long long)m * n + 255) / 256), 256, 0, s, m, n, ks,
                   alpha, part, beta, C, ldc, flags + 1, flags, bn, gx, 0);
-    left = DgemmTcTiles{flags + 1, flags, bn, gx};
+    left = DgemmTcTiles{flags + 1, flags, bn, gx, lower ? err : nullptr};
     taken = true;
     return RL_OK;
 }

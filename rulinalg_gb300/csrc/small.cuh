@@ -175,19 +175,24 @@ struct SmallCholSmem {
 };
 
 // Lower Cholesky in place; only the lower triangle is read or written. A diagonal with
-// |d| < tiny or d < 0 sets *status = RL_ERR_DECOMP_FAILURE. The diagonal is stored as
+// |d| < tiny or d < 0 sets *status = RL_ERR_DECOMP_FAILURE and leaves A as it came, as does a
+// status that is set already (an earlier block's); a failure also sets *host_word (page-locked memory,
+// may be null) to host_mark. The diagonal is stored as
 // d / sqrt(d) (cholesky.rs:160-163).
 template <class T>
-static __global__ void __launch_bounds__(256) small_chol_kernel(T *A, int lda, int n, int *status, T tiny) {
+static __global__ void __launch_bounds__(256) small_chol_kernel(T *A, int lda, int n, int *status, T tiny, int *host_word,
+                                                                int host_mark) {
     constexpr int L = 16;
     __shared__ SmallCholSmem<T> S;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = tid & 3, r = tid >> 2;
+    const int failed = *status;  // read with A in flight
     T a[L];
 #pragma unroll
     for (int i = 0; i < L; i++) {
         const int c = 4 * i + q;
         a[i] = (r < n && c <= r) ? A[(long long)r * lda + c] : T(0);
     }
+    if (failed) return;
     if (tid == 0) S.bad = 0;
     for (int jo = 0; 4 * jo < n; jo++) {
 #pragma unroll
@@ -205,7 +210,10 @@ static __global__ void __launch_bounds__(256) small_chol_kernel(T *A, int lda, i
             }
             __syncthreads();
             if (S.bad) {
-                if (tid == 0) atomicCAS(status, 0, RL_ERR_DECOMP_FAILURE);
+                if (tid == 0) {
+                    atomicCAS(status, 0, RL_ERR_DECOMP_FAILURE);
+                    if (host_word) *(volatile int *)host_word = host_mark;
+                }
                 return;
             }
             const T s = S.s, inv = S.inv, own = S.col[slot][r];
