@@ -17,6 +17,29 @@ namespace {
 
 // ------------------------------------------------------------- host entry points --
 
+// The status word of a call whose products wait (gemm()): the thread's page-locked word, which costs
+// neither an allocation nor a copy and which no kernel touches unless a wait runs out; device memory
+// where there is none.
+struct CallStatus {
+    int *p = nullptr;
+    DevBuf<int> dev;
+    rl_status begin(cudaStream_t s) {
+        if (status_watch().begin()) {
+            p = status_watch().word;
+            return RL_OK;
+        }
+        RL_TRY(dev.alloc(1, s));
+        p = dev.p;
+        RL_TRY_CUDA(cudaMemsetAsync(p, 0, sizeof(int), s));
+        return RL_OK;
+    }
+    rl_status end(cudaStream_t s) {  // waits for the stream
+        if (dev.p) return read_status<int>(dev.p, s);
+        RL_TRY_CUDA(cudaStreamSynchronize(s));
+        return *(volatile int *)p;
+    }
+};
+
 // The public GEMM: FP32 with at least one 128 x 128 tile's worth of C and K >= 256 runs
 // on the tensor cores (3xTF32, FP32 accuracy), FP64 from 6e6 multiply-adds on as exact BF16
 // slices; everything else on the SIMT kernel; both split a long K when the product has few output tiles (gemm()).
@@ -41,18 +64,11 @@ rl_status gemm_host(size_t m, size_t k, size_t n, const T *a, size_t rsa, const 
     RL_TRY(dC.alloc(m * n, s));
     RL_TRY(copy_h2d(dA.p, k, a, rsa, m, k, s));
     RL_TRY(copy_h2d(dB.p, n, b, rsb, k, n, s));
-    DevBuf<int> st;
-    const bool waits = std::is_same<T, float>::value ? sgemm_tc_eligible((int)m, (int)n, (int)k)
-                                                     : dgemm_tc_eligible((int)m, (int)n, (int)k);
-    if (waits) {
-        RL_TRY(st.alloc(1, s));
-        RL_TRY_CUDA(cudaMemsetAsync(st.p, 0, sizeof(int), s));
-    }
+    CallStatus st;
+    RL_TRY(st.begin(s));
     RL_TRY(gemm_public<T>((int)m, (int)n, (int)k, dA.p, (long long)k, dB.p, (long long)n, dC.p, (long long)n, s, st.p));
     RL_TRY(copy_d2h(c, rsc, dC.p, n, m, n, s));
-    if (waits) return read_status<T>(st.p, s);
-    RL_TRY_CUDA(cudaStreamSynchronize(s));
-    return RL_OK;
+    return st.end(s);
 }
 
 template <class T>
@@ -248,12 +264,11 @@ rl_status qr_first_k_host(size_t m, size_t n, const T *qr, size_t lda, const T *
     RL_TRY(dQ.alloc(m * k, s));
     RL_TRY(copy_h2d(dA.p, n, qr, lda, m, n, s));
     if (p) RL_TRY_CUDA(cudaMemcpyAsync(dt.p, tau, p * sizeof(T), cudaMemcpyHostToDevice, s));
-    DevBuf<int> st;
-    RL_TRY(st.alloc(1, s));
-    RL_TRY_CUDA(cudaMemsetAsync(st.p, 0, sizeof(int), s));
+    CallStatus st;
+    RL_TRY(st.begin(s));
     RL_TRY(qr_first_k_dev<T>(dA.p, (long long)n, (int)m, (int)n, dt.p, (int)k, dQ.p, (long long)k, s, st.p));
     RL_TRY(copy_d2h(q, ldq, dQ.p, k, m, k, s));
-    return read_status<T>(st.p, s);
+    return st.end(s);
 }
 
 template <class T>
@@ -272,12 +287,11 @@ rl_status qr_apply_q_host(size_t m, size_t n, const T *qr, size_t lda, const T *
     RL_TRY(copy_h2d(dA.p, n, qr, lda, m, n, s));
     if (p) RL_TRY_CUDA(cudaMemcpyAsync(dt.p, tau, p * sizeof(T), cudaMemcpyHostToDevice, s));
     RL_TRY(copy_h2d(dX.p, q, x, ldx, m, q, s));
-    DevBuf<int> st;
-    RL_TRY(st.alloc(1, s));
-    RL_TRY_CUDA(cudaMemsetAsync(st.p, 0, sizeof(int), s));
+    CallStatus st;
+    RL_TRY(st.begin(s));
     RL_TRY(qr_apply_q_dev<T>(dA.p, (long long)n, (int)m, (int)n, dt.p, (int)q, dX.p, (long long)q, trans, s, st.p));
     RL_TRY(copy_d2h(x, ldx, dX.p, q, m, q, s));
-    return read_status<T>(st.p, s);
+    return st.end(s);
 }
 
 // U X = B (upper = true, back_substitution) or L X = B (forward_substitution) for an
