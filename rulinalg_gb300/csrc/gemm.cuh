@@ -44,12 +44,12 @@ __device__ __forceinline__ void lds4<double>(const double *p, double (&o)[4]) {
 // op(A) is m x k: A[i * lda + p] (TA = false) or A[p * lda + i] (TA = true).
 // op(B) is k x n: B[p * ldb + j] (TB = false) or B[j * ldb + p] (TB = true).
 // LOWER = true computes only the tiles that touch the lower triangle (i >= j) and only
-// writes elements with i >= j (the SYRK form used by Cholesky). only.flags restricts the
-// output to the tiles that the tensor-core kernel left (FP64, gemm_f64tc.cuh).
+// writes elements with i >= j (the SYRK form used by Cholesky). stop (FP64 LOWER, may be null): a
+// status word; if it is set C stays as it is.
 template <class T, bool TA, bool TB, bool LOWER>
 __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T>::BN / GemmCfg<T>::TN))
     gemm_kernel(int m, int n, int k, T alpha, const T *__restrict__ A, long long lda, const T *__restrict__ B,
-                long long ldb, T beta, T *__restrict__ C, long long ldc, int kslice, long long zstride, DgemmTcTiles only) {
+                long long ldb, T beta, T *__restrict__ C, long long ldc, int kslice, long long zstride, const int *stop) {
     constexpr int BM = GemmCfg<T>::BM, BN = GemmCfg<T>::BN, BK = GemmCfg<T>::BK;
     constexpr int TM = GemmCfg<T>::TM, TN = GemmCfg<T>::TN;
     constexpr int NTX = BN / TN, NTY = BM / TM, NT = NTX * NTY;
@@ -71,18 +71,6 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
     const int tx = tid % NTX, ty = tid / NTX;
     const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
     if (LOWER && col0 > row0 + BM - 1) return;  // tile strictly above the diagonal
-    constexpr bool FLAGS = std::is_same<T, double>::value;  // compiled into FP32 the test cost 4% at 2000 x 100 x 2000
-    const int *flag_row = nullptr;
-    if (FLAGS && only.flags) {
-        if (*only.nfail == 0) return;
-        static_assert(!FLAGS || tc64::BM % BM == 0, "one flag row per tile");
-        flag_row = only.flags + (row0 / tc64::BM) * only.gx;
-        const int c1 = min(n, col0 + BN) - 1;
-        int any = 0;
-        for (int c = col0 / only.bn; c <= c1 / only.bn; c++) any |= flag_row[c];
-        if (!any) return;
-    }
-
     T acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; i++)
@@ -157,8 +145,8 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
     const int ktiles = (k + BK - 1) / BK;
     if (ktiles > 0) {
         int stopped = 0;  // read with the first tile in flight
-    if constexpr (LOWER && FLAGS)
-        if (only.stop) stopped = *only.stop;
+    if constexpr (LOWER && std::is_same<T, double>::value)
+        if (stop) stopped = *stop;
     load_tile(0);
     if (stopped) return;
         store_tile(0);
@@ -202,7 +190,6 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
             const int gj = col0 + (j / 4) * (BN / SN_) + tx * 4 + (j % 4);
             if (gj >= n) continue;
             if (LOWER && gj > gi) continue;
-            if (FLAGS && flag_row && !flag_row[gj / only.bn]) continue;
             T *cp = C + (long long)gi * ldc + gj;
             T v = alpha * acc[i][j];
             if (beta != T(0)) v = fma(beta, *cp, v);
@@ -221,14 +208,13 @@ template <class T>
 constexpr int gemm_few_tile() {
     return sizeof(T) == 4 ? 32 : 16;
 }
-template <class T, bool TA, bool TB>
-static __global__ void __launch_bounds__(128)
-    gemm_few_kernel(int m, int n, int k, T alpha, const T *__restrict__ A, long long lda, const T *__restrict__ B, long long ldb,
-                    T beta, T *__restrict__ C, long long ldc) {
+template <class T, bool TA, bool TB, bool LOWER>
+__device__ __forceinline__ void gemm_few_product(int row0, int col0, int m, int n, int k, T alpha, const T *__restrict__ A,
+                                                 long long lda, const T *__restrict__ B, long long ldb, T beta,
+                                                 T *__restrict__ C, long long ldc) {
     constexpr int BT = gemm_few_tile<T>(), BK = 32, R = BT * BT / 128, RS = 128 / BT;  // outputs a thread: rows ty + RS i
     __shared__ T As[BK][BT + 1], Bs[BK][BT + 1];
     const int tid = threadIdx.x, tx = tid % BT, ty = tid / BT;
-    const int row0 = blockIdx.y * BT, col0 = blockIdx.x * BT;
     constexpr int PER = BK * BT / 128;
     T ra[PER], rb[PER], acc[R];
 #pragma unroll
@@ -275,12 +261,54 @@ static __global__ void __launch_bounds__(128)
 #pragma unroll
     for (int i = 0; i < R; i++) {
         const int gi = row0 + ty + RS * i, gj = col0 + tx;
-        if (gi < m && gj < n) {
+        if (gi < m && gj < n && !(LOWER && gj > gi)) {
             T *cp = C + (long long)gi * ldc + gj;
             T v = alpha * acc[i];
             if (beta != T(0)) v = fma(beta, *cp, v);
             *cp = v;
         }
+    }
+}
+
+template <class T, bool TA, bool TB>
+static __global__ void __launch_bounds__(128)
+    gemm_few_kernel(int m, int n, int k, T alpha, const T *__restrict__ A, long long lda, const T *__restrict__ B, long long ldb,
+                    T beta, T *__restrict__ C, long long ldc) {
+    constexpr int BT = gemm_few_tile<T>();
+    gemm_few_product<T, TA, TB, false>(blockIdx.y * BT, blockIdx.x * BT, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
+}
+
+// The tiles of a product that the tensor-core form left (gemm_f64tc.cuh): usually none, and then
+// this is a launch of CTAs that read one word. kLeftCtas CTAs per SM go over the 16 x 16 tiles, each
+// inside one tile of the flags, so that a few flagged tiles still spread over the SMs (LOWER: the
+// elements i >= j). Sums run over k in order, as in gemm_kernel, whose 64 x 64 tiles took them before
+// (us, and the whole product on gemm_kernel without the tensor-core form): identity times dense
+// 192^3 49 (230, 204), 512^3 269 (568, 532), 1024^3 1,861 (2,112, 2,070), 2048^3 14,205 (14,407,
+// 14,303); lower triangle times dense 256^3 94 (336, 270), 2048^3 1,575 (2,753, 14,303). Nothing left:
+// 2048^3 648 (654).
+constexpr int kLeftCtas = 8;
+template <bool TA, bool TB, bool LOWER>
+static __global__ void __launch_bounds__(128)
+    gemm_left_kernel(int m, int n, int k, double alpha, const double *__restrict__ A, long long lda, const double *__restrict__ B,
+                     long long ldb, double beta, double *__restrict__ C, long long ldc, int kslice, long long zstride,
+                     DgemmTcTiles only) {
+    constexpr int BT = gemm_few_tile<double>();
+    static_assert(tc64::BM % BT == 0 && 64 % BT == 0 && 80 % BT == 0, "inside one tile of the flags");
+    if (*only.nfail == 0) return;
+    if (gridDim.z > 1) {  // split K, as in gemm_kernel
+        const int kz = blockIdx.z * kslice;
+        k = max(0, min(kslice, k - kz));
+        A += TA ? (long long)kz * lda : kz;
+        B += TB ? kz : (long long)kz * ldb;
+        C += blockIdx.z * zstride;
+    }
+    const int tn = (n + BT - 1) / BT;
+    const long long total = (long long)tn * ((m + BT - 1) / BT);
+    for (long long t = blockIdx.x; t < total; t += gridDim.x) {
+        const int row0 = (int)(t / tn) * BT, col0 = (int)(t % tn) * BT;
+        if (LOWER && col0 > row0 + BT - 1) continue;
+        if (only.flags[(row0 / tc64::BM) * only.gx + col0 / only.bn])
+            gemm_few_product<double, TA, TB, LOWER>(row0, col0, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
     }
 }
 
@@ -321,7 +349,6 @@ rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T 
     }
     DevBuf<unsigned char> ws;
     DgemmTcTiles left;
-    if (LOWER) left.stop = err;
     if constexpr (std::is_same<T, double>::value) {  // FP64 with enough work: exact slices on the tensor cores
         bool taken = false;
         const int max_k = dgemm_tc_eligible(m, n, k) ? dgemm_tc_max_k(m, n, LOWER) : k;
@@ -336,6 +363,20 @@ rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T 
             RL_TRY((dgemm_tc<TA, TB>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, LOWER, stream, err, ws, left, taken)));
         // what follows computes the tiles that were left (usually none), or all of C
     }
+    auto launch = [&](int nz, T al, T be, T *out, long long ldo, int kslice, long long zstride) -> rl_status {
+        if constexpr (std::is_same<T, double>::value)
+            if (left.flags) {
+                constexpr int BT = gemm_few_tile<T>();
+                const long long small = (long long)ceil_div(n, BT) * ceil_div(m, BT);
+                RL_LAUNCH((gemm_left_kernel<TA, TB, LOWER>), dim3((int)std::min<long long>(small, kLeftCtas * sms), 1, nz), 128, 0,
+                          stream, m, n, k, al, A, lda, B, ldb, be, out, ldo, kslice, zstride, left);
+                return RL_OK;
+            }
+        grid.z = nz;
+        RL_LAUNCH((gemm_kernel<T, TA, TB, LOWER>), grid, NT, 0, stream, m, n, k, al, A, lda, B, ldb, be, out, ldo, kslice, zstride,
+                  LOWER ? (const int *)err : nullptr);
+        return RL_OK;
+    };
     int ksplit = 1;
     if (!LOWER && tiles < sms && k >= 1024) ksplit = std::min({16, ceil_div(2 * sms, tiles), k / 256});
     if (ksplit > 1) {
@@ -343,10 +384,13 @@ rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T 
         ksplit = ceil_div(k, kslice);
         const long long zstride = (long long)m * n;
         DevBuf<T> part;
-        RL_TRY(part.alloc((size_t)ksplit * zstride, stream));
-        grid.z = ksplit;
-        RL_LAUNCH((gemm_kernel<T, TA, TB, LOWER>), grid, NT, 0, stream, m, n, k, T(1), A, lda, B, ldb, T(0), part.p, (long long)n,
-                  kslice, zstride, left);
+        const rl_status mem = part.alloc((size_t)ksplit * zstride, stream);
+        if (mem != RL_OK && left.flags) {  // usually nothing is left: not a reason to fail
+            cudaGetLastError();
+            return launch(1, alpha, beta, C, ldc, k, 0ll);
+        }
+        RL_TRY(mem);
+        RL_TRY(launch(ksplit, T(1), T(0), part.p, (long long)n, kslice, zstride));
         const int rg = std::min(4 * sms, ceil_div(zstride, 256));
         if constexpr (std::is_same<T, double>::value)
             if (left.flags) {
@@ -357,9 +401,7 @@ rl_status gemm(int m, int n, int k, T alpha, const T *A, long long lda, const T 
         RL_LAUNCH(splitk_reduce_kernel<T>, rg, 256, 0, stream, m, n, ksplit, alpha, part.p, beta, C, ldc);
         return RL_OK;
     }
-    RL_LAUNCH((gemm_kernel<T, TA, TB, LOWER>), grid, NT, 0, stream, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, k,
-              0ll, left);
-    return RL_OK;
+    return launch(1, alpha, beta, C, ldc, k, 0ll);
 }
 
 }  // namespace rl

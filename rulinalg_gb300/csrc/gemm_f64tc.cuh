@@ -27,8 +27,8 @@
 // |b| 2^-F truncated to BF16 (a lower bound), and takes 28 or 36 products by it. A tile
 // with an element below both (rows and columns whose large entries do not meet, as after
 // grading or in sparse operands), with an infinity or NaN, or with a row whose largest
-// entry is outside 2^(+-400), is left to the FP64 unit (gemm_kernel over the flagged
-// tiles). Measured rms error in units of 2^-53 |A||B|, against the FP64 unit's kernel:
+// entry is outside 2^(+-400), is left to the FP64 unit (gemm_left_kernel over the
+// flagged tiles). Measured rms error in units of 2^-53 |A||B|, against the FP64 unit's kernel:
 // N(0,1) entries, 512^2 x 256 0.18 (0.47), 2048^3 0.08 (0.47); n on the diagonal 2.0 (8.2)
 // at n = 2048; lognormal entries 1.3 (11.3).
 //
@@ -596,7 +596,6 @@ inline int dgemm_tc_max_k(int m, int n, bool lower) {
 struct DgemmTcTiles {  // the tiles left to the FP64 unit
     const int *flags = nullptr, *nfail = nullptr;
     int bn = 0, gx = 0;
-    const int *stop = nullptr;  // a status word: if set, nothing is left to do (the SYRK form)
 };
 
 // C = alpha op(A) op(B) + beta C. `taken` = false: nothing was done (no memory for the
@@ -672,7 +671,7 @@ rl_status dgemm_tc(int m, int n, int k, double alpha, const double *A, long long
     if (ks > 1)
         RL_LAUNCH(dgemm_tc_reduce_kernel, (int)std::min<long long>(4LL * sms, ((long long)m * n + 255) / 256), 256, 0, s, m, n, ks,
                   alpha, part, beta, C, ldc, flags + 1, flags, bn, gx, 0);
-    left = DgemmTcTiles{flags + 1, flags, bn, gx, lower ? err : nullptr};
+    left = DgemmTcTiles{flags + 1, flags, bn, gx};
     taken = true;
     return RL_OK;
 }
