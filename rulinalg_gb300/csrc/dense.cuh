@@ -23,6 +23,20 @@ __device__ __forceinline__ T quotient(T a, T p, T r) {
     return e == e ? c : q;  // an infinite product has no remainder
 }
 
+// The biased exponent of x (0: zero or subnormal), and whether x times a value of exponent es could
+// leave the normal range: overflow, or lose bits that x has. On integers: a comparison of doubles takes
+// the FP64 unit.
+__device__ __forceinline__ int exponent_of(float x) { return (int)(__float_as_uint(x) >> 23) & 0xff; }
+__device__ __forceinline__ int exponent_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+__device__ __forceinline__ bool scaling_wide(float x, int es) {
+    const int e = exponent_of(x) + es - 127;  // of the product, or one below it
+    return (e < 3 || e > 252) && (__float_as_uint(x) << 1) != 0u;
+}
+__device__ __forceinline__ bool scaling_wide(double x, int es) {
+    const int e = exponent_of(x) + es - 1023;
+    return (e < 3 || e > 2044) && (__double_as_longlong(x) << 1) != 0;
+}
+
 // Largest panel width of the blocked paths.
 template <class T>
 struct PanelNB {
@@ -1462,7 +1476,8 @@ static __global__ void __launch_bounds__(128) trsm_diag_kernel(const T *D, long 
 //     blocks and are reduced once, after the last one;
 //   * the diagonal block is in shared memory from the start: as its inverse (Dinv, FP64 and one
 //     right-hand side: the solve is one more BR x BR product) or scaled by its reciprocal
-//     diagonal, so that a substitution step is one shuffle and one multiply-add.
+//     diagonal, so that a substitution step is one shuffle and one multiply-add (a block whose
+//     scaled entries leave the normal range is substituted unscaled).
 // BR = 128 for FP32; 64 for FP64, where the products of a tile are bound by the FP64 unit.
 // The form before (64-row blocks, a flag per block behind a fence, the folded sums through
 // shared memory) against this one, per sweep: FP64 by substitution n = 4096 992 and 461 us.
@@ -1614,6 +1629,7 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
             const int e = tid + q * THREADS, i = e / BR, j = e % BR;
             Ds[!(INV && Dinv) && trans ? j * LDD + i : i * LDD + j] = dv[q];
         }
+        bool scaled = true;
         if (!(INV && Dinv)) {
             __syncthreads();
             if (tid < BR) {
@@ -1622,8 +1638,23 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
                 inv[tid] = mode == 0 ? T(1) : T(1) / d;
             }
             __syncthreads();
-            if (mode != 0)
-                for (int e = tid; e < BR * BR; e += THREADS) Ds[(e / BR) * LDD + e % BR] *= inv[e / BR];
+            if (mode != 0) {
+                bool wide = false;
+                for (int e = tid; e < BR * BR; e += THREADS) {
+                    const int i = e / BR, j = e % BR;
+                    const T d = Ds[i * LDD + j], f = inv[i];
+                    wide |= (fwd ? j < i : j > i) && scaling_wide(d, exponent_of(f));
+                    Ds[i * LDD + j] = d * f;
+                }
+                if (__syncthreads_or(wide)) {  // the entries as they are, again
+                    scaled = false;
+                    for (int e = tid; e < BR * BR; e += THREADS) {
+                        const int i = e / BR, j = e % BR;
+                        Ds[trans ? j * LDD + i : i * LDD + j] =
+                            (i < bs && j < bs) ? T(A[(long long)(r0 + i) * lda + r0 + j]) : T(0);
+                    }
+                }
+            }
         }
         // the fold: acc[i][c] of row warp 8 + i over this lane's columns; L^T: acc[u][c] of
         // column lane + 32 u of the block over this warp's 8 rows of the earlier block
@@ -1769,10 +1800,26 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
             const int c = warp;
             T z[CPL];
 #pragma unroll
-            for (int h = 0; h < CPL; h++) z[h] = v[(lane + 32 * h) * RW + c] * inv[lane + 32 * h];
-            if (fwd) {
+            for (int h = 0; h < CPL; h++) z[h] = v[(lane + 32 * h) * RW + c] * (scaled ? inv[lane + 32 * h] : T(1));
+            // the 32 unknowns 32 hb ... being eliminated in turn
+            auto step = [&](int hb, int q, T xk, T (&zz)[CPL]) {
 #pragma unroll
-                for (int hb = 0; hb < CPL; hb++)  // the 32 unknowns being eliminated
+                for (int h = 0; h < CPL; h++)
+                    if (fwd ? h > hb || (h == hb && lane > q) : h < hb || (h == hb && lane < q))
+                        zz[h] = fma(-Ds[(lane + 32 * h) * LDD + hb * 32 + q], xk, zz[h]);
+            };
+            if (!scaled) {
+                for (int k = 0; k < BR; k++) {
+                    const int kk = fwd ? k : BR - 1 - k;
+#pragma unroll
+                    for (int hb = 0; hb < CPL; hb++)
+                        if (kk / 32 == hb) step(hb, kk & 31, __shfl_sync(0xffffffffu, z[hb], kk & 31) * inv[kk], z);
+                }
+#pragma unroll
+                for (int h = 0; h < CPL; h++) z[h] *= inv[lane + 32 * h];
+            } else if (fwd) {
+#pragma unroll
+                for (int hb = 0; hb < CPL; hb++)
 #pragma unroll 4
                     for (int q = 0; q < 32; q++) {
                         const T xk = __shfl_sync(0xffffffffu, z[hb], q);

@@ -54,7 +54,8 @@ static __global__ void __launch_bounds__(256) small_lu_kernel(T *A, int lda, int
     }
     if (tid == 0) S.bad = 0;
     const unsigned long long ktiny = amax_key(tiny);
-    int my_piv = 0;  // thread j: the pivot of column j
+    int my_piv = 0;   // thread j: the pivot of column j
+    int my_inv = 0;   // the exponent of 1 / U's diagonal in row r
     for (int jo = 0; 4 * jo < n; jo++) {
 #pragma unroll
         for (int qj = 0; qj < 4; qj++) {
@@ -103,6 +104,7 @@ static __global__ void __launch_bounds__(256) small_lu_kernel(T *A, int lda, int
             const T yj = none ? S.rhsj[slot] : S.rhs[slot][bw];
             if (tid == j) my_piv = wi;
             __syncthreads();
+            if (r == j) my_inv = exponent_of(S.inv);
             if (S.bad) {
                 if (tid == 0) atomicCAS(status, 0, RL_ERR_DIV_BY_ZERO);
                 return;
@@ -130,19 +132,22 @@ static __global__ void __launch_bounds__(256) small_lu_kernel(T *A, int lda, int
     // full rotations so far; a[i] is the local column (done + i) mod 16
     const int done = n / 4;
     if (ipiv && tid < n) ipiv[tid] = my_piv;
+    bool wide = false;  // an entry of U too far from its row's diagonal to be scaled by it
 #pragma unroll
     for (int i = 0; i < L; i++) {
         const int c = 4 * ((done + i) & (L - 1)) + q;
         if (r < n && c < n) {
+            wide |= c > r && scaling_wide(a[i], my_inv);
             A[(long long)r * lda + c] = a[i];
             S.M[r][c] = a[i];
         }
     }
     if (!b) return;
     if (q == 0) S.y[r] = y;
-    __syncthreads();
+    const bool lost = __syncthreads_or(wide) != 0;
     // U x = y by one warp, lane l the rows l and l + 32; rows scaled by the reciprocal
-    // diagonal, so a step is one shuffle and one multiply-add
+    // diagonal, so a step is one shuffle and one multiply-add; with the entries as they are if a
+    // scaled one could leave the normal range.
     if (warp == 0) {
         T z[2], d[2];
 #pragma unroll
@@ -159,6 +164,19 @@ static __global__ void __launch_bounds__(256) small_lu_kernel(T *A, int lda, int
         for (int k = min(n, 32) - 1; k > 0; k--) {
             const T x = __shfl_sync(0xffffffffu, z[0], k);
             if (lane < k) z[0] = fma(-(S.M[lane][k] * d[0]), x, z[0]);
+        }
+        if (lost) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) z[h] = lane + 32 * h < n ? S.y[lane + 32 * h] : T(0);
+            for (int k = n - 1; k >= 0; k--) {
+                const T x = __shfl_sync(0xffffffffu, k < 32 ? z[0] : z[1], k & 31) / S.M[k][k];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int i = lane + 32 * h;
+                    if (i == k) z[h] = x;
+                    if (i < k) z[h] = fma(-S.M[i][k], x, z[h]);
+                }
+            }
         }
 #pragma unroll
         for (int h = 0; h < 2; h++)
