@@ -194,15 +194,18 @@ rl_status launch_cluster(K kern, int C, size_t smem, cudaStream_t s, Args... arg
     return RL_OK;
 }
 
-// The LU panel on one cluster when it fits (launched = true), else nothing. Threads per row
-// and rows per thread follow the rows a CTA holds (256 threads).
+// The LU panel on one cluster when it fits (launched = true), else nothing: the cooperative panel
+// takes it. Threads per row and rows per thread follow the rows a CTA holds (256 threads); each
+// instance says for itself how large a cluster it can have.
 template <class T, int TPR, int RPT>
 static rl_status lu_panel_cluster_launch(T *P, long long lda, int mrows, int kb, int k0, int C, int rows_per, int *ipiv, int *err,
-                                  T tiny, cudaStream_t s) {
+                                         T tiny, cudaStream_t s, bool &launched) {
     static const int cmax = probe_cluster(lu_panel_cluster_kernel<T, TPR, RPT>, kPanelSmem<T>);
-    if (C > cmax) return RL_ERR_CUDA;
-    return launch_cluster(lu_panel_cluster_kernel<T, TPR, RPT>, C, (size_t)rows_per * (PanelNB<T>::value + 1) * sizeof(T), s, P,
-                          lda, mrows, kb, k0, rows_per, ipiv, err, tiny, wait_ns());
+    if (C > cmax) return RL_OK;
+    RL_TRY(launch_cluster(lu_panel_cluster_kernel<T, TPR, RPT>, C, (size_t)rows_per * (PanelNB<T>::value + 1) * sizeof(T), s, P,
+                          lda, mrows, kb, k0, rows_per, ipiv, err, tiny, wait_ns()));
+    launched = true;
+    return RL_OK;
 }
 
 template <class T>
@@ -231,16 +234,15 @@ static rl_status lu_panel_cluster(T *P, long long lda, int mrows, int kb, int k0
                                 std::min<int>(cmax_hw, (int)tune(RL_TUNE_PANEL_CLUSTER_MAX)), panel_target_rows<T>(), rows_per);
     if (C == 0) return RL_OK;
     if (rows_per <= 64)
-        RL_TRY((lu_panel_cluster_launch<T, 4, 1>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s)));
-    else if (rows_per <= 128)
-        RL_TRY((lu_panel_cluster_launch<T, 2, 1>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s)));
-    else if (rows_per <= 256)
-        RL_TRY((lu_panel_cluster_launch<T, 1, 1>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s)));
-    else if (rows_per <= 512)
-        RL_TRY((lu_panel_cluster_launch<T, 1, 2>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s)));
-    else if constexpr (sizeof(T) == 4)  // FP64 rows of 520 bytes end at 407
-        RL_TRY((lu_panel_cluster_launch<T, 1, 4>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s)));
-    launched = true;
+        return lu_panel_cluster_launch<T, 4, 1>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s, launched);
+    if (rows_per <= 128)
+        return lu_panel_cluster_launch<T, 2, 1>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s, launched);
+    if (rows_per <= 256)
+        return lu_panel_cluster_launch<T, 1, 1>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s, launched);
+    if (rows_per <= 512)
+        return lu_panel_cluster_launch<T, 1, 2>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s, launched);
+    if constexpr (sizeof(T) == 4)  // FP64 rows of 520 bytes end at 407
+        return lu_panel_cluster_launch<T, 1, 4>(P, lda, mrows, kb, k0, C, rows_per, ipiv, err, tiny, s, launched);
     return RL_OK;
 }
 
