@@ -306,6 +306,14 @@ __device__ __forceinline__ bool cl_mbar_wait(uint64_t *bar, unsigned parity, uns
     }
 }
 
+// After a wait that ran out: st.async stores of other CTAs into this one may still be under way, which
+// neither the mbarrier (given up) nor a cluster barrier waits for. They take about a microsecond; a CTA
+// stays for 100 before it gives up its shared memory.
+__device__ __forceinline__ void cl_settle() {
+    const unsigned long long t0 = global_ns();
+    while (global_ns() - t0 < 100000) __nanosleep(1000);
+}
+
 // LU panel on one thread-block cluster (up to 16 CTAs): the same algorithm as
 // lu_panel_kernel with the cross-CTA exchange on chip. CTA g owns the rows
 // [g * rows_per, ...), staged in shared memory. The panel is factored 16 columns at a time
@@ -713,6 +721,7 @@ static __global__ void __launch_bounds__(256) lu_panel_cluster_kernel(T *P, long
         P[(long long)(r0 + r) * lda + c] = R[r * LDR + c];
     }
     cluster.sync();  // no CTA leaves while another may still use its shared memory
+    if (*(volatile int *)&S.dead) cl_settle();
 }
 
 // The same panel with look-ahead across columns. After column j's winner is known a CTA
@@ -1173,6 +1182,7 @@ static __global__ void __launch_bounds__(256) qr_panel_cluster_kernel(T *P, long
         P[(long long)(r0 + r) * lda + c] = R[r * LDR + c];
     }
     cluster.sync();  // no CTA leaves while another may still store into its shared memory
+    if (*(volatile int *)&S.fail[0] | *(volatile int *)&S.fail[1]) cl_settle();
 }
 
 // ------------------------------------------------------------------- row swaps --
