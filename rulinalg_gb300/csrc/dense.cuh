@@ -1582,8 +1582,8 @@ __device__ __forceinline__ void sweep_put(double *p, double v) {
 template <class T, int RW>
 struct SweepCfg {
     static constexpr int BR = sweep_rows<T>(), WARPS = BR / 8, THREADS = 32 * WARPS, CPL = BR / 32, LDD = BR + 1;
-    // the diagonal block; v and the awaited solution, or the warps' column sums (L^T)
-    static constexpr size_t SMEM = sizeof(T) * (BR * LDD + 2 * BR * RW + (size_t)WARPS * BR * RW);
+    // the diagonal block, v and the awaited solution; behind them the warps' column sums (L^T only)
+    static constexpr size_t SMEM = sizeof(T) * (BR * LDD + 2 * BR * RW), SMEM_LT = SMEM + sizeof(T) * WARPS * BR * RW;
 };
 
 template <class T, class TA, int RW>
@@ -1650,7 +1650,7 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
             __syncthreads();
             if (mode != 0) {
                 bool wide = false;
-                for (int e = tid; e < BR * BR; e += THREADS) {
+                for (int e = tid; e < bs * BR; e += THREADS) {
                     const int i = e / BR, j = e % BR;
                     const T d = Ds[i * LDD + j], f = inv[i];
                     wide |= (fwd ? j < i : j > i) && scaling_wide(d, exponent_of(f));
@@ -1819,8 +1819,8 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
                         zz[h] = fma(-Ds[(lane + 32 * h) * LDD + hb * 32 + q], xk, zz[h]);
             };
             if (!scaled) {
-                for (int k = 0; k < BR; k++) {
-                    const int kk = fwd ? k : BR - 1 - k;
+                for (int k = 0; k < bs; k++) {
+                    const int kk = fwd ? k : bs - 1 - k;
 #pragma unroll
                     for (int hb = 0; hb < CPL; hb++)
                         if (kk / 32 == hb) step(hb, kk & 31, __shfl_sync(0xffffffffu, z[hb], kk & 31) * inv[kk], z);
@@ -1829,19 +1829,21 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_ke
                 for (int h = 0; h < CPL; h++) z[h] *= inv[lane + 32 * h];
             } else if (fwd) {
 #pragma unroll
-                for (int hb = 0; hb < CPL; hb++)
+                for (int hb = 0; hb < CPL; hb++) {
+                    const int lim = min(32, bs - hb * 32);  // a short block's steps only
 #pragma unroll 4
-                    for (int q = 0; q < 32; q++) {
+                    for (int q = 0; q < lim; q++) {
                         const T xk = __shfl_sync(0xffffffffu, z[hb], q);
 #pragma unroll
                         for (int h = hb; h < CPL; h++)
                             if (h > hb || lane > q) z[h] = fma(-Ds[(lane + 32 * h) * LDD + hb * 32 + q], xk, z[h]);
                     }
+                }
             } else {
 #pragma unroll
                 for (int hb = CPL - 1; hb >= 0; hb--)
 #pragma unroll 4
-                    for (int q = 31; q >= 0; q--) {
+                    for (int q = min(32, bs - hb * 32) - 1; q >= 0; q--) {
                         const T xk = __shfl_sync(0xffffffffu, z[hb], q);
 #pragma unroll
                         for (int h = 0; h <= hb; h++)

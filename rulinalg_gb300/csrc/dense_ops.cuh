@@ -607,15 +607,15 @@ static rl_status sweep_launch_w(const TA *A, long long lda, int n, const T *Dinv
     auto kern = trsv_sweep_kernel<T, TA, RW>;
     static int per_sm = 0;
     static const cudaError_t attr = [&] {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg::SMEM);
-        return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, cfg::THREADS, cfg::SMEM);
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg::SMEM_LT);
+        return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, cfg::THREADS, cfg::SMEM_LT);
     }();
     RL_TRY_CUDA(attr);
     const int groups = sweep_groups(nrhs), nb = ceil_div(n, cfg::BR);
     T *x = static_cast<T *>(ws);
     int *tickets = reinterpret_cast<int *>(x + (size_t)groups * n * RW);
     const dim3 grid(std::min(nb, std::max(1, per_sm) * num_sms()), groups);
-    RL_LAUNCH(kern, grid, cfg::THREADS, cfg::SMEM, s, A, lda, n, Y, ldy, nrhs, mode, x, tickets, dstatus, tiny, wait_ns(),
+    RL_LAUNCH(kern, grid, cfg::THREADS, mode == 3 ? cfg::SMEM_LT : cfg::SMEM, s, A, lda, n, Y, ldy, nrhs, mode, x, tickets, dstatus, tiny, wait_ns(),
               (int)tune(RL_TUNE_TEST_WITHHOLD_SWEEP_BLOCK), Dinv);
     return RL_OK;
 }
