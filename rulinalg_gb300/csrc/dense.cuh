@@ -1579,20 +1579,20 @@ __device__ __forceinline__ void sweep_put(double *p, double v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(u == ~0ull ? 0x7fffffffffffffffull : u) : "memory");
 }
 
-template <class T, int RW>
+template <class T, int RW, int ROWS>
 struct SweepCfg {
-    static constexpr int BR = sweep_rows<T>(), WARPS = BR / 8, THREADS = 32 * WARPS, CPL = BR / 32, LDD = BR + 1;
+    static constexpr int BR = ROWS, WARPS = BR / 8, THREADS = 32 * WARPS, CPL = BR / 32, LDD = BR + 1;
     // the diagonal block, v and the awaited solution; behind them the warps' column sums (L^T only)
     static constexpr size_t SMEM = sizeof(T) * (BR * LDD + 2 * BR * RW), SMEM_LT = SMEM + sizeof(T) * WARPS * BR * RW;
 };
 
-template <class T, class TA, int RW>
-static __global__ void __launch_bounds__(SweepCfg<T, RW>::THREADS) trsv_sweep_kernel(const TA *__restrict__ A, long long lda,
+template <class T, class TA, int RW, int ROWS>
+static __global__ void __launch_bounds__(SweepCfg<T, RW, ROWS>::THREADS) trsv_sweep_kernel(const TA *__restrict__ A, long long lda,
                                                              int n, T *__restrict__ Y, long long ldy, int nrhs, int mode,
                                                              T *ws, int *tickets, int *status, T tiny,
                                                              unsigned long long wait_ns, int withhold,
                                                              const T *__restrict__ Dinv) {
-    using cfg = SweepCfg<T, RW>;
+    using cfg = SweepCfg<T, RW, ROWS>;
     constexpr int BR = cfg::BR, CPL = cfg::CPL, LDD = cfg::LDD, THREADS = cfg::THREADS, WARPS = cfg::WARPS;
     constexpr bool INV = sizeof(T) == 8 && RW == 1;  // the instance that is called with Dinv
     extern __shared__ __align__(16) unsigned char smem_raw[];

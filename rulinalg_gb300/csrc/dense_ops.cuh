@@ -600,11 +600,11 @@ rl_status qr_apply_q_dev(const T *QR, long long lda, int m, int n, const T *tau,
 // inverted diagonal blocks Dinv: the 1-wide instance for one right-hand side (the 8-wide one would
 // issue 8 FMAs per element, 7 of them predicated off, each a full issue of the FP64 pipe for T =
 // double). ws as trsv_sweep_kernel takes it.
-template <class T, class TA, int RW>
+template <class T, class TA, int RW, int ROWS = sweep_rows<T>()>
 static rl_status sweep_launch_w(const TA *A, long long lda, int n, const T *Dinv, T *Y, long long ldy, int nrhs, int mode,
                                 int *dstatus, cudaStream_t s, T tiny, void *ws) {
-    using cfg = SweepCfg<T, RW>;
-    auto kern = trsv_sweep_kernel<T, TA, RW>;
+    using cfg = SweepCfg<T, RW, ROWS>;
+    auto kern = trsv_sweep_kernel<T, TA, RW, ROWS>;
     static int per_sm = 0;
     static const cudaError_t attr = [&] {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg::SMEM_LT);
@@ -622,6 +622,11 @@ static rl_status sweep_launch_w(const TA *A, long long lda, int n, const T *Dinv
 template <class T, class TA>
 static rl_status sweep_launch(const TA *A, long long lda, int n, const T *Dinv, T *Y, long long ldy, int nrhs, int mode,
                               int *dstatus, cudaStream_t s, T tiny, void *ws) {
+    if constexpr (sweep_rows<T>() > 64)
+        if (n <= 64)  // one block either way: half the threads and shared memory
+            return sweep_width(nrhs) == 1
+                       ? sweep_launch_w<T, TA, 1, 64>(A, lda, n, Dinv, Y, ldy, nrhs, mode, dstatus, s, tiny, ws)
+                       : sweep_launch_w<T, TA, kSweepRhs, 64>(A, lda, n, Dinv, Y, ldy, nrhs, mode, dstatus, s, tiny, ws);
     return sweep_width(nrhs) == 1 ? sweep_launch_w<T, TA, 1>(A, lda, n, Dinv, Y, ldy, nrhs, mode, dstatus, s, tiny, ws)
                                   : sweep_launch_w<T, TA, kSweepRhs>(A, lda, n, Dinv, Y, ldy, nrhs, mode, dstatus, s, tiny, ws);
 }
