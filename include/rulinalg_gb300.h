@@ -108,6 +108,12 @@ RL_API rl_status rl_tune_get(int key, int64_t *value);
 /* C = A * B with A m x k, B k x n, C m x n; alpha = 1, beta = 0. Large products wait on the
  * tensor cores, bounded by RL_TUNE_WAIT_TIMEOUT_NS: a wait that runs out leaves NaN in its tile
  * of C, and the host-pointer calls return RL_ERR_TIMEOUT.
+ * FP64 products of 6e6 multiply-adds and more (1e6 with K > 512) take 18 bytes of device memory per
+ * element of A and of B, and 8 per element of C and slice when few outputs make them split K, from the
+ * device's memory pool, which keeps freed blocks; without them they run on the FP64 unit, as they do in
+ * a stream capture. The FP64 factorisations and the residuals of mixed solves with more than 4
+ * right-hand sides are made of such products (a residual slices the n x n matrix each time: 4.8 GB at
+ * n = 16384).
  * Replaces the matrixmultiply::{sgemm,dgemm} calls of mat_mul_general!
  * (src/matrix/mat_mul.rs:33-43 and :57-67): rsa/rsb are the row strides that
  * `row_stride()` supplies there, rsc = n for a new Matrix. */

@@ -1,5 +1,5 @@
 // Batched solve kernels (thousands of independent systems, n <= 512, one launch) and
-// the one-CTA kernels used by the single-matrix entry points for n <= 512.
+// the one-CTA kernels used by the single-matrix entry points (dense_ops.cuh has their sizes).
 #pragma once
 
 #include <cfloat>
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(CTA_THREADS, CtaOcc<TF>::value) batch_solve_ke
     }
 }
 
-// ------------------------------------------------ single matrices with n <= 512 --
+// ------------------------------------------------ single matrices on one CTA --
 
 // Factor one matrix in place. kind 0: LU (ipiv receives LAPACK-style pivots),
 // 1: Cholesky. status[0] receives the result.

@@ -1,8 +1,9 @@
 // Single-matrix entry points: GEMM, PartialPivLu, Cholesky, HouseholderQr and the
 // Matrix::solve/inverse/det conveniences. Host-pointer calls copy the operands to the
 // GPU (row stride preserved by 2D copies), run the kernels on the calling thread's
-// default stream and copy the results back. Matrices with n <= 512 are factored by one
-// CTA (factor_cta.cuh); larger ones by the blocked multi-CTA path (dense.cuh + GEMM).
+// default stream and copy the results back. Matrices up to one_cta_lu / one_cta_chol rows
+// (dense_ops.cuh) are factored by one CTA (small.cuh, factor_cta.cuh); larger ones by the
+// blocked multi-CTA path (dense.cuh + GEMM).
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -40,9 +41,9 @@ struct CallStatus {
     }
 };
 
-// The public GEMM: FP32 with at least one 128 x 128 tile's worth of C and K >= 256 runs
-// on the tensor cores (3xTF32, FP32 accuracy), FP64 from 6e6 multiply-adds on as exact BF16
-// slices; everything else on the SIMT kernel; both split a long K when the product has few output tiles (gemm()).
+// The public GEMM: FP32 products that sgemm_tc_eligible names run on the tensor cores (3xTF32,
+// FP32 accuracy), FP64 ones that dgemm_tc_eligible names as exact BF16 slices; everything else on
+// the SIMT kernels; all split a long K when the product has few output tiles (gemm()).
 template <class T>
 rl_status gemm_public(int m, int n, int k, const T *a, long long lda, const T *b, long long ldb, T *c, long long ldc,
                       cudaStream_t s, int *err) {

@@ -1,5 +1,5 @@
-// Kernels of the blocked (multi-CTA) factorisations used for n > 512 and for every
-// HouseholderQr: cooperative panel kernels with a bounded grid barrier, row swaps,
+// Kernels of the blocked (multi-CTA) factorisations used above one_cta_lu / one_cta_chol rows
+// (dense_ops.cuh) and for every HouseholderQr: cooperative panel kernels with a bounded grid barrier, row swaps,
 // diagonal-block triangular solves and the compact-WY T factor. Trailing updates are
 // GEMMs (gemm.cuh).
 #pragma once

@@ -158,8 +158,8 @@ struct Dots {
 // backward-error test passes. Restarted GMRES(m) in FP64 on M^-1 A d = M^-1 r with
 // CGS2 orthogonalisation; Givens rotations and the small triangular solve on the GPU.
 // It gives up (ok = false) when a restart cycle does not cut the residual tenfold or when
-// the host clock passes `deadline` (seconds, host_seconds()): past that an FP64
-// refactorisation is the cheaper way to the answer.
+// the host clock passes `deadline` (seconds, host_seconds()); the caller then refactors in
+// FP64.
 inline double host_seconds() {
     return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
@@ -556,10 +556,12 @@ struct MixedFactor {
             need_fp64 = diverged;
         }
         if (!need_fp64) {
-            // GMRES-IR on each remaining column, within a budget of the estimated time of
-            // the FP64 refactor it would otherwise save: the panel chain (~3.3 us per column
-            // measured) plus 2/3 n^3 flops for LU, 1/3 n^3 for Cholesky, at the ~1 TFLOP/s
-            // of the FP64 blocked factorisations. A first correction that grew
+            // GMRES-IR on each remaining column, within a budget of host time: 3.3 us per column
+            // of a panel chain plus 2/3 n^3 flops for LU, 1/3 n^3 for Cholesky, at 1 TFLOP/s. That
+            // was the time of the FP64 refactor it saves when products ran on the FP64 unit; a
+            // refactor takes a fraction of it now (LU n = 4096 26 of 59 ms, 8192 88 of 394). The
+            // budget stays, as it decides which systems end here and which in FP64 arithmetic: a
+            // system that uses it up costs the budget and the refactor. A first correction that grew
             // (kappa u_32 > 1) does not tell a system GMRES-IR converges on (kappa ~ 1e8)
             // from one it never will (kappa ~ 1e10); the GMRES residual does (gmres_ir).
             out.path = RL_PATH_GMRES;

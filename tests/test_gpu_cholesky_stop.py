@@ -39,3 +39,24 @@ def test_early_failure_is_cheap(gpu, n):
     bad = [once() for _ in range(5)]
     assert all(st == 0 for st, _ in good) and all(st != 0 for st, _ in bad)
     assert sorted(t for _, t in bad)[2] <= 0.3 * sorted(t for _, t in good)[2]
+
+
+def test_threads_keep_their_own_outcome(gpu):
+    from concurrent.futures import ThreadPoolExecutor
+    rng = np.random.default_rng(9)
+    g = rng.standard_normal((300, 300))
+    good = g @ g.T + 300 * np.eye(300)
+    bad = good.copy()
+    bad[70, 70] = -1.0
+
+    def job(i):
+        if i % 3 == 2:
+            return np.abs(gpu.mat_mul(good, g) - good @ g).max() <= 300 * 2.0 ** -52 * np.abs(good).max() * np.abs(g).max() * 4
+        try:
+            l = gpu.Cholesky.decompose(bad if i % 3 else good).unpack()
+            return i % 3 == 0 and np.abs(l @ l.T - good).max() <= 300 * 2.0 ** -52 * np.abs(good).max()
+        except gpu.RulinalgError as e:
+            return i % 3 == 1 and e.kind == "DecompFailure"
+
+    with ThreadPoolExecutor(6) as ex:
+        assert all(ex.map(job, range(90)))
