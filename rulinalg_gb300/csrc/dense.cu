@@ -26,7 +26,7 @@ struct CallStatus {
     DevBuf<int> dev;
     rl_status begin(cudaStream_t s) {
         if (status_watch().begin()) {
-            p = status_watch().word;
+            p = status_watch().call_word();
             return RL_OK;
         }
         RL_TRY(dev.alloc(1, s));

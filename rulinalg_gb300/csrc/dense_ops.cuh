@@ -77,11 +77,12 @@ rl_status factor_small(T *A, long long lda, int n, int kind, int *ipiv, cudaStre
 
 // A calling thread's view of a factorisation in progress: a page-locked status word that kernels set
 // to this call's mark (a kernel that an earlier call left behind sets an older one) and an event behind
-// the kernel to look at, kept until the thread ends. Without them (no memory) the host reads the status
-// at the end only.
+// the kernel to look at, kept until the thread ends; a second word is the status of host calls
+// (dense.cu). Without them (no memory) the host reads a status in device memory at the end.
 struct StatusWatch {
     int *word = nullptr, mark = 0;
     cudaEvent_t ev = nullptr;
+    int *call_word() const { return word + 8; }
     ~StatusWatch() {
         if (word) cudaFreeHost(word);
         if (ev) cudaEventDestroy(ev);
@@ -93,7 +94,7 @@ struct StatusWatch {
             cudaGetLastError();
             return false;
         }
-        *(volatile int *)word = 0;
+        *(volatile int *)word = *(volatile int *)call_word() = 0;
         mark = mark % INT_MAX + 1;
         return true;
     }

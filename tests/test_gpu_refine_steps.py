@@ -62,3 +62,39 @@ def test_several_right_hand_sides_converge(gpu, nrhs):
     assert info["path"] == "refinement"
     r = np.abs(bs - a @ x).max(axis=0)
     assert (r <= 4 * np.sqrt(1024) * 2.0 ** -53 * np.abs(a).sum(axis=1).max() * np.abs(x).max(axis=0)).all()
+
+
+@pytest.mark.parametrize("n", [1, 5, 33, 63, 64, 65, 100, 300])
+def test_small_orders(gpu, n):
+    """Below the sizes with inverted blocks: the substitution sweeps in every mode, one and three columns."""
+    rng = np.random.default_rng(n)
+    a = rng.uniform(-1, 1, (n, n)) + 3 * np.eye(n)
+    g = rng.standard_normal((n, n))
+    for m, kind in ((a, "lu"), (g @ g.T + n * np.eye(n), "cholesky")):
+        for b in (rng.standard_normal(n), rng.standard_normal((n, 3))):
+            x, info = gpu.solve_mixed(m, b, kind)
+            assert info["path"] == "refinement"
+            assert np.abs(b - m @ x).max() <= 4 * np.sqrt(n) * 2.0 ** -53 * np.abs(m).sum(axis=1).max() * np.abs(x).max()
+
+
+@pytest.mark.parametrize("kind,nrhs", [("lu", 1), ("cholesky", 1), ("lu", 9)])
+def test_withheld_block_is_reported(gpu, kind, nrhs):
+    """A block of the refinement's sweeps (and of the FP64 fallback's) is never published: the waits for
+    it end by their own limit, the call returns the timeout, and the next one is right."""
+    from rulinalg_gb300 import _lib as L
+    n = 1000
+    rng = np.random.default_rng(n)
+    g = rng.standard_normal((n, n))
+    a = g @ g.T + n * np.eye(n) if kind == "cholesky" else g + 40 * np.eye(n)
+    b = rng.standard_normal((n, nrhs))
+    try:
+        gpu.tune_set(L.TUNE_WAIT_TIMEOUT_NS, 20_000_000)
+        gpu.tune_set(L.TUNE_TEST_WITHHOLD_SWEEP_BLOCK, 5)
+        with pytest.raises(gpu.DeviceError) as e:
+            gpu.solve_mixed(a, b, kind)
+        assert e.value.status == 35
+    finally:
+        gpu.tune_set(L.TUNE_TEST_WITHHOLD_SWEEP_BLOCK, -1)
+        gpu.tune_set(L.TUNE_WAIT_TIMEOUT_NS, 10 ** 9)
+    x, info = gpu.solve_mixed(a, b, kind)
+    assert info["path"] == "refinement" and np.abs(b - a @ x).max() <= 1e-11 * np.abs(b).max()
