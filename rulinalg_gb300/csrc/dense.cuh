@@ -1488,7 +1488,7 @@ static __global__ void __launch_bounds__(128) trsm_diag_kernel(const T *D, long 
 //     right-hand side: the solve is one more BR x BR product) or scaled by its reciprocal
 //     diagonal, so that a substitution step is one shuffle and one multiply-add (a block whose
 //     scaled entries leave the normal range is substituted unscaled).
-// BR = 128 for FP32; 64 for FP64, where the products of a tile are bound by the FP64 unit.
+// BR = 128 for FP32 (64 up to 64 rows); 64 for FP64, where the products of a tile are bound by the FP64 unit.
 // The form before (64-row blocks, a flag per block behind a fence, the folded sums through
 // shared memory) against this one, per sweep: FP64 by substitution n = 4096 992 and 461 us.
 // A CTA waits only on tickets taken before its own, by CTAs that are running, so the sweep
@@ -1808,47 +1808,56 @@ static __global__ void __launch_bounds__(SweepCfg<T, RW, ROWS>::THREADS) trsv_sw
             // substitution with the scaled rows: warp c solves right-hand side c, lane l
             // holds the rows l + 32 h
             const int c = warp;
-            T z[CPL];
+            // The products with each other group of 32 unknowns are summed apart (t) and subtracted
+            // once: fewer roundings at the size of z.
+            T z[CPL], t[CPL];
 #pragma unroll
-            for (int h = 0; h < CPL; h++) z[h] = v[(lane + 32 * h) * RW + c] * (scaled ? inv[lane + 32 * h] : T(1));
-            // the 32 unknowns 32 hb ... being eliminated in turn
-            auto step = [&](int hb, int q, T xk, T (&zz)[CPL]) {
-#pragma unroll
-                for (int h = 0; h < CPL; h++)
-                    if (fwd ? h > hb || (h == hb && lane > q) : h < hb || (h == hb && lane < q))
-                        zz[h] = fma(-Ds[(lane + 32 * h) * LDD + hb * 32 + q], xk, zz[h]);
-            };
+            for (int h = 0; h < CPL; h++) {
+                z[h] = v[(lane + 32 * h) * RW + c] * (scaled ? inv[lane + 32 * h] : T(1));
+                t[h] = T(0);
+            }
             if (!scaled) {
                 for (int k = 0; k < bs; k++) {
-                    const int kk = fwd ? k : bs - 1 - k;
+                    const int kk = fwd ? k : bs - 1 - k, q = kk & 31;
 #pragma unroll
-                    for (int hb = 0; hb < CPL; hb++)
-                        if (kk / 32 == hb) step(hb, kk & 31, __shfl_sync(0xffffffffu, z[hb], kk & 31) * inv[kk], z);
+                    for (int hb = 0; hb < CPL; hb++) {
+                        if (kk / 32 != hb) continue;
+                        const T xk = __shfl_sync(0xffffffffu, z[hb], q) * inv[kk];
+#pragma unroll
+                        for (int h = 0; h < CPL; h++)
+                            if (fwd ? h > hb || (h == hb && lane > q) : h < hb || (h == hb && lane < q))
+                                z[h] = fma(-Ds[(lane + 32 * h) * LDD + kk], xk, z[h]);
+                    }
                 }
 #pragma unroll
                 for (int h = 0; h < CPL; h++) z[h] *= inv[lane + 32 * h];
             } else if (fwd) {
 #pragma unroll
-                for (int hb = 0; hb < CPL; hb++) {
+                for (int hb = 0; hb < CPL; hb++) {  // the 32 unknowns being eliminated
                     const int lim = min(32, bs - hb * 32);  // a short block's steps only
 #pragma unroll 4
                     for (int q = 0; q < lim; q++) {
                         const T xk = __shfl_sync(0xffffffffu, z[hb], q);
+                        if (lane > q) z[hb] = fma(-Ds[(lane + 32 * hb) * LDD + hb * 32 + q], xk, z[hb]);
 #pragma unroll
-                        for (int h = hb; h < CPL; h++)
-                            if (h > hb || lane > q) z[h] = fma(-Ds[(lane + 32 * h) * LDD + hb * 32 + q], xk, z[h]);
+                        for (int h = hb + 1; h < CPL; h++) t[h] = fma(Ds[(lane + 32 * h) * LDD + hb * 32 + q], xk, t[h]);
                     }
+#pragma unroll
+                    for (int h = hb + 1; h < CPL; h++) z[h] -= t[h], t[h] = T(0);
                 }
             } else {
 #pragma unroll
-                for (int hb = CPL - 1; hb >= 0; hb--)
+                for (int hb = CPL - 1; hb >= 0; hb--) {
 #pragma unroll 4
                     for (int q = min(32, bs - hb * 32) - 1; q >= 0; q--) {
                         const T xk = __shfl_sync(0xffffffffu, z[hb], q);
+                        if (lane < q) z[hb] = fma(-Ds[(lane + 32 * hb) * LDD + hb * 32 + q], xk, z[hb]);
 #pragma unroll
-                        for (int h = 0; h <= hb; h++)
-                            if (h < hb || lane < q) z[h] = fma(-Ds[(lane + 32 * h) * LDD + hb * 32 + q], xk, z[h]);
+                        for (int h = 0; h < hb; h++) t[h] = fma(Ds[(lane + 32 * h) * LDD + hb * 32 + q], xk, t[h]);
                     }
+#pragma unroll
+                    for (int h = 0; h < hb; h++) z[h] -= t[h], t[h] = T(0);
+                }
             }
 #pragma unroll
             for (int h = 0; h < CPL; h++) publish(lane + 32 * h, c, z[h]);

@@ -4,7 +4,7 @@
 // updates use all four schedulers: FP64 work issues at 2 multiply-adds per cycle and SM here,
 // and the one-CTA factorisation of factor_cta.cuh, with a row per thread, took 229 us for
 // n = 47 in FP64 and its solve another 37 (two thirds of a warp's lanes idle, a division per
-// thread); this takes 82 us with the solve (n = 16: 60 + 18, 27 now). A column's reciprocal (and square root) is formed by one warp and shared, two CTA
+// thread); this takes 84 us with the solve (n = 16: 60 + 18, 27 now). A column's reciprocal (and square root) is formed by one warp and shared, two CTA
 // barriers per column; multipliers are corrected to the quotient a / p by its remainder
 // (Markstein, IBM J. Res. Dev. 34, 1990), so they are the reference's (lu.rs:609,
 // cholesky.rs:160-171) in all but rare last-bit cases.
@@ -25,11 +25,17 @@ __device__ __forceinline__ void rotate4(T (&a)[16]) {
     a[15] = first;
 }
 
+// a + b in a call: under a predicate the addition would take the FP64 unit of warps that do not need it.
+template <class T>
+__device__ __noinline__ T add_apart(T a, T b) {
+    return a + b;
+}
+
 template <class T>
 struct SmallLuSmem {
     T row[2][8][kSmallN];  // the warps' candidate rows by column parity (entry q 16 + i, rotated)
     T rowj[2][kSmallN];    // the row at position j
-    T rhs[2][8], rhsj[2];
+    T rhs[2][8], rhs0[2][8], rhsj[2];
     T M[kSmallN][kSmallN + 1];
     T y[kSmallN];
     T piv, inv;
@@ -46,7 +52,11 @@ static __global__ void __launch_bounds__(256) small_lu_kernel(T *A, int lda, int
     constexpr int L = 16;
     __shared__ __align__(16) SmallLuSmem<T> S;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = tid & 3, r = tid >> 2;
-    T a[L], y = (b && r < n) ? b[r] : T(0);
+    // The right-hand side's products with the first 32 unknowns are summed apart from it in the rows
+    // from 32 on (warps 4 to 7: y the sum, y0 the right-hand side, until column 32): fewer roundings at
+    // its size (n = 64, diagonally weighted: forward error 1.01 of blocked substitution's, 1.22 without).
+    T a[L], y = (b && r < n) ? b[r] : T(0), y0 = T(0);
+    if (warp >= 4) y0 = y, y = T(0);
 #pragma unroll
     for (int i = 0; i < L; i++) {
         const int c = 4 * i + q;
@@ -70,7 +80,7 @@ static __global__ void __launch_bounds__(256) small_lu_kernel(T *A, int lda, int
             warp_amax_key<T>(bk, bi);
             if (bk != 0ull && r == bi) {
                 stv<L>(&S.row[slot][warp][q * L], a);
-                if (q == 0) S.rhs[slot][warp] = y;
+                if (q == 0) S.rhs[slot][warp] = y, S.rhs0[slot][warp] = y0;
             }
             if (r == j) {
                 stv<L>(&S.rowj[slot][q * L], a);
@@ -97,11 +107,15 @@ static __global__ void __launch_bounds__(256) small_lu_kernel(T *A, int lda, int
             }
             T pr[L];
             ldv<L>(prow + q * L, pr);
+            T yj = none ? S.rhsj[slot] : S.rhs[slot][bw];
+            if (!none && bw >= 4 && j < 32) yj = add_apart(yj, S.rhs0[slot][bw]);
             if (wi != j && (r == j || r == wi)) {
                 ldv<L>((r == j ? prow : S.rowj[slot]) + q * L, a);
-                y = r == j ? S.rhs[slot][bw] : S.rhsj[slot];
+                const T old = S.rhsj[slot];
+                const bool apart = warp >= 4 && j < 32;  // row wi, there
+                y = r == j ? yj : (apart ? T(0) : old);
+                y0 = old;
             }
-            const T yj = none ? S.rhsj[slot] : S.rhs[slot][bw];
             if (tid == j) my_piv = wi;
             __syncthreads();
             if (r == j) my_inv = exponent_of(S.inv);
@@ -128,6 +142,7 @@ static __global__ void __launch_bounds__(256) small_lu_kernel(T *A, int lda, int
             }
         }
         if (4 * jo + 4 <= n) rotate4(a);
+        if (jo == 7 && warp >= 4) y = add_apart(y, y0);
     }
     // full rotations so far; a[i] is the local column (done + i) mod 16
     const int done = n / 4;
@@ -156,11 +171,13 @@ static __global__ void __launch_bounds__(256) small_lu_kernel(T *A, int lda, int
             d[h] = i < n ? T(1) / S.M[i][i] : T(0);
             z[h] = i < n ? quotient(S.y[i], S.M[i][i], d[h]) : T(0);
         }
+        T t = T(0);  // the products with the unknowns from 32 on, summed apart
         for (int k = n - 1; k >= 32; k--) {
             const T x = __shfl_sync(0xffffffffu, z[1], k - 32);
-            z[0] = fma(-(S.M[lane][k] * d[0]), x, z[0]);
+            t = fma(S.M[lane][k] * d[0], x, t);
             if (lane + 32 < k) z[1] = fma(-(S.M[lane + 32][k] * d[1]), x, z[1]);
         }
+        z[0] -= t;
         for (int k = min(n, 32) - 1; k > 0; k--) {
             const T x = __shfl_sync(0xffffffffu, z[0], k);
             if (lane < k) z[0] = fma(-(S.M[lane][k] * d[0]), x, z[0]);
